@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libaieplace_gb300.so")
 CLI = os.path.join(HERE, "aieplace")  # the command-line placer (csrc/cli.cpp), linked to LIB
-SOURCES = ["capi.cu", "k_wirelength.cu", "k_density.cu", "k_field_simt.cu", "k_field_tc.cu", "k_surrogate.cu",
+SOURCES = ["capi.cu", "k_wirelength.cu", "k_density.cu", "k_field_fft.cu", "k_field_tc.cu", "k_surrogate.cu",
            "synth.cpp", "lefdef.cpp", "config.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

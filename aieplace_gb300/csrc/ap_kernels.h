@@ -188,19 +188,20 @@ void launch_perturb(int n_mov, const float *vx, const float *vy, const float *gx
                     const float *w, const float *h, cudaStream_t st);
 
 // ---- field solve ------------------------------------------------------------
-// Spectral solver state for an m x m grid (square, m a multiple of 32).
+// Spectral solver state for an m x m grid (square, m a power of two, 32..4096).
 constexpr int kTcCandidates = 5;  // tensor-core solve variants the autotuner times
 
 struct FieldSolver {
     int m;
     float bin_ratio;
-    // constant transform matrices, row-major m x m:
+    // FP32 path (k_field_fft.cu): twiddle tables, spectral frequencies per
+    // index, scratch maps between its passes (m^2 and 2 m^2 floats)
+    float2 *tab;
+    float *wx, *wy;
+    float *t, *u;
+    // tensor-core path: constant transform matrices, row-major m x m, as BF16 hi/lo pairs:
     //   C[k][i] = cos(pi k (i+1/2)/m), Ct = C^T, St[i][k] = sin(pi k (i+1/2)/m)
-    float *C, *Ct, *St;
     __nv_bfloat16 *C_hi, *C_lo, *Ct_hi, *Ct_lo, *St_hi, *St_lo;
-    float *wx, *wy;          // spectral frequencies per index
-    // scratch (fp32 path)
-    float *t0, *px, *py, *ux, *uy;
     // scratch (bf16 path): hi/lo pairs
     __nv_bfloat16 *b_t_hi, *b_t_lo, *b_px_hi, *b_px_lo, *b_py_hi, *b_py_lo, *b_ux_hi, *b_ux_lo,
         *b_uy_hi, *b_uy_lo;
@@ -214,8 +215,8 @@ struct FieldSolver {
                              // 3, 4: one persistent launch of 128 x 128 tiles, K of stages 1-2
                              // split in two (3) or not (4)
     float tc_tune_ms[kTcCandidates];  // measured solve time of each variant (-1: not run)
-    int simt_bm;             // FP32 path tile (32 or 64); 0 = size rule
-    float simt_tune_ms[2];   // measured solve time with 32 / 64 tiles
+    int simt_tile;           // FP32 path: 32 (blocks of up to 256 threads) or 64 (512 threads)
+    float simt_ms[2];        // its measured solve time, at [simt_tile == 64]; the other -1
     // failure injection (ap_debug_inject): the tcgen05 kernels issue no loads
     // and bound each wait by fault_wait_ns, so their waits run out
     int fault_stall;
@@ -224,7 +225,7 @@ struct FieldSolver {
 
 int field_solver_init(FieldSolver &f, int m, float bin_ratio, int want_bf16);
 void field_solver_free(FieldSolver &f);
-// density d (x-major) -> ex, ey; FP32 SIMT contraction
+// density d (x-major) -> ex, ey; FP32 fast transforms
 // gate: the launches run only if gate is null or (1 << *gate) & gate_mask
 // (the loop's surrogate schedule lives in device memory)
 void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cudaStream_t st,
@@ -262,29 +263,31 @@ int gather_grid(int n_mov, int block_nodes);
 // the blocks of all four bucket launches
 int wa_plan(WaArgs &a);
 
-// One contraction stage of an FP32 field solve (S1..S4 of k_field_simt.cu):
-// D[z] = A[z] B[z]^T on an m x m grid in bm x bm tiles, `batch` values of z,
-// the spectral epilogue (phi -> px, py) when `spectral`.
+// One pass of an FP32 field solve (k_field_fft.cu).
 struct FieldRec {
-    const float *A[2];
-    const float *B[2];
-    float *C[2];
-    float *px, *py;
+    const float *d;       // P1 in: the density map
+    float *t, *u;         // between the passes
+    float *ex, *ey;       // P3 out
+    const float2 *tab;
     const float *wx, *wy;
-    float scale;
-    int m, bm, spectral, batch;
+    float scale;          // 4 / m^2
+    int m, pass;
+    int row_lo, row_hi;   // P3: rows of this record
+    int wide;             // ex, ey aligned to 8 bytes
 };
-// the four stages of field_solve_fp32(f, d, ex, ey) with the solver's tuned tile
-void field_records(const FieldSolver &f, const float *d, float *ex, float *ey, FieldRec rec[4]);
-inline int field_rec_blocks(const FieldRec &r) { return (r.m / r.bm) * (r.m / r.bm) * r.batch; }
+// the passes of field_solve_fp32(f, d, ex, ey) as four records (P3 in two
+// halves) for blocks of 8 tile threads; false if a block of the tile is too
+// small for the grid (tile 32: more than 1024 bins)
+bool field_records(const FieldSolver &f, const float *d, float *ex, float *ey, int tile, FieldRec rec[4]);
+int field_rec_blocks(const FieldRec &r, int tile);
 
 // one persistent launch of a stage over the records `recs` (device memory)
 // with the grid persist_*_wave() (one wave of resident blocks)
 int persist_density_wave(int stage);
 int persist_wa_wave(int bucket);  // 0, 1, 2: the thread-per-net buckets; 3: the larger nets
-int persist_field_wave();
+int persist_field_wave(int tile, int m);  // m: the largest grid of the launch
 void launch_persist_density(int stage, const PersistQueue &q, const void *recs, cudaStream_t st);
 void launch_persist_wa(int bucket, const PersistQueue &q, const WaArgs *recs, cudaStream_t st);
-void launch_persist_field(const PersistQueue &q, const FieldRec *recs, cudaStream_t st);
+void launch_persist_field(const PersistQueue &q, const FieldRec *recs, int tile, int m, cudaStream_t st);
 
 }  // namespace ap

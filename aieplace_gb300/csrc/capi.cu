@@ -1156,10 +1156,10 @@ int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *sim
     if (tc_variant) *tc_variant = h->fs.tc_ready ? h->fs.tc_variant : -1;
     if (tc_ms)
         for (int v = 0; v < kTcCandidates; ++v) tc_ms[v] = h->fs.tc_tune_ms[v];
-    if (simt_tile) *simt_tile = h->fs.simt_bm;
+    if (simt_tile) *simt_tile = h->fs.simt_tile;
     if (simt_ms) {
-        simt_ms[0] = h->fs.simt_tune_ms[0];
-        simt_ms[1] = h->fs.simt_tune_ms[1];
+        simt_ms[0] = h->fs.simt_ms[0];
+        simt_ms[1] = h->fs.simt_ms[1];
     }
     return AP_OK;
 }
@@ -1781,7 +1781,7 @@ int ap_surrogate_collect(ap_handle *h, ap_surrogate *s, int32_t n_trials, int32_
 
 // The persistent form's device tables, rebuilt whenever the set of active
 // instances changes.  Stage records in item order; the field stage holds
-// four records per instance (its contractions S1..S4), all instances' S1
+// four records per instance (field_records), all instances' first passes
 // first, record k + 1 of an instance depending on its record k.
 struct PersistPlan {
     int n_rec[PS_COUNT] = {};
@@ -1797,7 +1797,8 @@ struct PersistPlan {
     // four WA launches, [8] field, [9 ..) field done counters (the gather
     // follows the field and the WA launches)
     unsigned int *d_cnt = nullptr;
-    int field_bm = 0;  // 0: each instance's own tuned tile; else 32 or 64 for all
+    int field_tile = 32;  // blocks of the field launch have 8 field_tile threads (32 or 64)
+    int field_m = 0;      // the largest grid of the field launch
     int item_blocks = 0;  // blocks per work item of the non-field stages; 0: the size rule
 };
 
@@ -1821,9 +1822,9 @@ struct ap_batch {
     unsigned int *d_status = nullptr;  // a dependency wait of a persistent launch gave up
     unsigned long long wait_ns = 1000000000ull;
     int never_arrive = 0;
-    int tuned_bm = 0;                  // the field tile the batch autotuner chose (0: not tuned)
+    int tuned_tile = 0;                  // the field tile the batch autotuner chose (0: not tuned)
     int item_blocks = 0;               // blocks per work item (0: the size rule)
-    float tune_ms[2] = {0.f, 0.f};     // persistent field launch with 32 / 64 tiles
+    float tune_ms[2] = {0.f, 0.f};     // persistent field launch with tile 32 / 64 (-1: not run)
 };
 
 namespace {
@@ -1841,9 +1842,9 @@ void plan_free(PersistPlan &pp) {
     }
     if (pp.d_dep) cudaFree(pp.d_dep);
     if (pp.d_cnt) cudaFree(pp.d_cnt);
-    const int bm = pp.field_bm, ib = pp.item_blocks;
+    const int tile = pp.field_tile, ib = pp.item_blocks;
     pp = PersistPlan();
-    pp.field_bm = bm;
+    pp.field_tile = tile;
     pp.item_blocks = ib;
 }
 
@@ -1868,14 +1869,14 @@ int stage_wave(int k) {
     case PS_WA:
         return persist_wa_wave(3);
     case PS_FIELD:
-        return persist_field_wave();
+        return persist_field_wave(32, 512);  // not asked for: a field item is one block
     default:
         return persist_density_wave(k);
     }
 }
 
 // Blocks per work item of a stage: every stage but the field (whose items
-// are contraction tiles waited on one by one) takes about kItemsPerBlock
+// are transform passes waited on one by one) takes about kItemsPerBlock
 // items per resident block, so that the per-item costs (queue fetch,
 // argument copy, barriers) stay small against the work.
 constexpr int kItemsPerBlock = 4;
@@ -1951,12 +1952,9 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
         bw[3].push_back(all - wr.small_blocks);
         wa.push_back(wr);
         FieldRec fr[4];
-        field_records(h->fs, h->d_dens, h->d_ex, h->d_ey, fr);
-        for (int k = 0; k < 4; ++k) {
-            if (pp.field_bm == 64 && fr[k].m % 64 == 0) fr[k].bm = 64;
-            if (pp.field_bm == 32) fr[k].bm = 32;
-            fld[k].push_back(fr[k]);
-        }
+        if (!field_records(h->fs, h->d_dens, h->d_ex, h->d_ey, pp.field_tile, fr)) return AP_ERR_UNSUPPORTED;
+        for (int k = 0; k < 4; ++k) fld[k].push_back(fr[k]);
+        pp.field_m = std::max(pp.field_m, h->fs.m);
         gat.push_back(loop_gather_args(h));
         bg.push_back(gather_grid(h->n_mov, h->p.block_nodes));
     }
@@ -1967,8 +1965,8 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
     for (int k = 0; k < 4; ++k)
         for (int i = 0; i < ni; ++i) {
             fall.push_back(fld[k][i]);
-            bf.push_back(field_rec_blocks(fld[k][i]));
-            dep.push_back(k == 0 ? -1 : (k - 1) * ni + i);
+            bf.push_back(field_rec_blocks(fld[k][i], pp.field_tile));
+            dep.push_back(k == 0 ? -1 : std::min(k - 1, 1) * ni + i);  // both halves of P3 wait for P2
         }
     int r = upload_stage(pp, PS_UPDATE, upd, bu);
     if (r == AP_OK) r = upload_stage(pp, PS_SCATTER, sct, bs);
@@ -2044,7 +2042,8 @@ int enqueue_persist(ap_batch *b, cudaStream_t st) {
     CK(cudaEventRecord(b->wa_join, b->wa_stream));
     launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.d_recs[PS_SCATTER], st);
     launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.d_recs[PS_RHO], st);
-    launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]), st);
+    launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]),
+                         pp.field_tile, pp.field_m, st);
     CK(cudaStreamWaitEvent(st, b->wa_join, 0));
     launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.d_recs[PS_GATHER], st);
     return cudaGetLastError() == cudaSuccess ? AP_OK : AP_ERR_CUDA;
@@ -2071,7 +2070,8 @@ int persist_profile(ap_batch *b, int n_trials, float *ms) {
         CK(cudaEventRecord(ev[3], st));
         launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.d_recs[PS_RHO], st);
         CK(cudaEventRecord(ev[4], st));
-        launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]), st);
+        launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]),
+                         pp.field_tile, pp.field_m, st);
         CK(cudaEventRecord(ev[5], st));
         launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.d_recs[PS_GATHER],
                                st);
@@ -2126,11 +2126,10 @@ int batch_build_graph(ap_batch *b) {
     return ei == cudaSuccess ? AP_OK : AP_ERR_CUDA;
 }
 
-// Tile autotuner of the persistent field launch: every active instance's
-// four contractions with 32 x 32 and with 64 x 64 tiles (instances whose
-// grid is not a multiple of 64 keep 32), 2 warm and 5 timed launches each on
-// the instances' own scratch; the faster is kept.  The tile does not change
-// the results (each output sums its products in the same order).
+// Tile autotuner of the persistent field launch: blocks of 256 and of 512
+// threads (tile 32 and 64), 2 warm and 5 timed launches each on the
+// instances' own scratch; the faster is kept.  Grids of more than 1024 bins
+// need 64 (the other is not run: -1).  The tile does not change the results.
 int batch_tune_field(ap_batch *b) {
     if (b->form != AP_BATCH_PERSISTENT) return AP_OK;
     cudaEvent_t e0, e1;
@@ -2138,8 +2137,13 @@ int batch_tune_field(ap_batch *b) {
     CK(cudaEventCreate(&e1));
     int r = AP_OK;
     const int cand[2] = {32, 64};
+    int largest = 0;
+    for (size_t i = 0; i < b->inst.size(); ++i)
+        if (b->active[i]) largest = std::max(largest, b->inst[i]->fs.m);
     for (int v = 0; v < 2 && r == AP_OK; ++v) {
-        b->plan.field_bm = cand[v];
+        b->tune_ms[v] = -1.f;
+        if (v == 0 && largest > 1024) continue;
+        b->plan.field_tile = cand[v];
         r = plan_build(b, b->plan);
         if (r != AP_OK) break;
         const int nf = b->plan.n_rec[PS_FIELD];
@@ -2150,7 +2154,8 @@ int batch_tune_field(ap_batch *b) {
                 cudaSuccess)
                 r = AP_ERR_CUDA;
             launch_persist_field(plan_queue(b, PS_FIELD, 3, 0),
-                                 static_cast<const FieldRec *>(b->plan.d_recs[PS_FIELD]), b->main);
+                                 static_cast<const FieldRec *>(b->plan.d_recs[PS_FIELD]),
+                                 b->plan.field_tile, b->plan.field_m, b->main);
         }
         if (r == AP_OK && (cudaEventRecord(e1, b->main) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess))
             r = AP_ERR_CUDA;
@@ -2161,8 +2166,8 @@ int batch_tune_field(ap_batch *b) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (r == AP_OK) r = batch_sync(b);
-    b->tuned_bm = b->tune_ms[0] <= b->tune_ms[1] ? 32 : 64;
-    b->plan.field_bm = b->tuned_bm;
+    b->tuned_tile = b->tune_ms[0] >= 0.f && b->tune_ms[0] <= b->tune_ms[1] ? 32 : 64;
+    b->plan.field_tile = b->tuned_tile;
     return r;
 }
 
@@ -2235,7 +2240,7 @@ int ap_batch_set_form(ap_batch *b, int32_t form) {
     CK(cudaStreamSynchronize(b->main));
     const bool rebuild = b->graph != nullptr;
     b->form = form;
-    if (form == AP_BATCH_PERSISTENT && !b->tuned_bm) {
+    if (form == AP_BATCH_PERSISTENT && !b->tuned_tile) {
         const int r = batch_tune_field(b);
         if (r != AP_OK) return r;
     }
@@ -2250,7 +2255,7 @@ int ap_batch_get_info(ap_batch *b, ap_batch_info *info) {
     int act = 0;
     for (char a : b->active) act += a ? 1 : 0;
     info->active = act;
-    info->field_tile = b->tuned_bm;
+    info->field_tile = b->tuned_tile;
     info->field_tune_ms[0] = b->tune_ms[0];
     info->field_tune_ms[1] = b->tune_ms[1];
     for (int k = 0; k < 6; ++k) {  // the WA entry: the launch of the larger nets; its items: all four launches'

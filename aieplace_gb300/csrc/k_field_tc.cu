@@ -1,6 +1,6 @@
 // Electrostatic field solve on the 5th-generation tensor cores (sm_103a).
 //
-// Same four contraction stages as the FP32 path (k_field_simt.cu, restating
+// Same four contraction stages as the FP32 path (once dense contractions; now k_field_fft.cu, restating
 // replace::FFT::doFFT, python/AIEmath/fft_replace/fft.cpp:204-299), each
 //   D[i][j] = sum_k A[i][k] B[j][k]
 // with A a constant transform matrix and B the data, both stored as a BF16
@@ -1342,9 +1342,9 @@ int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv
     for (int pass = 0; pass < 2; ++pass) {
         for (int v = 0; v < kTcVariants; ++v) {
             if (v >= 3 && persist_capacity<Tile128>() <= 0) continue;
-            for (int w = 0; w < 3; ++w) run_variant(v, f, f.ux, f.uy, 0);
+            for (int w = 0; w < 3; ++w) run_variant(v, f, f.u, f.u + (size_t)f.m * f.m, 0);
             cudaEventRecord(e0, 0);
-            for (int t = 0; t < 5; ++t) run_variant(v, f, f.ux, f.uy, 0);
+            for (int t = 0; t < 5; ++t) run_variant(v, f, f.u, f.u + (size_t)f.m * f.m, 0);
             cudaEventRecord(e1, 0);
             if (cudaEventSynchronize(e1) != cudaSuccess) {
                 cudaEventDestroy(e0);

@@ -5,7 +5,7 @@
 // exact solve during the early, high-overflow iterations of the ePlace loop:
 //
 //   fine density (M x M)  --pool f x f-->  coarse density (R x R, R = M / f)
-//   coarse density  --exact spectral solve at R (FP32, k_field_simt.cu)-->  coarse field
+//   coarse density  --exact spectral solve at R (FP32, k_field_fft.cu)-->  coarse field
 //   network input X0 [f^2 + 2][R][R]: the f x f sub-bin densities of each
 //       coarse bin (space-to-depth) and the coarse field scaled by f / s
 //   4-layer conv net (32 channels, ReLU)  -->  Y [2 f^2][R][R]

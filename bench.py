@@ -46,9 +46,11 @@ KERNELS_BESIDE_FIELD = 8
 
 
 def field_launches(info: dict, solver: str) -> int:
-    """Launches of one field solve: four stage launches, or one for the
-    persistent tensor-core candidates (3, 4)."""
-    return 1 if solver == "bf16x3" and info.get("tc_variant", -1) in (3, 4) else 4
+    """Launches of one field solve: three FP32 passes; of the tensor-core solve
+    four stage launches, or one for its persistent candidates (3, 4)."""
+    if solver == "fp32":
+        return 3
+    return 1 if info.get("tc_variant", -1) in (3, 4) else 4
 
 
 STAGES = ["scatter+update", "density+overflow", "wirelength", "field", "gather+control"]

@@ -46,7 +46,7 @@ enum {
 
 /* ---- field solvers ----------------------------------------------------- */
 enum {
-    AP_FIELD_FP32 = 0,   /* dense per-axis transforms, FP32 SIMT contraction */
+    AP_FIELD_FP32 = 0,   /* fast per-axis transforms, FP32 */
     AP_FIELD_BF16X3 = 1  /* dense per-axis transforms, tcgen05 BF16 x3 split, FP32 accumulate */
 };
 
@@ -181,8 +181,9 @@ int ap_set_log(ap_handle *h, const char *path, int32_t capacity);
  * 128 x 64, 2 stages, two CTAs per SM; 3: one persistent launch over the four
  * stages' 128 x 128 tiles, K of the first two stages split in two; 4: the
  * same without the split; -1 if the
- * tensor-core path is unavailable), simt_tile the FP32 tile side (32 or 64);
- * tc_ms[5] and simt_ms[2] the candidates' times (-1: not run).  The
+ * tensor-core path is unavailable), simt_tile the FP32 solve's block (32: up to
+ * 256 threads, 64: 512 threads); tc_ms[5] the candidates' times, simt_ms[0]
+ * or [1] the FP32 solve's by its block (-1: not run).  The
  * environment variable AP_TC_VARIANT=0..4, read at ap_create, pins a
  * candidate that ran instead of the fastest (for testing each one). */
 int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *simt_tile, float *simt_ms);
@@ -251,7 +252,7 @@ int ap_node_force(ap_handle *h, const float *x, const float *y, const float *ex,
  * budget, a path where cudaMalloc must not run -- this is the FP32 solve of
  * ap_field_solve on caller-owned DEVICE buffers (density in; ex, ey out;
  * x-major bins*bins floats) that allocates nothing: its scratch is one fixed
- * array in the library's static device memory, sized for bins <= 256 (2.1 MB,
+ * array in the library's static device memory, sized for bins <= 256 (0.8 MB,
  * held on every GPU that loads the library until the process exits).  bins
  * must be a multiple of 32 in [32, 256]; other sizes return
  * AP_ERR_INVALID_ARG.  bin_ratio is bin height / bin width (ap_create uses
@@ -306,7 +307,7 @@ int ap_restore(ap_handle *h, const void *buf, size_t bytes);
  *                        (instance, block)
  *                        work items off a device queue, so instances of uneven
  *                        size share the GPU; the field solve's four
- *                        contractions of an instance wait on one another
+ *                        passes of an instance wait on one another
  *                        inside the launch (bounded waits, below), with the
  *                        tile chosen by the batch's autotuner.  Needs the FP32
  *                        field solve and no surrogate; the default where it
