@@ -207,6 +207,7 @@ struct FieldSolver {
         *b_uy_hi, *b_uy_lo;
     void *tc_maps;           // tensor maps of the tcgen05 path (host table)
     int tc_ready;
+    int tc_pinned;           // AP_TC_VARIANT chose the candidate: the mixed-precision solver runs it
     unsigned int *tc_status; // device error flag of the tcgen05 kernels
     unsigned int *tc_sync;   // row-block counters of the persistent tcgen05 solve
     float *tc_part;          // its split-K partials
@@ -223,7 +224,8 @@ struct FieldSolver {
     unsigned long long fault_wait_ns;
 };
 
-int field_solver_init(FieldSolver &f, int m, float bin_ratio, int want_bf16);
+int field_solver_init(FieldSolver &f, int m, float bin_ratio);
+int field_solver_matrices(FieldSolver &f);  // the tensor-core path's constants and scratch
 void field_solver_free(FieldSolver &f);
 // density d (x-major) -> ex, ey; FP32 fast transforms
 // gate: the launches run only if gate is null or (1 << *gate) & gate_mask

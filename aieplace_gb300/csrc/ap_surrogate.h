@@ -34,9 +34,6 @@ struct SurrState {
     int R = 0, M = 0;
     FieldSolver coarse{};
     float *d_pool = nullptr, *d_cex = nullptr, *d_cey = nullptr;  // R x R
-    // tcgen05 coarse solve (R a multiple of 128): pooled density as BF16 hi/lo
-    int tc = 0;
-    __nv_bfloat16 *d_phi = nullptr, *d_plo = nullptr;
     float *d_scale = nullptr;                                     // [1]
     float *d_x0 = nullptr, *d_act[2] = {nullptr, nullptr}, *d_y = nullptr;
     float *d_sex = nullptr, *d_sey = nullptr;  // M x M: the surrogate field of a judged trial

@@ -120,9 +120,31 @@ namespace {
 
 int solver_of(const ap_handle *h, int32_t solver) { return solver >= 0 ? solver : h->p.field_solver; }
 
+// Whether the mixed-precision solver of this handle runs on the tensor cores:
+// only where AP_TC_VARIANT pins a candidate or a failure is injected.
+// Otherwise it takes the FP32 fast transforms too, which are the faster at
+// every grid it serves and the more exact (solve alone, tensor cores against
+// transforms: 128^2 bins 23.8 / 9, 512^2 31 / 11, 1024^2 53 / 18 us; 2-norm
+// error at 1024^2 1.3e-5 / 2e-7).
+bool on_tensor_cores(const ap_handle *h, int solver) {
+    return solver == AP_FIELD_BF16X3 && h->fs.tc_ready && (h->fs.tc_pinned || h->fs.fault_stall);
+}
+
+// The tensor-core solve's matrices, buffers and candidates' times, made on
+// first use; nothing of the handle may be in flight (the tuning runs on the
+// solver's scratch).
+int ensure_tensor_cores(ap_handle *h) {
+    if (h->fs.tc_ready) return AP_OK;
+    if (h->fs.m % 128 != 0) return AP_ERR_UNSUPPORTED;  // the tcgen05 tiles need bins a multiple of 128
+    const size_t nb = (size_t)h->fs.m * h->fs.m;
+    if (!h->d_dens_hi) CK(dalloc(&h->d_dens_hi, nb));
+    if (!h->d_dens_lo) CK(dalloc(&h->d_dens_lo, nb));
+    return field_solver_bind_bf16(h->fs, h->d_dens_hi, h->d_dens_lo);
+}
+
 // density map (bf16 split or fp32 already in place) -> ex, ey
 int run_field(ap_handle *h, int solver, cudaStream_t st, const int *gate = nullptr, int gate_mask = 0) {
-    if (solver == AP_FIELD_BF16X3) {
+    if (on_tensor_cores(h, solver)) {
         int r = field_solve_bf16x3(h->fs, h->d_dens_hi, h->d_dens_lo, h->d_ex, h->d_ey, st, gate, gate_mask);
         if (r != AP_OK) return r;
     } else {
@@ -168,7 +190,7 @@ RhoArgs rho_args(ap_handle *h, int mode, double *out) {
     a.inv_ab = h->inv_ab;
     a.inv_ab_f = (float)h->inv_ab;
     a.d_shift = h->d_shift;
-    if (h->p.field_solver == AP_FIELD_BF16X3) {
+    if (on_tensor_cores(h, h->p.field_solver)) {
         a.d_hi = h->d_dens_hi;
         a.d_lo = h->d_dens_lo;
     } else {
@@ -280,7 +302,7 @@ GatherArgs loop_gather_args(ap_handle *h) {
 // launches of that source only (one body of the graph's switch node).
 int enqueue_field_surrogate(ap_handle *h, cudaStream_t st, int branch) {
     const int *gate = &h->d_sc->field_mode;
-    const bool f32 = h->p.field_solver != AP_FIELD_BF16X3;
+    const bool f32 = !on_tensor_cores(h, h->p.field_solver);
     if (branch != kFieldExact)
         surr_enqueue_field(h->surr->net, h->surr_state, f32 ? h->d_dens : nullptr, f32 ? nullptr : h->d_dens_hi,
                            f32 ? nullptr : h->d_dens_lo, h->d_ex, h->d_ey, gate, st);
@@ -349,7 +371,7 @@ int enqueue_eval(ap_handle *h, int at, int rho_mode, int wa_mode, cudaStream_t s
 // one wait covers both (a separate read after the wait was a second round
 // trip per call).
 int sync(ap_handle *h) {
-    const bool tc = h->fs.tc_ready && h->fs.tc_status;
+    const bool tc = h->fs.tc_ready && (h->fs.tc_pinned || h->fs.fault_stall);
     if (tc)
         CK(cudaMemcpyAsync(h->h_status, h->fs.tc_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
@@ -908,8 +930,6 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(dalloc(&h->d_fix_q, nb));
     A(dalloc(&h->d_fixs_q, nb));
     A(dalloc(&h->d_dens, nb));
-    A(dalloc(&h->d_dens_hi, nb));
-    A(dalloc(&h->d_dens_lo, nb));
     A(dalloc(&h->d_ex, nb));
     A(dalloc(&h->d_ey, nb));
     A(dalloc(&h->d_sx, N));
@@ -994,13 +1014,14 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
         A(cudaMemcpy(h->d_fixs_q, fs.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice));
         A(cudaMemset(h->d_mov_q, 0, sizeof(ull) * nb));
     }
-    int r = ok ? field_solver_init(h->fs, p.bins_x, g.bh / g.bw, 1)
-               : AP_ERR_CUDA;
+    int r = ok ? field_solver_init(h->fs, p.bins_x, g.bh / g.bw) : AP_ERR_CUDA;
     if (r == AP_OK && p.bins_x % 128 == 0) {
-        r = field_solver_bind_bf16(h->fs, h->d_dens_hi, h->d_dens_lo);
-        if (r != AP_OK && p.field_solver != AP_FIELD_BF16X3) r = AP_OK;  // tensor path optional here
+        if (getenv("AP_TC_VARIANT")) {
+            r = ensure_tensor_cores(h);
+            if (r != AP_OK && p.field_solver != AP_FIELD_BF16X3) r = AP_OK;  // tensor path optional here
+        }
     } else if (r == AP_OK && p.field_solver == AP_FIELD_BF16X3) {
-        r = AP_ERR_UNSUPPORTED;  // the tcgen05 tiles need bins a multiple of 128
+        r = AP_ERR_UNSUPPORTED;  // the mixed-precision solver takes bins a multiple of 128
     }
     if (r != AP_OK) {
         ap_destroy(h);
@@ -1153,6 +1174,11 @@ int ap_set_log(ap_handle *h, const char *path, int32_t capacity) {
 
 int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *simt_tile, float *simt_ms) {
     if (!h) return AP_ERR_INVALID_ARG;
+    if (h->fs.m % 128 == 0 && !h->fs.tc_ready) {
+        CK(cudaStreamSynchronize(h->stream));
+        const int r = ensure_tensor_cores(h);
+        if (r != AP_OK) return r;
+    }
     if (tc_variant) *tc_variant = h->fs.tc_ready ? h->fs.tc_variant : -1;
     if (tc_ms)
         for (int v = 0; v < kTcCandidates; ++v) tc_ms[v] = h->fs.tc_tune_ms[v];
@@ -1478,7 +1504,7 @@ int ap_field_solve(ap_handle *h, const float *density, float *ex, float *ey, int
     const int sv = solver_of(h, solver);
     if (sv != AP_FIELD_FP32 && sv != AP_FIELD_BF16X3) return AP_ERR_INVALID_ARG;
     const int nb = h->p.bins_x * h->p.bins_y;
-    if (sv == AP_FIELD_BF16X3 && !h->fs.tc_ready) return AP_ERR_UNSUPPORTED;
+    if (sv == AP_FIELD_BF16X3 && h->fs.m % 128 != 0) return AP_ERR_UNSUPPORTED;
     // the field does not depend on the map's mean (phi_00 = 0); taking it off
     // keeps the transforms' DC sums from swamping the AC terms in rounding
     double mean = 0.0;
@@ -1487,7 +1513,7 @@ int ap_field_solve(ap_handle *h, const float *density, float *ex, float *ey, int
     std::vector<float> shifted((size_t)nb);
     for (int b = 0; b < nb; ++b) shifted[(size_t)b] = density[b] - (float)mean;
     CK(cudaMemcpyAsync(h->d_dens, shifted.data(), sizeof(float) * nb, cudaMemcpyHostToDevice, h->stream));
-    if (sv == AP_FIELD_BF16X3) launch_split_bf16(nb, h->d_dens, h->d_dens_hi, h->d_dens_lo, h->stream);
+    if (on_tensor_cores(h, sv)) launch_split_bf16(nb, h->d_dens, h->d_dens_hi, h->d_dens_lo, h->stream);
     int r = run_field(h, sv, h->stream);
     if (r != AP_OK) return r;
     CK(cudaGetLastError());
@@ -1560,10 +1586,13 @@ int ap_debug_inject(ap_handle *h, int32_t kind, int64_t wait_ns) {
     if (!h) return AP_ERR_INVALID_ARG;
     if (kind != AP_FAULT_NONE && kind != AP_FAULT_TC_STALL) return AP_ERR_INVALID_ARG;
     if (kind == AP_FAULT_TC_STALL && (wait_ns < 1000000 || wait_ns > 2000000000)) return AP_ERR_INVALID_ARG;
-    if (kind == AP_FAULT_TC_STALL && !h->fs.tc_ready) return AP_ERR_UNSUPPORTED;
     // nothing of this handle may be in flight while the solver changes
     CK(cudaStreamSynchronize(h->stream));
     if (h->wa_stream) CK(cudaStreamSynchronize(h->wa_stream));
+    if (kind == AP_FAULT_TC_STALL) {
+        const int r = ensure_tensor_cores(h);
+        if (r != AP_OK) return r;
+    }
     h->fs.fault_stall = kind == AP_FAULT_TC_STALL;
     h->fs.fault_wait_ns = kind == AP_FAULT_TC_STALL ? (unsigned long long)wait_ns : 0ull;
     if (kind == AP_FAULT_NONE) {
@@ -1742,7 +1771,7 @@ int ap_surrogate_collect(ap_handle *h, ap_surrogate *s, int32_t n_trials, int32_
     ap_surrogate *attached = h->surr;
     h->surr = nullptr;
     r = upload_schedule(h);
-    const bool f32 = h->p.field_solver != AP_FIELD_BF16X3;
+    const bool f32 = !on_tensor_cores(h, h->p.field_solver);
     const size_t RR = (size_t)s->R * s->R;
     int got = 0;
     cudaStream_t st = h->stream;

@@ -649,8 +649,6 @@ void fill_tables(const FieldSolver &f, cudaStream_t st) {
     field_table_kernel<<<(n + 127) / 128, 128, 0, st>>>(f.tab, f.wx, f.wy, f.m, f.bin_ratio);
 }
 
-// The constant transform matrices of the tensor-core solve as BF16 hi/lo
-// pairs: C[k][i] = cos(pi k (i+1/2)/m), Ct = C^T, St[i][k] = sin(pi k (i+1/2)/m).
 __global__ void split_kernel(int n, const float *src, __nv_bfloat16 *hi, __nv_bfloat16 *lo) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float v = src[i];
@@ -665,7 +663,18 @@ int dmalloc(T **p, size_t n) {
     return cudaMalloc((void **)p, sizeof(T) * (n ? n : 1)) == cudaSuccess ? 0 : -1;
 }
 
-int init_matrices(FieldSolver &f) {
+}  // namespace
+
+void launch_split_bf16(int n, const float *src, __nv_bfloat16 *hi, __nv_bfloat16 *lo, cudaStream_t st) {
+    int blocks = (n + 255) / 256;
+    if (blocks > 4096) blocks = 4096;
+    split_kernel<<<blocks, 256, 0, st>>>(n, src, hi, lo);
+}
+
+// The tensor-core solve's constant transform matrices as BF16 hi/lo pairs,
+// and its scratch.
+int field_solver_matrices(FieldSolver &f) {
+    if (f.C_hi) return AP_OK;
     const int m = f.m;
     const size_t nn = (size_t)m * m;
     std::vector<float> C(nn), Ct(nn), St(nn);
@@ -683,7 +692,7 @@ int init_matrices(FieldSolver &f) {
          dmalloc(&f.b_py_hi, nn) | dmalloc(&f.b_py_lo, nn) | dmalloc(&f.b_ux_hi, nn) | dmalloc(&f.b_ux_lo, nn) |
          dmalloc(&f.b_uy_hi, nn) | dmalloc(&f.b_uy_lo, nn);
     if (e) return AP_ERR_CUDA;
-    // staged through the solve's scratch (nothing has used it yet)
+    // staged through the solve's scratch
     struct {
         const float *src;
         __nv_bfloat16 *hi, *lo;
@@ -693,14 +702,6 @@ int init_matrices(FieldSolver &f) {
         launch_split_bf16((int)nn, f.t, q.hi, q.lo, 0);
     }
     return AP_OK;
-}
-
-}  // namespace
-
-void launch_split_bf16(int n, const float *src, __nv_bfloat16 *hi, __nv_bfloat16 *lo, cudaStream_t st) {
-    int blocks = (n + 255) / 256;
-    if (blocks > 4096) blocks = 4096;
-    split_kernel<<<blocks, 256, 0, st>>>(n, src, hi, lo);
 }
 
 static bool field_fft_size(int m) {
@@ -732,7 +733,7 @@ void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cuda
     }
 }
 
-int field_solver_init(FieldSolver &f, int m, float bin_ratio, int want_bf16) {
+int field_solver_init(FieldSolver &f, int m, float bin_ratio) {
     f = FieldSolver();
     if (!field_fft_size(m)) return AP_ERR_UNSUPPORTED;
     f.m = m;
@@ -742,10 +743,6 @@ int field_solver_init(FieldSolver &f, int m, float bin_ratio, int want_bf16) {
         dmalloc(&f.u, 2 * nn))
         return AP_ERR_CUDA;
     fill_tables(f, 0);
-    if (want_bf16) {
-        const int r = init_matrices(f);
-        if (r != AP_OK) return r;
-    }
     // the solve's time for ap_solver_info (2 warm, 4 timed; the values do not
     // matter), on its own scratch: the map read is the first pass's output
     cudaEvent_t e0, e1;

@@ -1,7 +1,8 @@
 // Electrostatic field solve on the 5th-generation tensor cores (sm_103a).
 //
-// Same four contraction stages as the FP32 path (once dense contractions; now k_field_fft.cu, restating
-// replace::FFT::doFFT, python/AIEmath/fft_replace/fft.cpp:204-299), each
+// The solve of k_field_fft.cu (restating replace::FFT::doFFT, python/AIEmath/
+// fft_replace/fft.cpp:204-299) as four contractions with dense transform
+// matrices, each
 //   D[i][j] = sum_k A[i][k] B[j][k]
 // with A a constant transform matrix and B the data, both stored as a BF16
 // pair (hi = bf16(x), lo = bf16(x - hi)).  Every k-step issues three MMAs into
@@ -1305,7 +1306,9 @@ void run_variant(int v, FieldSolver &f, float *ex, float *ey, cudaStream_t st, c
 // The scratch outputs are overwritten.
 int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
     using namespace tc;
-    if (f.m < BM || (f.m % BM) != 0 || !f.C_hi) return AP_ERR_UNSUPPORTED;
+    if (f.m < BM || (f.m % BM) != 0) return AP_ERR_UNSUPPORTED;
+    const int mr = field_solver_matrices(f);
+    if (mr != AP_OK) return mr;
     TcState s{};
     if (!build_stage_maps(s.maps[0], f, d_hi, d_lo, Tile64::BN) ||
         !build_stage_maps(s.maps[1], f, d_hi, d_lo, Tile128::BN))
@@ -1365,7 +1368,10 @@ int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv
     // AP_TC_VARIANT=0..4 pins a candidate that ran (tests of each variant)
     if (const char *pin = getenv("AP_TC_VARIANT")) {
         const int v = atoi(pin);
-        if (v >= 0 && v < kTcVariants && f.tc_tune_ms[v] >= 0.f) f.tc_variant = v;
+        if (v >= 0 && v < kTcVariants && f.tc_tune_ms[v] >= 0.f) {
+            f.tc_variant = v;
+            f.tc_pinned = 1;
+        }
     }
     unsigned int st = 0;
     if (cudaMemcpy(&st, f.tc_status, sizeof(st), cudaMemcpyDeviceToHost) != cudaSuccess) return AP_ERR_CUDA;

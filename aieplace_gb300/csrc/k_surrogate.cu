@@ -68,8 +68,7 @@ __device__ __forceinline__ float bilinear_up(const float *c, int R, int f, int X
 // result goes to `coarse` (FP32) or, for the tensor-core coarse solve, to
 // its own hi/lo split (c_hi, c_lo).
 __global__ void pool_kernel(int M, int f, const float *d_f32, const __nv_bfloat16 *d_hi,
-                            const __nv_bfloat16 *d_lo, float *coarse, __nv_bfloat16 *c_hi, __nv_bfloat16 *c_lo,
-                            const int *gate, int mask) {
+                            const __nv_bfloat16 *d_lo, float *coarse, const int *gate, int mask) {
     if (!gate_open(gate, mask)) return;
     const int R = M / f;
     const float inv = 1.f / (float)(f * f);
@@ -81,14 +80,7 @@ __global__ void pool_kernel(int M, int f, const float *d_f32, const __nv_bfloat1
                 const size_t k = (size_t)(I * f + a) * M + (J * f + b);
                 s += d_f32 ? d_f32[k] : __bfloat162float(d_hi[k]) + __bfloat162float(d_lo[k]);
             }
-        const float v = s * inv;
-        if (c_hi) {
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            c_hi[q] = h;
-            c_lo[q] = __float2bfloat16_rn(v - __bfloat162float(h));
-        } else {
-            coarse[q] = v;
-        }
+        coarse[q] = s * inv;
     }
 }
 
@@ -767,25 +759,18 @@ int surr_state_init(SurrState &ss, const SurrNet &net, int M, float bin_ratio) {
         surr_state_free(ss);
         return AP_ERR_CUDA;
     }
-    // the coarse solve on the tensor cores when R allows 128-row tiles
-    const bool want_tc = R % 128 == 0;
-    int r = field_solver_init(ss.coarse, R, bin_ratio, want_tc ? 1 : 0);
+    int r = field_solver_init(ss.coarse, R, bin_ratio);
     if (r != AP_OK) {
         surr_state_free(ss);
         return r;
     }
-    if (want_tc && dmalloc(&ss.d_phi, RR) && dmalloc(&ss.d_plo, RR) &&
-        cudaMemset(ss.d_phi, 0, sizeof(__nv_bfloat16) * RR) == cudaSuccess &&
-        cudaMemset(ss.d_plo, 0, sizeof(__nv_bfloat16) * RR) == cudaSuccess &&
-        field_solver_bind_bf16(ss.coarse, ss.d_phi, ss.d_plo) == AP_OK)
-        ss.tc = 1;
     return AP_OK;
 }
 
 void surr_state_free(SurrState &ss) {
     if (ss.R) field_solver_free(ss.coarse);
     void *p[] = {ss.d_pool, ss.d_cex, ss.d_cey, ss.d_scale, ss.d_x0, ss.d_act[0], ss.d_act[1], ss.d_y,
-                 ss.d_sex, ss.d_sey, ss.d_part, ss.d_cnt, ss.d_phi, ss.d_plo};
+                 ss.d_sex, ss.d_sey, ss.d_part, ss.d_cnt};
     for (void *q : p)
         if (q) cudaFree(q);
     ss = SurrState{};
@@ -795,13 +780,8 @@ void surr_enqueue_input(const SurrNet &net, SurrState &ss, const float *d_f32, c
                         const __nv_bfloat16 *d_lo, const int *gate, int mask, cudaStream_t st, bool with_net_input) {
     const int R = ss.R, M = ss.M, f = net.f;
     const int g = grid_for((size_t)R * R);
-    if (ss.tc) {
-        sg::pool_kernel<<<g, 256, 0, st>>>(M, f, d_f32, d_hi, d_lo, nullptr, ss.d_phi, ss.d_plo, gate, mask);
-        field_solve_bf16x3(ss.coarse, ss.d_phi, ss.d_plo, ss.d_cex, ss.d_cey, st, gate, mask);
-    } else {
-        sg::pool_kernel<<<g, 256, 0, st>>>(M, f, d_f32, d_hi, d_lo, ss.d_pool, nullptr, nullptr, gate, mask);
-        field_solve_fp32(ss.coarse, ss.d_pool, ss.d_cex, ss.d_cey, st, gate, mask);
-    }
+    sg::pool_kernel<<<g, 256, 0, st>>>(M, f, d_f32, d_hi, d_lo, ss.d_pool, gate, mask);
+    field_solve_fp32(ss.coarse, ss.d_pool, ss.d_cex, ss.d_cey, st, gate, mask);
     sg::scale_kernel<<<g, 256, 0, st>>>(R, f, ss.d_cex, ss.d_cey, ss.d_part, ss.d_cnt + 0, ss.d_scale, gate, mask);
     if (with_net_input)
         sg::prep_kernel<<<g, 256, 0, st>>>(M, f, d_f32, d_hi, d_lo, ss.d_cex, ss.d_cey, ss.d_scale, ss.d_x0, gate,

@@ -45,10 +45,17 @@ UNIT = "iters/s"
 KERNELS_BESIDE_FIELD = 8
 
 
+def tensor_cores(solver: str) -> bool:
+    """Whether the field solve runs on the tensor cores (AP_TC_VARIANT pins a
+    candidate of the mixed-precision solver) and not as FP32 fast transforms."""
+    return solver == "bf16x3" and bool(os.environ.get("AP_TC_VARIANT"))
+
+
 def field_launches(info: dict, solver: str) -> int:
-    """Launches of one field solve: three FP32 passes; of the tensor-core solve
-    four stage launches, or one for its persistent candidates (3, 4)."""
-    if solver == "fp32":
+    """Launches of one field solve: three FP32 passes; of a tensor-core solve
+    that AP_TC_VARIANT pins four stage launches, or one for its persistent
+    candidates (3, 4)."""
+    if not tensor_cores(solver):
         return 3
     return 1 if info.get("tc_variant", -1) in (3, 4) else 4
 
@@ -72,7 +79,7 @@ def workload_desc(nl, preset):
     }
 
 
-def stage_model(nl):
+def stage_model(nl, solver):
     """Algorithmic bytes (HBM) or FLOPs per launch of each stage."""
     n_nodes = len(nl["node_w"])
     n_mov = int((nl["node_fixed"] == 0).sum())
@@ -88,8 +95,9 @@ def stage_model(nl):
         "density+overflow": ("hbm", 36 * m2),
         # net_ptr, pin_node, node positions, int64 gradient per movable node
         "wirelength": ("hbm", 4 * (e + 1) + 4 * p + 8 * n_nodes + 16 * n_mov),
-        # 6 dense m x m x m contractions (useful FLOPs)
-        "field": ("tensor", 12 * m3),
+        # density in, both fields out; pinned to the tensor cores: 6 dense
+        # m x m x m contractions (useful FLOPs)
+        "field": ("tensor", 12 * m3) if tensor_cores(solver) else ("hbm", 12 * m2),
         # bin record, int64 WA gradient read+clear, pins, charge, g_prev, g out; field maps
         "gather+control": ("hbm", 60 * n_mov + 8 * m2),
     }
@@ -608,7 +616,7 @@ def main():
     ttt = None
     cpu = None
     if rank == 0:
-        model = stage_model(nl)
+        model = stage_model(nl, solver)
         dom = max(range(len(stage_ms)), key=lambda i: stage_ms[i])
         bound, amount = model[STAGES[dom]]
         peaks = {}
@@ -660,7 +668,7 @@ def main():
             "metric": METRIC, "value": total_iters / t_max, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32+bf16x3" if solver == "bf16x3" else "f32", "data": "synthetic",
+            "dtype": "f32+bf16x3" if tensor_cores(solver) else "f32", "data": "synthetic",
             "config": {**workload_desc(nl, args.preset), "field_solver": solver,
                        "step": "one trial step (one gradient evaluation); value counts accepted iterations",
                        "parallelism": "replicas" if world > 1 else "single"},

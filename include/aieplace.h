@@ -47,7 +47,11 @@ enum {
 /* ---- field solvers ----------------------------------------------------- */
 enum {
     AP_FIELD_FP32 = 0,   /* fast per-axis transforms, FP32 */
-    AP_FIELD_BF16X3 = 1  /* dense per-axis transforms, tcgen05 BF16 x3 split, FP32 accumulate */
+    /* mixed precision allowed; bins a multiple of 128.  Runs the FP32 fast
+     * transforms, which are the faster and the more exact at every grid, unless
+     * AP_TC_VARIANT (ap_solver_info) pins the tensor-core solve: dense per-axis
+     * transforms, tcgen05 BF16 x3 split, FP32 accumulate */
+    AP_FIELD_BF16X3 = 1
 };
 
 /* Netlist in CSR form.  Replaces the object graph the reference builds from
@@ -175,8 +179,8 @@ int ap_profile_stages(ap_handle *h, int32_t n_trials, float *stage_ms, int32_t *
  * drain are counted in a {"lost_trials": n} line.  path NULL stops logging. */
 int ap_set_log(ap_handle *h, const char *path, int32_t capacity);
 
-/* Tile shapes the autotuner picked at ap_create for this bin count, and the
- * solve times it measured: tc_variant is the tensor-core candidate (0: four
+/* Tile shapes the autotuner picked for this bin count, and the solve times it
+ * measured (the tensor-core solve's on the first call that needs them): tc_variant is the tensor-core candidate (0: four
  * launches of 128 x 64 tiles, 4 pipeline stages; 1: 128 x 128, 3 stages; 2:
  * 128 x 64, 2 stages, two CTAs per SM; 3: one persistent launch over the four
  * stages' 128 x 128 tiles, K of the first two stages split in two; 4: the
@@ -185,7 +189,7 @@ int ap_set_log(ap_handle *h, const char *path, int32_t capacity);
  * 256 threads, 64: 512 threads); tc_ms[5] the candidates' times, simt_ms[0]
  * or [1] the FP32 solve's by its block (-1: not run).  The
  * environment variable AP_TC_VARIANT=0..4, read at ap_create, pins a
- * candidate that ran instead of the fastest (for testing each one). */
+ * candidate: the mixed-precision solver then runs it (for testing each one). */
 int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *simt_tile, float *simt_ms);
 
 /* Iterates until overflow < params.target_overflow or max_iterations;
