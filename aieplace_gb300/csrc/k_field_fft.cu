@@ -26,10 +26,12 @@
 // block from 256 points up.  T and U are kept in tiles of a few rows,
 // T[x/4][v][x%4] and U[x/2][v][x%2] (ux, uy), so that the passes along y
 // read and write whole rows of tiles and the pass along x whole 32-byte
-// sectors.  Measured (m = 1024, launches alone under ncu): 6.8 + 15.1 + 8.7 us;
-// a 2M-cell loop's iteration 755 us with the matrices' 460 us solve, 240 with
-// this one; 200k cells, m = 512: 210 and 79 us; 32 instances of 128 and 256
-// bins in the persistent launch: 8.62 and 7.29 ms for ten steps and the positions' read-back.
+// sectors; within 64 registers a thread, so that every block of a pass is
+// resident at once (72: 15.1 us for P2, a second wave).  Measured (m = 1024,
+// launches alone under ncu): 6.3 + 13.7 + 9.0 us, shared memory 61-77% busy;
+// a 2M-cell loop's iteration 727 us with the matrices' 460 us solve, 234 with
+// this one; 200k cells, m = 512: 208 and 79 us; 32 instances of 128 and 256
+// bins in the persistent launch: 8.57 and 6.92 ms for ten steps and the positions' read-back.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -211,6 +213,9 @@ __device__ __forceinline__ void dft(float2 (&v)[R]) {
 // A block of NT threads holds S = NT / (m / E) FFTs ("slots"), slot `slot`'s
 // points at sm + slot * fft_slot(m), element i at fft_pad(i) (no bank
 // conflicts at the stages' power-of-two strides).
+// No sum of two indices below carries into bit 4 (one of them is a multiple of
+// the stride that bounds the other), so fft_pad(i + c) = fft_pad(i) + fft_pad(c)
+// and a constant c becomes an offset of the access.
 __host__ __device__ constexpr int fft_pad(int i) { return i + (i >> 4); }
 __host__ __device__ constexpr int fft_slot(int m) { return m + m / 16; }
 __host__ __device__ constexpr int fft_slots(int m, int nt) { return nt / fft_threads(m); }
@@ -228,51 +233,59 @@ __device__ __forceinline__ void fft_sync() {
         __syncthreads();
 }
 
-// Stage ST onwards of the FFT of x[q] = element j + q m/E; the result comes
-// back in the same order.  Stockham: the output of butterfly jj, point r goes
-// to (jj / ns) ns R + jj % ns + r ns.
-template <int M, bool INV, int ST>
-__device__ __forceinline__ void fft_stage(float2 (&x)[fft_points(M)], float2 *sm, int j, const float2 *tw) {
-    constexpr int E = fft_points(M), TPF = M / E, R = fft_radix(M, ST), NS = fft_ns(M, ST), B = E / R;
-    static_assert(E % R == 0, "whole butterflies per thread");
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-        const int k = (j + b * TPF) % NS;
-        float2 v[R];
-        v[0] = x[b];
-#pragma unroll
-        for (int r = 1; r < R; ++r) {
-            v[r] = x[b + r * B];
-            if constexpr (NS > 1) v[r] = twiddle<INV>(v[r], __ldg(tw + fft_tw_off(M, ST) + (r - 1) * NS + k));
-        }
-        dft<R, INV>(v);
-#pragma unroll
-        for (int r = 0; r < R; ++r) x[b + r * B] = v[r];
-    }
-    if constexpr (NS * R < M) {
-        fft_sync<M>();  // every earlier read of the slot is done
-#pragma unroll
-        for (int b = 0; b < B; ++b) {
-            const int jj = j + b * TPF, o = (jj / NS) * (NS * R) + jj % NS;
-#pragma unroll
-            for (int r = 0; r < R; ++r) sm[fft_pad(o + r * NS)] = x[b + r * B];
-        }
-        fft_sync<M>();
-#pragma unroll
-        for (int q = 0; q < E; ++q) x[q] = sm[fft_pad(j + q * TPF)];
-        fft_stage<M, INV, ST + 1>(x, sm, j, tw);
-    }
-}
-
 template <int M>
 __device__ __forceinline__ void slot_load(float2 (&x)[fft_points(M)], const float2 *sm, int j) {
+    sm += fft_pad(j);
 #pragma unroll
-    for (int q = 0; q < fft_points(M); ++q) x[q] = sm[fft_pad(j + q * fft_threads(M))];
+    for (int q = 0; q < fft_points(M); ++q) x[q] = sm[fft_pad(q * fft_threads(M))];
 }
 template <int M>
 __device__ __forceinline__ void slot_store(const float2 (&x)[fft_points(M)], float2 *sm, int j) {
+    sm += fft_pad(j);
 #pragma unroll
-    for (int q = 0; q < fft_points(M); ++q) sm[fft_pad(j + q * fft_threads(M))] = x[q];
+    for (int q = 0; q < fft_points(M); ++q) sm[fft_pad(q * fft_threads(M))] = x[q];
+}
+
+// Stage ST onwards of the FFT of x[q] = element j + q m/E; the result comes
+// back in the same order.  Stockham: the output of butterfly jj, point r goes
+// to (jj / ns) ns R + jj % ns + r ns.  `on`: false for the threads of a slot
+// without work, which only meet the barriers.
+template <int M, bool INV, int ST>
+__device__ __forceinline__ void fft_stage(float2 (&x)[fft_points(M)], float2 *sm, int j, const float2 *tw,
+                                          bool on = true) {
+    constexpr int E = fft_points(M), TPF = M / E, R = fft_radix(M, ST), NS = fft_ns(M, ST), B = E / R;
+    static_assert(E % R == 0, "whole butterflies per thread");
+    if (on) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const float2 *w = tw + fft_tw_off(M, ST) + (j + b * TPF) % NS;
+            float2 v[R];
+            v[0] = x[b];
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+                v[r] = x[b + r * B];
+                if constexpr (NS > 1) v[r] = twiddle<INV>(v[r], __ldg(w + (r - 1) * NS));
+            }
+            dft<R, INV>(v);
+#pragma unroll
+            for (int r = 0; r < R; ++r) x[b + r * B] = v[r];
+        }
+    }
+    if constexpr (NS * R < M) {
+        fft_sync<M>();  // every earlier read of the slot is done
+        if (on) {
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const int jj = j + b * TPF;
+                float2 *o = sm + fft_pad((jj / NS) * (NS * R) + jj % NS);
+#pragma unroll
+                for (int r = 0; r < R; ++r) o[fft_pad(r * NS)] = x[b + r * B];
+            }
+        }
+        fft_sync<M>();
+        if (on) slot_load<M>(x, sm, j);
+        fft_stage<M, INV, ST + 1>(x, sm, j, tw, on);
+    }
 }
 
 // the two real lines a + i b behind one complex DFT: cosine coefficients of
@@ -346,11 +359,8 @@ __device__ __forceinline__ void fft_columns(const FieldRec &a, int vb, float2 *s
     __syncthreads();
     float2 x[E];
     const bool fwd = slot < P && vb * P + slot < M / 2;
-#pragma unroll
-    for (int q = 0; q < E; ++q) x[q] = make_float2(0.f, 0.f);
     if (fwd) slot_load<M>(x, sm + slot * SL, j);
-    // the idle slots run along on zeros (the barriers are the block's)
-    fft_stage<M, false, 0>(x, sm + slot * SL, j, a.tab);
+    fft_stage<M, false, 0>(x, sm + slot * SL, j, a.tab, fwd);
     __syncthreads();
     if (fwd) slot_store<M>(x, sm + slot * SL, j);
     __syncthreads();
@@ -575,7 +585,7 @@ __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.la
 __device__ __forceinline__ bool gated_off(const int *gate, int mask) { return gate && !((1 << *gate) & mask); }
 
 template <int M, int NT, int PASS>
-__global__ void __launch_bounds__(NT) fft_kernel(FieldRec a, const int *gate, int mask) {
+__global__ void __launch_bounds__(NT, odd_part(M) == 1 && M <= 2048 ? 1024 / NT : 1) fft_kernel(FieldRec a, const int *gate, int mask) {
     extern __shared__ __align__(16) float2 fft_sm[];
     if (PASS < 2) grid_release();
     if (PASS > 0) grid_wait();
@@ -817,7 +827,7 @@ __device__ __forceinline__ void fft_record(const FieldRec &r, int vb, float2 *sm
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT) persist_field_kernel(PersistQueue q, const FieldRec *recs) {
+__global__ void __launch_bounds__(NT, 1024 / NT) persist_field_kernel(PersistQueue q, const FieldRec *recs) {
     extern __shared__ __align__(16) float2 persist_sm[];
     persist_loop(q, recs, [](const FieldRec &r, VBlock vb, int) {
         switch (r.m) {
