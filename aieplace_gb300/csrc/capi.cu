@@ -81,7 +81,8 @@ struct ap_handle {
     unsigned int *d_counters = nullptr;
     double *d_out = nullptr;
     double *h_out = nullptr;  // pinned [4]
-    unsigned int *h_status = nullptr;  // pinned: the tensor-core solve's status word, read by sync()
+    // pinned: [0] the tensor-core solve's status word, read by sync(); [1] import_positions' flag
+    unsigned int *h_status = nullptr;
     int bucket_lo[kWaBuckets + 1] = {};
     FieldSolver fs{};
     cudaStream_t stream = nullptr;
@@ -105,6 +106,12 @@ struct ap_handle {
     cudaStream_t copy_in = nullptr;
     cudaEvent_t ev_start = nullptr, ev_in[4] = {nullptr, nullptr, nullptr, nullptr};
     float *d_ix = nullptr, *d_iy = nullptr;
+    // calls on host arrays in netlist order: internal node -> netlist node
+    // (null: the same), and kIo arrays of n_io floats that the copies go
+    // through (made on first use)
+    int *d_int2ext = nullptr;
+    float *d_io = nullptr;
+    size_t n_io = 0;
     ap_surrogate_policy policy{0.3f, 8, 0.02f, 1};
     // trajectory log: device ring of per-trial records, drained into `log`
     // (JSON lines) whenever the scalars are read
@@ -450,24 +457,148 @@ int build_graphs(ap_handle *h) {
     return AP_OK;
 }
 
-// external-order host arrays -> internal positions of buffer `at` (movable
+// ---- host arrays in netlist order ------------------------------------------------
+// The caller's arrays are copied as they are; the order, the die's offset,
+// the check for finite values and the fixed point's conversion are kernels.
+// (As loops over vectors on the host they were most of these calls: the four
+// stage calls on 200k cells 3.9 ms, 1.0 now; a field solve of 1024^2 bins 1.31
+// ms, 0.30 now; reading back 32 designs' positions 2.3 ms, 1.7 now.)
+constexpr int kIo = 6;  // 0-3: netlist order, in or out; 4, 5: internal order
+
+int ensure_io(ap_handle *h) {
+    if (h->d_io) return AP_OK;
+    h->n_io = (size_t)std::max(std::max(h->n_ext, h->n_mov), 1);
+    CK(dalloc(&h->d_io, kIo * h->n_io));
+    if (!h->identity && !h->d_int2ext) {
+        CK(dalloc(&h->d_int2ext, (size_t)h->n_nodes));
+        CK(cudaMemcpy(h->d_int2ext, h->int2ext.data(), sizeof(int) * h->n_nodes, cudaMemcpyHostToDevice));
+    }
+    return AP_OK;
+}
+
+int node_blocks(int n) { return std::max(1, std::min((n + kThreads - 1) / kThreads, 4096)); }
+
+// internal nodes [0, n): positions relative to the die's corner; filler cells
+// (no netlist node) at 0; *bad set if one is not finite
+__global__ void import_kernel(int n, const int *__restrict__ int2ext, const float *__restrict__ x,
+                              const float *__restrict__ y, float xl, float yl, float *ix, float *iy,
+                              unsigned int *bad) {
+    bool b = false;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int e = int2ext ? __ldg(int2ext + i) : i;
+        float vx = 0.f, vy = 0.f;
+        if (e >= 0) {
+            vx = __fsub_rn(x[e], xl);
+            vy = __fsub_rn(y[e], yl);
+            b = b || !isfinite(vx) || !isfinite(vy);
+        }
+        ix[i] = vx;
+        iy[i] = vy;
+    }
+    if (b) *bad = 1u;
+}
+
+// Host positions of internal nodes [0, n) -> dx, dy; AP_ERR_NONFINITE (with
+// only dx, dy written) if one is not finite.
+int import_positions(ap_handle *h, int n, const float *x, const float *y, float *dx, float *dy) {
+    int r = ensure_io(h);
+    if (r != AP_OK) return r;
+    float *ex = h->d_io, *ey = h->d_io + h->n_io;
+    unsigned int *bad = h->d_counters + 4;
+    CK(cudaMemcpyAsync(ex, x, sizeof(float) * h->n_ext, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(ey, y, sizeof(float) * h->n_ext, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemsetAsync(bad, 0, sizeof(*bad), h->stream));
+    import_kernel<<<node_blocks(n), kThreads, 0, h->stream>>>(n, h->d_int2ext, ex, ey, h->die_xl, h->die_yl, dx, dy,
+                                                              bad);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h->h_status + 1, bad, sizeof(*bad), cudaMemcpyDeviceToHost, h->stream));
+    r = sync(h);
+    return r != AP_OK ? r : h->h_status[1] ? AP_ERR_NONFINITE : AP_OK;
+}
+
+// netlist-order host arrays -> internal positions of buffer `at` (movable
 // nodes only; fixed nodes keep their place)
 int upload_positions(ap_handle *h, int at, const float *x, const float *y) {
-    std::vector<float> ix((size_t)h->n_mov), iy((size_t)h->n_mov);
-    for (int i = 0; i < h->n_mov; ++i) {
-        const int e = h->int2ext[(size_t)i];
-        if (e < 0) {  // filler cells start where ap_create put them
-            ix[(size_t)i] = h->fill_x0[(size_t)(i - h->n_real)];
-            iy[(size_t)i] = h->fill_y0[(size_t)(i - h->n_real)];
-            continue;
-        }
-        ix[(size_t)i] = x[e] - h->die_xl;
-        iy[(size_t)i] = y[e] - h->die_yl;
-        if (!std::isfinite(ix[(size_t)i]) || !std::isfinite(iy[(size_t)i])) return AP_ERR_NONFINITE;
+    const int r = import_positions(h, h->n_mov, x, y, h->d_sx, h->d_sy);
+    if (r != AP_OK) return r;
+    CK(cudaMemcpyAsync(h->d_px[at], h->d_sx, sizeof(float) * h->n_real, cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->d_py[at], h->d_sy, sizeof(float) * h->n_real, cudaMemcpyDeviceToDevice, h->stream));
+    if (h->n_fill) {  // filler cells start where ap_create put them
+        const size_t b = sizeof(float) * (size_t)h->n_fill;
+        CK(cudaMemcpyAsync(h->d_px[at] + h->n_real, h->fill_x0.data(), b, cudaMemcpyHostToDevice, h->stream));
+        CK(cudaMemcpyAsync(h->d_py[at] + h->n_real, h->fill_y0.data(), b, cudaMemcpyHostToDevice, h->stream));
     }
-    CK(cudaMemcpyAsync(h->d_px[at], ix.data(), sizeof(float) * h->n_mov, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_py[at], iy.data(), sizeof(float) * h->n_mov, cudaMemcpyHostToDevice, h->stream));
     return sync(h);
+}
+
+// positions of the accepted buffer, netlist order and die coordinates
+__global__ void export_positions_kernel(int n, const int *__restrict__ int2ext, const DevScalars *sc, const float *x0,
+                                        const float *y0, const float *x1, const float *y1, float xl, float yl,
+                                        float *ox, float *oy) {
+    const int cur = sc->cur;
+    const float *x = cur ? x1 : x0, *y = cur ? y1 : y0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int e = int2ext ? __ldg(int2ext + i) : i;
+        if (e < 0) continue;  // filler cells are internal
+        ox[e] = __fadd_rn(x[i], xl);
+        oy[e] = __fadd_rn(y[i], yl);
+    }
+}
+
+// The WA gradient accumulators -> float, netlist order (packed halves, y 2^32
+// + x, plus the per-axis sums of nodes of many pins); cleared.
+__global__ void export_gradient_kernel(int n, const int *__restrict__ int2ext, ull *gq, ull *gqx, ull *gqy, float *ox,
+                                       float *oy) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int e = int2ext ? __ldg(int2ext + i) : i;
+        long long sx, sy;
+        unpack_q(gq[i], sx, sy);
+        sx += (long long)gqx[i];
+        sy += (long long)gqy[i];
+        gq[i] = gqx[i] = gqy[i] = 0ull;
+        if (e < 0) continue;
+        ox[e] = i64_to_float(sx) * kInvGradScale;  // exact power-of-two scaling
+        oy[e] = i64_to_float(sy) * kInvGradScale;
+    }
+}
+
+// per-node values of movable nodes (internal order) -> netlist order, 0 for
+// the other nodes; gx null: forces only
+__global__ void export_force_kernel(int n, int n_mov, const int *__restrict__ int2ext, const float *fx, const float *fy,
+                                    const float *gx, const float *gy, float *ofx, float *ofy, float *ogx, float *ogy) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int e = int2ext ? __ldg(int2ext + i) : i;
+        if (e < 0) continue;
+        const bool mov = i < n_mov;
+        ofx[e] = mov ? fx[i] : 0.f;
+        ofy[e] = mov ? fy[i] : 0.f;
+        if (gx) {
+            ogx[e] = mov ? gx[i] : 0.f;
+            ogy[e] = mov ? gy[i] : 0.f;
+        }
+    }
+}
+
+// the mean of a map (sums in FP64, blocks folded in order by the last one)
+__global__ void __launch_bounds__(kThreads) mean_kernel(int n, const float *__restrict__ d, double *partials,
+                                                        unsigned int *counter, float *mean) {
+    __shared__ double red[32];
+    double s = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += (double)d[i];
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (arrive_last(counter, gridDim.x)) {
+        const double t = reduce_partials(partials, gridDim.x, red);
+        if (threadIdx.x == 0) {
+            *mean = (float)(t / (double)n);
+            *counter = 0u;
+        }
+    }
+}
+
+__global__ void subtract_kernel(int n, float *d, const float *mean) {
+    const float m = *mean;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) d[i] = __fsub_rn(d[i], m);
 }
 
 // Writes the trajectory records of the trials run since the last drain (the
@@ -941,7 +1072,7 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(dalloc(&h->d_out, 8));
     A(cudaMallocHost((void **)&h->h_sc, sizeof(DevScalars)));
     A(cudaMallocHost((void **)&h->h_out, sizeof(double) * 8));
-    A(cudaMallocHost((void **)&h->h_status, sizeof(unsigned int)));
+    A(cudaMallocHost((void **)&h->h_status, 2 * sizeof(unsigned int)));
     // the WA launches run beside the density chain (scatter -> rho -> field)
     // at the same priority: with the chain's stream at the highest priority a
     // 2M-cell trial took 1.5% longer (its blocks kept the WA blocks waiting
@@ -1064,7 +1195,7 @@ int ap_destroy(ap_handle *h) {
                     h->d_mov_q,   h->d_fill_q,   h->d_fix_q,  h->d_fixs_q,  h->d_dens,  h->d_ex,    h->d_ey,
                     h->d_dens_hi, h->d_dens_lo,  h->d_sx,     h->d_sy,      h->d_sc,    h->d_partials,
                     h->d_partials_ll, h->d_counters, h->d_out, h->d_rec_bin, h->d_rec_ov, h->d_gq,
-                    h->d_ix,      h->d_iy,       h->d_xy_loop, h->d_xy_tmp, h->d_whq};
+                    h->d_ix,      h->d_iy,       h->d_xy_loop, h->d_xy_tmp, h->d_whq, h->d_int2ext, h->d_io};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (h->h_sc) cudaFreeHost(h->h_sc);
@@ -1259,19 +1390,16 @@ int ap_get_positions(ap_handle *h, float *x, float *y) {
     if (!h || !x || !y) return AP_ERR_INVALID_ARG;
     int r = read_scalars(h);
     if (r != AP_OK) return r;
-    const int cur = h->h_sc->cur;
-    std::vector<float> ix((size_t)h->n_nodes), iy((size_t)h->n_nodes);
-    CK(cudaMemcpyAsync(ix.data(), h->d_px[cur], sizeof(float) * h->n_nodes, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(iy.data(), h->d_py[cur], sizeof(float) * h->n_nodes, cudaMemcpyDeviceToHost, h->stream));
-    r = sync(h);
+    r = ensure_io(h);
     if (r != AP_OK) return r;
-    for (int i = 0; i < h->n_nodes; ++i) {
-        const int e = h->int2ext[(size_t)i];
-        if (e < 0) continue;  // filler cells are internal
-        x[e] = ix[(size_t)i] + h->die_xl;
-        y[e] = iy[(size_t)i] + h->die_yl;
-    }
-    return AP_OK;
+    float *ox = h->d_io, *oy = h->d_io + h->n_io;
+    export_positions_kernel<<<node_blocks(h->n_nodes), kThreads, 0, h->stream>>>(
+        h->n_nodes, h->d_int2ext, h->d_sc, h->d_px[0], h->d_py[0], h->d_px[1], h->d_py[1], h->die_xl, h->die_yl, ox,
+        oy);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(x, ox, sizeof(float) * h->n_ext, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(y, oy, sizeof(float) * h->n_ext, cudaMemcpyDeviceToHost, h->stream));
+    return sync(h);
 }
 
 int ap_step_host(ap_handle *h, const float *x_in, const float *y_in, float *x_out, float *y_out,
@@ -1420,23 +1548,10 @@ int ap_overflow(ap_handle *h, double *overflow, double *overflow_abs) {
 // ---- per-stage entry points ----------------------------------------------
 
 namespace {
-// external-order positions of all nodes -> internal scratch (d_sx, d_sy)
+// netlist-order positions of all nodes -> internal scratch (d_sx, d_sy);
+// filler cells anywhere (no per-stage result depends on them)
 int stage_positions(ap_handle *h, const float *x, const float *y) {
-    std::vector<float> ix((size_t)h->n_nodes), iy((size_t)h->n_nodes);
-    for (int i = 0; i < h->n_nodes; ++i) {
-        const int e = h->int2ext[(size_t)i];
-        if (e < 0) {  // filler cells: their starting points (no per-stage result depends on them)
-            ix[(size_t)i] = h->fill_x0[(size_t)(i - h->n_real)];
-            iy[(size_t)i] = h->fill_y0[(size_t)(i - h->n_real)];
-            continue;
-        }
-        ix[(size_t)i] = x[e] - h->die_xl;
-        iy[(size_t)i] = y[e] - h->die_yl;
-        if (!std::isfinite(ix[(size_t)i]) || !std::isfinite(iy[(size_t)i])) return AP_ERR_NONFINITE;
-    }
-    CK(cudaMemcpyAsync(h->d_sx, ix.data(), sizeof(float) * h->n_nodes, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->d_sy, iy.data(), sizeof(float) * h->n_nodes, cudaMemcpyHostToDevice, h->stream));
-    return sync(h);
+    return import_positions(h, h->n_nodes, x, y, h->d_sx, h->d_sy);
 }
 }  // namespace
 
@@ -1451,26 +1566,15 @@ int ap_wirelength_grad(ap_handle *h, const float *x, const float *y, float gamma
     CK(cudaMemsetAsync(h->d_gqy, 0, sizeof(ull) * N, h->stream));
     launch_wirelength(wa_args(h, h->d_sx, h->d_sy, gamma, h->n_nodes, WA_OUT_ONLY, h->d_out), h->stream);
     CK(cudaGetLastError());
-    std::vector<unsigned long long> q(N), qx(N), qy(N);
-    CK(cudaMemcpyAsync(q.data(), h->d_gq, sizeof(ull) * N, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(qx.data(), h->d_gqx, sizeof(ull) * N, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(qy.data(), h->d_gqy, sizeof(ull) * N, cudaMemcpyDeviceToHost, h->stream));
+    float *ox = h->d_io, *oy = h->d_io + h->n_io;
+    export_gradient_kernel<<<node_blocks(h->n_nodes), kThreads, 0, h->stream>>>(
+        h->n_nodes, h->d_int2ext, h->d_gq, h->d_gqx, h->d_gqy, ox, oy);
+    CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h->h_out, h->d_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemsetAsync(h->d_gq, 0, sizeof(ull) * N, h->stream));
-    CK(cudaMemsetAsync(h->d_gqx, 0, sizeof(ull) * N, h->stream));
-    CK(cudaMemsetAsync(h->d_gqy, 0, sizeof(ull) * N, h->stream));
+    CK(cudaMemcpyAsync(gx, ox, sizeof(float) * h->n_ext, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(gy, oy, sizeof(float) * h->n_ext, cudaMemcpyDeviceToHost, h->stream));
     r = sync(h);
     if (r != AP_OK) return r;
-    for (size_t i = 0; i < N; ++i) {
-        // packed halves (y 2^32 + x, x the signed low word) plus the per-axis sums
-        const long long lo = (long long)(int32_t)(uint32_t)q[i];
-        const long long sx = lo + (long long)qx[i];
-        const long long sy = (((long long)q[i] - lo) >> 32) + (long long)qy[i];
-        const int e = h->int2ext[i];
-        if (e < 0) continue;
-        gx[e] = (float)ldexp((double)sx, -20);  // kGradScale = 2^20
-        gy[e] = (float)ldexp((double)sy, -20);
-    }
     if (hpwl) *hpwl = h->h_out[0];
     if (wa) *wa = h->h_out[1];
     return AP_OK;
@@ -1507,12 +1611,11 @@ int ap_field_solve(ap_handle *h, const float *density, float *ex, float *ey, int
     if (sv == AP_FIELD_BF16X3 && h->fs.m % 128 != 0) return AP_ERR_UNSUPPORTED;
     // the field does not depend on the map's mean (phi_00 = 0); taking it off
     // keeps the transforms' DC sums from swamping the AC terms in rounding
-    double mean = 0.0;
-    for (int b = 0; b < nb; ++b) mean += (double)density[b];
-    mean /= (double)nb;
-    std::vector<float> shifted((size_t)nb);
-    for (int b = 0; b < nb; ++b) shifted[(size_t)b] = density[b] - (float)mean;
-    CK(cudaMemcpyAsync(h->d_dens, shifted.data(), sizeof(float) * nb, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->d_dens, density, sizeof(float) * nb, cudaMemcpyHostToDevice, h->stream));
+    float *mean = reinterpret_cast<float *>(h->d_out + 4);
+    mean_kernel<<<std::min(node_blocks(nb), 512), kThreads, 0, h->stream>>>(nb, h->d_dens, h->d_partials,
+                                                                           h->d_counters + 5, mean);
+    subtract_kernel<<<node_blocks(nb), kThreads, 0, h->stream>>>(nb, h->d_dens, mean);
     if (on_tensor_cores(h, sv)) launch_split_bf16(nb, h->d_dens, h->d_dens_hi, h->d_dens_lo, h->stream);
     int r = run_field(h, sv, h->stream);
     if (r != AP_OK) return r;
@@ -1529,15 +1632,13 @@ int ap_node_force(ap_handle *h, const float *x, const float *y, const float *ex,
     if (grad && (!(gamma > 0.f) || !(lambda >= 0.f) || !std::isfinite(lambda))) return AP_ERR_INVALID_ARG;
     int r = stage_positions(h, x, y);
     if (r != AP_OK) return r;
-    const size_t nb = (size_t)h->p.bins_x * h->p.bins_y, N = (size_t)h->n_nodes, M = (size_t)h->n_mov;
+    const size_t nb = (size_t)h->p.bins_x * h->p.bins_y, N = (size_t)h->n_nodes;
     CK(cudaMemcpyAsync(h->d_ex, ex, sizeof(float) * nb, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_ey, ey, sizeof(float) * nb, cudaMemcpyHostToDevice, h->stream));
     // the bin records of this point, as a loop trial's position update makes
     // them, so that the gather below runs the loop's record path
     launch_records(h->g, h->n_mov, h->d_sx, h->d_sy, h->d_w, h->d_h, h->d_rec_bin, h->d_rec_ov, h->stream);
-    float *d_g = nullptr;
     if (grad) {
-        CK(cudaMallocAsync((void **)&d_g, sizeof(float) * 2 * std::max<size_t>(M, 1), h->stream));
         CK(cudaMemsetAsync(h->d_gq, 0, sizeof(ull) * N, h->stream));
         CK(cudaMemsetAsync(h->d_gqx, 0, sizeof(ull) * N, h->stream));
         CK(cudaMemsetAsync(h->d_gqy, 0, sizeof(ull) * N, h->stream));
@@ -1551,35 +1652,18 @@ int ap_node_force(ap_handle *h, const float *x, const float *y, const float *ex,
     a.fx = h->d_ix;  // host-step input staging, n_mov floats each
     a.fy = h->d_iy;
     a.lambda = lambda;
-    a.gxo = grad ? d_g : nullptr;
-    a.gyo = grad ? d_g + M : nullptr;
-    launch_gather(a, h->stream);
-    const cudaError_t le = cudaGetLastError();
-    std::vector<float> hf(2 * std::max<size_t>(M, 1)), hg(grad ? 2 * std::max<size_t>(M, 1) : 0);
-    cudaError_t ce = cudaSuccess;
-    if (M) {
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(hf.data(), h->d_ix, sizeof(float) * M, cudaMemcpyDeviceToHost, h->stream);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(hf.data() + M, h->d_iy, sizeof(float) * M, cudaMemcpyDeviceToHost, h->stream);
-        if (grad && ce == cudaSuccess)
-            ce = cudaMemcpyAsync(hg.data(), d_g, sizeof(float) * 2 * M, cudaMemcpyDeviceToHost, h->stream);
-    }
-    if (d_g) cudaFreeAsync(d_g, h->stream);
-    CK(le);
-    CK(ce);
-    r = sync(h);
-    if (r != AP_OK) return r;
-    for (size_t i = 0; i < N; ++i) {
-        const int e = h->int2ext[i];
-        if (e < 0) continue;
-        const bool mov = i < M;
-        fx[e] = mov ? hf[i] : 0.f;
-        fy[e] = mov ? hf[M + i] : 0.f;
-        if (grad) {
-            gx[e] = mov ? hg[i] : 0.f;
-            gy[e] = mov ? hg[M + i] : 0.f;
-        }
-    }
-    return AP_OK;
+    float *io[kIo];
+    for (int k = 0; k < kIo; ++k) io[k] = h->d_io + k * h->n_io;
+    a.gxo = grad ? io[4] : nullptr;
+    a.gyo = grad ? io[5] : nullptr;
+    if (h->n_mov > 0) launch_gather(a, h->stream);
+    export_force_kernel<<<node_blocks(h->n_nodes), kThreads, 0, h->stream>>>(
+        h->n_nodes, h->n_mov, h->d_int2ext, h->d_ix, h->d_iy, a.gxo, a.gyo, io[0], io[1], io[2], io[3]);
+    CK(cudaGetLastError());
+    float *out[4] = {fx, fy, gx, gy};
+    for (int k = 0; k < (grad ? 4 : 2); ++k)
+        CK(cudaMemcpyAsync(out[k], io[k], sizeof(float) * h->n_ext, cudaMemcpyDeviceToHost, h->stream));
+    return sync(h);
 }
 
 int ap_debug_inject(ap_handle *h, int32_t kind, int64_t wait_ns) {
