@@ -155,6 +155,7 @@ struct GatherArgs {
     float *vx[2], *vy[2];   // evaluation point [at], comparison point [1 - at]
     const float *w, *h;
     const float *ex, *ey;   // field per bin
+    const float2 *exy;      // GATHER_STEP: the field as (ex, ey) pairs, or null
     ull *gq;                // WA gradient accumulators, packed (cleared after reading)
     ull *gqx, *gqy;         // per-axis accumulators of nodes of more than kPackMaxPins pins
     const float *pins;      // pin count per movable node
@@ -230,8 +231,9 @@ void field_solver_free(FieldSolver &f);
 // density d (x-major) -> ex, ey; FP32 fast transforms
 // gate: the launches run only if gate is null or (1 << *gate) & gate_mask
 // (the loop's surrogate schedule lives in device memory)
+// exy: the field as (ex, ey) pairs here instead of in ex, ey (or null)
 void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cudaStream_t st,
-                      const int *gate = nullptr, int gate_mask = 0);
+                      const int *gate = nullptr, int gate_mask = 0, float2 *exy = nullptr);
 // Builds the TMA tensor maps of the tcgen05 path with (d_hi, d_lo) as the
 // density input; needs m a multiple of 128.
 int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo);
@@ -269,7 +271,8 @@ int wa_plan(WaArgs &a);
 struct FieldRec {
     const float *d;       // P1 in: the density map
     float *t, *u;         // between the passes
-    float *ex, *ey;       // P3 out
+    float *ex, *ey;       // P3 out, or
+    float2 *exy;          // (ex, ey) pairs
     const float2 *tab;
     const float *wx, *wy;
     float scale;          // 4 / m^2
@@ -280,7 +283,8 @@ struct FieldRec {
 // the passes of field_solve_fp32(f, d, ex, ey) as four records (P3 in two
 // halves) for blocks of 8 tile threads; false if a block of the tile is too
 // small for the grid (tile 32: more than 1024 bins)
-bool field_records(const FieldSolver &f, const float *d, float *ex, float *ey, int tile, FieldRec rec[4]);
+// (the field as (ex, ey) pairs)
+bool field_records(const FieldSolver &f, const float *d, float2 *exy, int tile, FieldRec rec[4]);
 int field_rec_blocks(const FieldRec &r, int tile);
 
 // one persistent launch of a stage over the records `recs` (device memory)

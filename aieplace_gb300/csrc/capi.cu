@@ -72,6 +72,7 @@ struct ap_handle {
     ull *d_fill_q = nullptr;  // filler cells' map: in the field, not in the overflow
     long long *d_fix_q = nullptr, *d_fixs_q = nullptr;
     float *d_dens = nullptr, *d_ex = nullptr, *d_ey = nullptr;
+    float2 *d_exy = nullptr;  // a loop trial's field as pairs (loop_pairs)
     __nv_bfloat16 *d_dens_hi = nullptr, *d_dens_lo = nullptr;
     float *d_sx = nullptr, *d_sy = nullptr;  // staging (external order / scratch positions)
     DevScalars *d_sc = nullptr;
@@ -149,13 +150,19 @@ int ensure_tensor_cores(ap_handle *h) {
     return field_solver_bind_bf16(h->fs, h->d_dens_hi, h->d_dens_lo);
 }
 
-// density map (bf16 split or fp32 already in place) -> ex, ey
-int run_field(ap_handle *h, int solver, cudaStream_t st, const int *gate = nullptr, int gate_mask = 0) {
+// Whether a loop trial's field is written as (ex, ey) pairs, one load a bin for
+// the gather: not where other kernels read or write it (a surrogate, the
+// tensor-core solve).
+bool loop_pairs(const ap_handle *h) { return !h->surr && !on_tensor_cores(h, h->p.field_solver); }
+
+// density map (bf16 split or fp32 already in place) -> ex, ey, or pairs
+int run_field(ap_handle *h, int solver, cudaStream_t st, const int *gate = nullptr, int gate_mask = 0,
+              float2 *pairs = nullptr) {
     if (on_tensor_cores(h, solver)) {
         int r = field_solve_bf16x3(h->fs, h->d_dens_hi, h->d_dens_lo, h->d_ex, h->d_ey, st, gate, gate_mask);
         if (r != AP_OK) return r;
     } else {
-        field_solve_fp32(h->fs, h->d_dens, h->d_ex, h->d_ey, st, gate, gate_mask);
+        field_solve_fp32(h->fs, h->d_dens, h->d_ex, h->d_ey, st, gate, gate_mask, pairs);
     }
     return AP_OK;
 }
@@ -292,8 +299,9 @@ void launch_movable_bins(ap_handle *h, ScatterArgs s, cudaStream_t st) {
     }
 }
 
-GatherArgs loop_gather_args(ap_handle *h) {
+GatherArgs loop_gather_args(ap_handle *h, bool pairs) {
     GatherArgs a = gather_args(h, 0, GATHER_STEP);
+    a.exy = pairs ? h->d_exy : nullptr;
     a.rec_bin = h->d_rec_bin;
     a.rec_ov = h->d_rec_ov;
     return a;
@@ -347,12 +355,12 @@ int enqueue_after_update(ap_handle *h, cudaStream_t st) {
         r = enqueue_field_surrogate(h, st, -1);
         if (r != AP_OK) return r;
     } else {
-        r = run_field(h, h->p.field_solver, st);
+        r = run_field(h, h->p.field_solver, st, nullptr, 0, loop_pairs(h) ? h->d_exy : nullptr);
         if (r != AP_OK) return r;
     }
     r = join_wa(h, st);
     if (r != AP_OK) return r;
-    launch_gather(loop_gather_args(h), st);
+    launch_gather(loop_gather_args(h, loop_pairs(h)), st);
     return cudaGetLastError() == cudaSuccess ? AP_OK : AP_ERR_CUDA;
 }
 
@@ -436,7 +444,7 @@ int capture_trial_switched(ap_handle *h) {
     CK(cudaStreamUpdateCaptureDependencies(st, &sw, nullptr, 1, cudaStreamSetCaptureDependencies));
     const int jr = join_wa(h, st);
     if (jr != AP_OK) return jr;
-    launch_gather(loop_gather_args(h), st);
+    launch_gather(loop_gather_args(h, false), st);
     return cudaGetLastError() == cudaSuccess ? AP_OK : AP_ERR_CUDA;
 }
 
@@ -1063,6 +1071,7 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(dalloc(&h->d_dens, nb));
     A(dalloc(&h->d_ex, nb));
     A(dalloc(&h->d_ey, nb));
+    A(dalloc(&h->d_exy, nb));
     A(dalloc(&h->d_sx, N));
     A(dalloc(&h->d_sy, N));
     A(dalloc(&h->d_sc, 1));
@@ -1195,7 +1204,8 @@ int ap_destroy(ap_handle *h) {
                     h->d_mov_q,   h->d_fill_q,   h->d_fix_q,  h->d_fixs_q,  h->d_dens,  h->d_ex,    h->d_ey,
                     h->d_dens_hi, h->d_dens_lo,  h->d_sx,     h->d_sy,      h->d_sc,    h->d_partials,
                     h->d_partials_ll, h->d_counters, h->d_out, h->d_rec_bin, h->d_rec_ov, h->d_gq,
-                    h->d_ix,      h->d_iy,       h->d_xy_loop, h->d_xy_tmp, h->d_whq, h->d_int2ext, h->d_io};
+                    h->d_ix,      h->d_iy,       h->d_xy_loop, h->d_xy_tmp, h->d_whq, h->d_int2ext, h->d_io,
+                    h->d_exy};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (h->h_sc) cudaFreeHost(h->h_sc);
@@ -1345,9 +1355,9 @@ int ap_profile_stages(ap_handle *h, int32_t n_trials, float *stage_ms, int32_t *
         CK(cudaEventRecord(ev[2], st));
         launch_wirelength(wa_args(h, h->d_px[0], h->d_py[0], 0.f, h->n_mov, WA_LOOP, nullptr), st);
         CK(cudaEventRecord(ev[3], st));
-        r = run_field(h, h->p.field_solver, st);
+        r = run_field(h, h->p.field_solver, st, nullptr, 0, loop_pairs(h) ? h->d_exy : nullptr);
         CK(cudaEventRecord(ev[4], st));
-        launch_gather(loop_gather_args(h), st);
+        launch_gather(loop_gather_args(h, loop_pairs(h)), st);
         CK(cudaEventRecord(ev[5], st));
         CK(cudaEventSynchronize(ev[5]));
         for (int i = 0; i < S; ++i) {
@@ -1876,7 +1886,7 @@ int ap_surrogate_collect(ap_handle *h, ap_surrogate *s, int32_t n_trials, int32_
             s->n += 1;
             ++got;
         }
-        launch_gather(loop_gather_args(h), st);
+        launch_gather(loop_gather_args(h, false), st);
         if (cudaGetLastError() != cudaSuccess) r = AP_ERR_CUDA;
         if (r == AP_OK && t % 64 == 0) r = sync(h);
     }
@@ -2065,10 +2075,10 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
         bw[3].push_back(all - wr.small_blocks);
         wa.push_back(wr);
         FieldRec fr[4];
-        if (!field_records(h->fs, h->d_dens, h->d_ex, h->d_ey, pp.field_tile, fr)) return AP_ERR_UNSUPPORTED;
+        if (!field_records(h->fs, h->d_dens, h->d_exy, pp.field_tile, fr)) return AP_ERR_UNSUPPORTED;
         for (int k = 0; k < 4; ++k) fld[k].push_back(fr[k]);
         pp.field_m = std::max(pp.field_m, h->fs.m);
-        gat.push_back(loop_gather_args(h));
+        gat.push_back(loop_gather_args(h, true));
         bg.push_back(gather_grid(h->n_mov, h->p.block_nodes));
     }
     const int ni = (int)upd.size();

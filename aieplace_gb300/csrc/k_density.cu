@@ -147,8 +147,17 @@ __device__ __forceinline__ void emit_rec(const Grid &g, int bin, int xr, int wq,
         return;
     }
     const int nc = rec_nc(bin), nr = rec_nr(bin);
+    const int bw = (int)g.bw_q, bh = (int)g.bh_q;  // record bins: (span + 1) widths fit int32
+    if (nr <= 2) {  // cells of about a bin's height: the rows' overlaps once, not once a column
+        const int oh0 = overlap_1d32(0, bh, yr, hq), oh1 = overlap_1d32(bh, bh, yr, hq);
+        for (int j = 0; j < nc; ++j) {
+            const int ow = overlap_1d32(j * bw, bw, xr, wq);
+            add(c0 + j, r0, (long long)ow * oh0);
+            if (nr == 2) add(c0 + j, r0 + 1, (long long)ow * oh1);
+        }
+        return;
+    }
     for (int j = 0; j < nc; ++j) {
-        const int bw = (int)g.bw_q, bh = (int)g.bh_q;  // record bins: (span + 1) widths fit int32
         const int ow = overlap_1d32(j * bw, bw, xr, wq);
         for (int k = 0; k < nr; ++k) add(c0 + j, r0 + k, (long long)ow * overlap_1d32(k * bh, bh, yr, hq));
     }
@@ -747,18 +756,25 @@ __device__ void finish_trial(DevScalars *sc, double dv2, double dg2) {
     log_trial(sc, 1);
 }
 
+// MODE: GATHER_STEP, or -1 for the mode in the arguments (a loop trial's gather
+// has one sum and few arrays, and its registers suffice for four blocks an SM).
+// PAIRS: the field comes as (ex, ey) pairs, one load a bin: the stage
+// 43.0 -> 42.7 us at 2M cells, 21.9 -> 18.4 at 200k, 14.1 -> 12.9 at 20k.
+template <int MODE, bool PAIRS>
 __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
     __shared__ double red[64];  // 128 floats: four block sums
     const Grid g = a.g;
-    const float lam = a.mode == GATHER_NODE_OUT ? a.lambda : a.sc->f_lambda;
-    const int at = a.mode == GATHER_STEP ? 1 - a.sc->cur : a.at;
+    const int mode = MODE >= 0 ? MODE : a.mode;
+    const float lam = mode == GATHER_NODE_OUT ? a.lambda : a.sc->f_lambda;
+    const int at = mode == GATHER_STEP ? 1 - a.sc->cur : a.at;
+    auto field = [&](int b) { return PAIRS ? __ldg(a.exy + b) : make_float2(__ldg(a.ex + b), __ldg(a.ey + b)); };
     const float *vx = a.vx[at], *vy = a.vy[at], *vpx = a.vx[1 - at], *vpy = a.vy[1 - at];
     float *gx_out = a.gx[at], *gy_out = a.gy[at];
     const float *gpx = a.gx[1 - at], *gpy = a.gy[1 - at];
     // per-thread partials in FP32 (a thread owns a couple of nodes); FP64 from
     // the block sums on -- the FP64 pipe of this part is narrow
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    const bool use_rec = (a.mode == GATHER_STEP || a.mode == GATHER_NODE_OUT) && a.rec_bin != nullptr;
+    const bool use_rec = (mode == GATHER_STEP || mode == GATHER_NODE_OUT) && a.rec_bin != nullptr;
     for (int i = vb.id * blockDim.x + threadIdx.x; i < a.n_mov; i += vb.n * blockDim.x) {
         float fx = 0.f, fy = 0.f;
         int c0, c1, r0, r1;
@@ -770,14 +786,14 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
         const int4 o = use_rec ? __ldg(a.rec_ov + i) : make_int4(0, 0, 0, 0);  // xr, wq, yr, hq
         ull gqv = 0ull;
         float pc = 0.f, chg = 0.f, gpxv = 0.f, gpyv = 0.f;
-        if (a.mode != GATHER_FORCE_ONLY) {
+        if (mode != GATHER_FORCE_ONLY) {
             gqv = a.gq[i];
             pc = __ldg(a.pins + i);
         }
-        if (a.mode == GATHER_STEP || a.mode == GATHER_INIT_GRAD || a.mode == GATHER_INIT_PREV ||
-            a.mode == GATHER_NODE_OUT) {
+        if (mode == GATHER_STEP || mode == GATHER_INIT_GRAD || mode == GATHER_INIT_PREV ||
+            mode == GATHER_NODE_OUT) {
             chg = __ldg(a.charge + i);
-            if (a.mode != GATHER_INIT_GRAD && a.mode != GATHER_NODE_OUT) {
+            if (mode != GATHER_INIT_GRAD && mode != GATHER_NODE_OUT) {
                 gpxv = __ldg(gpx + i);
                 gpyv = __ldg(gpy + i);
             }
@@ -789,18 +805,53 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
             if (rb & kRecSmall) {
                 const int b = c0r * g.my + r0r;
                 const float wt = (i64_to_float(o.y) * i64_to_float(o.w)) * g.inv_ab;
-                fx = wt * __ldg(a.ex + b);
-                fy = wt * __ldg(a.ey + b);
+                const float2 e = field(b);
+                fx = wt * e.x;
+                fy = wt * e.y;
             } else {
                 const int nc = rec_nc(rb), nr = rec_nr(rb);
-                for (int j = 0; j < nc; ++j) {
+                int j0 = 0;
+                if (nr <= 2) {
+                    // cells of about a bin's height: the rows' overlaps once, and the
+                    // loads of the first two columns all in flight before the first
+                    // is used; the sum's order is that of the loop below
+                    const int bw = (int)g.bw_q, bh = (int)g.bh_q, b = c0r * g.my + r0r;
+                    const bool r2 = nr == 2, c2 = nc > 1;
+                    const float2 none = make_float2(0.f, 0.f);
+                    const float2 e00 = field(b), e01 = r2 ? field(b + 1) : none;
+                    const float2 e10 = c2 ? field(b + g.my) : none, e11 = c2 && r2 ? field(b + g.my + 1) : none;
+                    const float fh0 = i32_to_float(overlap_1d32(0, bh, o.z, o.w));
+                    const float fh1 = r2 ? i32_to_float(overlap_1d32(bh, bh, o.z, o.w)) : 0.f;
+                    auto add = [&](float fw, float fh, float2 e) {
+                        const float wt = (fw * fh) * g.inv_ab;
+                        fx = fmaf(wt, e.x, fx);
+                        fy = fmaf(wt, e.y, fy);
+                    };
+                    const float fw0 = i32_to_float(overlap_1d32(0, bw, o.x, o.y));
+                    add(fw0, fh0, e00);
+                    if (r2) add(fw0, fh1, e01);
+                    if (c2) {
+                        const float fw1 = i32_to_float(overlap_1d32(bw, bw, o.x, o.y));
+                        add(fw1, fh0, e10);
+                        if (r2) add(fw1, fh1, e11);
+                    }
+                    for (int j = 2; j < nc; ++j) {
+                        const float fw = i32_to_float(overlap_1d32(j * bw, bw, o.x, o.y));
+                        const int bc = b + j * g.my;
+                        add(fw, fh0, field(bc));
+                        if (r2) add(fw, fh1, field(bc + 1));
+                    }
+                    j0 = nc;
+                }
+                for (int j = j0; j < nc; ++j) {
                     const float fw = i32_to_float(overlap_1d32(j * (int)g.bw_q, (int)g.bw_q, o.x, o.y));
                     const int bc = (c0r + j) * g.my + r0r;
                     for (int k = 0; k < nr; ++k) {
                         const float fh = i32_to_float(overlap_1d32(k * (int)g.bh_q, (int)g.bh_q, o.z, o.w));
                         const float wt = (fw * fh) * g.inv_ab;
-                        fx += wt * __ldg(a.ex + bc + k);
-                        fy += wt * __ldg(a.ey + bc + k);
+                        const float2 e = field(bc + k);
+                        fx = fmaf(wt, e.x, fx);
+                        fy = fmaf(wt, e.y, fy);
                     }
                 }
             }
@@ -809,28 +860,28 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
             const float x = vx[i], y = vy[i], w = __ldg(a.w + i), h = __ldg(a.h + i);
             const long long xq = to_q(x), yq = to_q(y), wq = to_q(w), hq = to_q(h);
             if (small) {
-                const long long b = (long long)c0 * g.my + r0;
                 // both sides exact in float: one rounding, = (float)(wq * hq)
                 const float wt = (i64_to_float(wq) * i64_to_float(hq)) * g.inv_ab;
-                fx = wt * __ldg(a.ex + b);
-                fy = wt * __ldg(a.ey + b);
+                const float2 e = field(c0 * g.my + r0);
+                fx = wt * e.x;
+                fy = wt * e.y;
             } else {
                 for (int c = c0; c <= c1; ++c) {
                     const long long ow = overlap_1d((long long)c * g.bw_q, g.bw_q, xq, wq);
                     for (int r = r0; r <= r1; ++r) {
                         const long long oh = overlap_1d((long long)r * g.bh_q, g.bh_q, yq, hq);
-                        const long long b = (long long)c * g.my + r;
                         const float wt = (i64_to_float(ow) * i64_to_float(oh)) * g.inv_ab;
-                        fx += wt * __ldg(a.ex + b);
-                        fy += wt * __ldg(a.ey + b);
+                        const float2 e = field(c * g.my + r);
+                        fx = fmaf(wt, e.x, fx);
+                        fy = fmaf(wt, e.y, fy);
                     }
                 }
             }
         }
-        if (a.mode == GATHER_FORCE_ONLY || a.mode == GATHER_NODE_OUT) {
+        if (mode == GATHER_FORCE_ONLY || mode == GATHER_NODE_OUT) {
             a.fx[i] = fx;
             a.fy[i] = fy;
-            if (a.mode == GATHER_FORCE_ONLY) continue;
+            if (mode == GATHER_FORCE_ONLY) continue;
         }
         long long qx, qy;
         unpack_q(gqv, qx, qy);
@@ -841,7 +892,7 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
         }
         const float wlx = i64_to_float(qx) * kInvGradScale;
         const float wly = i64_to_float(qy) * kInvGradScale;
-        if (a.mode == GATHER_INIT_NORMS) {
+        if (mode == GATHER_INIT_NORMS) {
             s2 += fabsf(wlx) + fabsf(wly);
             s3 += fabsf(fx) + fabsf(fy);
             continue;
@@ -853,8 +904,9 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
         }
         const float hd = fmaxf(1.f, pc + lam * chg);
         const float ihd = __frcp_rn(hd);
-        const float gx = (wlx - lam * fx) * ihd, gy = (wly - lam * fy) * ihd;
-        if (a.mode == GATHER_NODE_OUT) {
+        // fused by hand: left to the compiler it depends on the mode's code
+        const float gx = fmaf(-lam, fx, wlx) * ihd, gy = fmaf(-lam, fy, wly) * ihd;
+        if (mode == GATHER_NODE_OUT) {
             if (a.gxo) {
                 a.gxo[i] = gx;
                 a.gyo[i] = gy;
@@ -863,11 +915,11 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
         }
         gx_out[i] = gx;
         gy_out[i] = gy;
-        if (a.mode == GATHER_INIT_GRAD) {
+        if (mode == GATHER_INIT_GRAD) {
             s2 = fmaxf(s2, fmaxf(fabsf(gx), fabsf(gy)));
         } else {
             // |v - v_prev|^2 of a loop trial comes from the position update
-            if (a.mode != GATHER_STEP) {
+            if (mode != GATHER_STEP) {
                 const float dx = vx[i] - vpx[i], dy = vy[i] - vpy[i];
                 s0 += dx * dx + dy * dy;
             }
@@ -875,16 +927,22 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
             s1 += ddx * ddx + ddy * ddy;
         }
     }
-    if (a.mode == GATHER_FORCE_ONLY || a.mode == GATHER_NODE_OUT) return;
-    const bool is_max = a.mode == GATHER_INIT_GRAD;
+    if (mode == GATHER_FORCE_ONLY || mode == GATHER_NODE_OUT) return;
+    const bool is_max = mode == GATHER_INIT_GRAD;
     // per-block partials in FP32; the last block sums them with compensation
     // and only its warp 0 adds in FP64 (the FP64 pipe of this part is narrow)
+    float *pf = reinterpret_cast<float *>(a.partials);
+    if (mode == GATHER_STEP) {
+        float v[1] = {s1};
+        block_sums_ff<1>(v, reinterpret_cast<float *>(red));
+        if (threadIdx.x == 0) pf[4 * vb.id + 1] = v[0];
+        return;
+    }
     float bs[4] = {s0, s1, s2, s3};
     if (is_max)
         bs[2] = (float)block_max_f(s2, red);  // s0, s1, s3 are zero in this mode
     else
         block_sums_ff<4>(bs, reinterpret_cast<float *>(red));
-    float *pf = reinterpret_cast<float *>(a.partials);
     if (threadIdx.x == 0) {
         float *p = pf + 4 * vb.id;
         p[0] = bs[0];
@@ -904,15 +962,17 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
                           ? 0.0
                           : block_sum_f(kahan_strided(pf + 0, threadIdx.x, nb, blockDim.x, 4), red);
     const double t1 = block_sum_f(kahan_strided(pf + 1, threadIdx.x, nb, blockDim.x, 4), red);
-    double t2;
-    if (is_max) {
+    double t2 = 0.0, t3 = 0.0;
+    if (a.mode == GATHER_STEP) {
+        // one sum: the others are the initial evaluation's
+    } else if (is_max) {
         float m = 0.f;
         for (int k = threadIdx.x; k < nb; k += blockDim.x) m = fmaxf(m, __ldcg(pf + 4 * k + 2));
         t2 = block_max_f(m, red);
     } else {
         t2 = block_sum_f(kahan_strided(pf + 2, threadIdx.x, nb, blockDim.x, 4), red);
     }
-    const double t3 = block_sum_f(kahan_strided(pf + 3, threadIdx.x, nb, blockDim.x, 4), red);
+    if (a.mode != GATHER_STEP) t3 = block_sum_f(kahan_strided(pf + 3, threadIdx.x, nb, blockDim.x, 4), red);
     if (threadIdx.x == 0) {
         DevScalars *sc = a.sc;
         if (a.mode == GATHER_INIT_NORMS) {
@@ -941,8 +1001,9 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
     }
 }
 
+template <int MODE, bool PAIRS>
 __global__ void __launch_bounds__(kThreads, 4) gather_kernel(GatherArgs a) {
-    gather_body(a, grid_block());
+    gather_body<MODE, PAIRS>(a, grid_block());
     if (a.mode == GATHER_FORCE_ONLY || a.mode == GATHER_NODE_OUT) return;
     if (arrive_last(a.counter, gridDim.x)) gather_fold(a, gridDim.x);
 }
@@ -952,7 +1013,7 @@ int gather_grid(int n_mov, int block_nodes) {
     // nodes against 4096 blocks (a partial last wave, 912 blocks, 59 us)
     static int wave = 0;
     if (wave <= 0) {
-        wave = wave_of((const void *)gather_kernel, kThreads, 608);
+        wave = wave_of((const void *)gather_kernel<GATHER_STEP, true>, kThreads, 608);
         if (wave > kGatherMaxBlocks) wave = 608;
     }
     const int per = block_nodes > kThreads ? block_nodes : kThreads;
@@ -962,7 +1023,11 @@ int gather_grid(int n_mov, int block_nodes) {
 }
 
 void launch_gather(const GatherArgs &a, cudaStream_t st) {
-    gather_kernel<<<gather_grid(a.n_mov, a.block_nodes), kThreads, 0, st>>>(a);
+    const int blocks = gather_grid(a.n_mov, a.block_nodes);
+    if (a.mode == GATHER_STEP && a.exy)
+        gather_kernel<GATHER_STEP, true><<<blocks, kThreads, 0, st>>>(a);
+    else
+        gather_kernel<-1, false><<<blocks, kThreads, 0, st>>>(a);
 }
 
 // Bin records of movable nodes at given positions, as update_kernel writes
@@ -1069,7 +1134,7 @@ __global__ void __launch_bounds__(kThreads) persist_rho_kernel(PersistQueue q, c
 
 __global__ void __launch_bounds__(kThreads, 4) persist_gather_kernel(PersistQueue q, const GatherArgs *recs) {
     persist_loop(q, recs, [](const GatherArgs &a, VBlock vb, int) {
-        gather_body(a, vb);
+        gather_body<GATHER_STEP, true>(a, vb);
         if (arrive_last(a.counter, vb.n)) gather_fold(a, vb.n);
     });
 }

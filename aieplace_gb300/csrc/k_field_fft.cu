@@ -464,7 +464,9 @@ __device__ __forceinline__ void fft_fields(const FieldRec &a, int vb, float2 *sm
         const float2 *z = sm + s * SL;
         const float2 e = z[fft_pad(t)], o = z[fft_pad(M - 1 - t)];  // y = 2 t, 2 t + 1
         const size_t at = (size_t)row * M + 2 * t;
-        if (a.wide) {
+        if (a.exy) {
+            *reinterpret_cast<float4 *>(a.exy + at) = make_float4(e.x, e.y, o.x, -o.y);
+        } else if (a.wide) {
             *reinterpret_cast<float2 *>(a.ex + at) = make_float2(e.x, o.x);
             *reinterpret_cast<float2 *>(a.ey + at) = make_float2(e.y, -o.y);
         } else {  // the caller's buffers, aligned to 4 bytes only
@@ -567,11 +569,12 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm) {
     for (int w = 0; w < 512 / NT; ++w) {  // S4: Ex[x][y], Ey[x][y]
         const int zz = z + w;
         dense_dot(zz ? sm.ct : sm.st, sm.b[zz], i, j, acc);
-        float *e = zz ? a.ey : a.ex;
+        float *e = a.exy ? reinterpret_cast<float *>(a.exy) + zz : zz ? a.ey : a.ex;
+        const int step = a.exy ? 2 : 1;
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int q = 0; q < 2; ++q) e[(i + 16 * r) * M + j + 16 * q] = acc[r][q];
+            for (int q = 0; q < 2; ++q) e[((i + 16 * r) * M + j + 16 * q) * step] = acc[r][q];
     }
 }
 
@@ -636,7 +639,7 @@ void launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask) {
 }
 
 // a solve's arguments: tables, scratch, all rows
-FieldRec solve_rec(const FieldSolver &f, const float *d, float *ex, float *ey) {
+FieldRec solve_rec(const FieldSolver &f, const float *d, float *ex, float *ey, float2 *exy) {
     FieldRec a{};
     a.m = f.m;
     a.d = d;
@@ -644,6 +647,7 @@ FieldRec solve_rec(const FieldSolver &f, const float *d, float *ex, float *ey) {
     a.u = f.u;
     a.ex = ex;
     a.ey = ey;
+    a.exy = exy;
     a.tab = f.tab;
     a.wx = f.wx;
     a.wy = f.wy;
@@ -725,8 +729,8 @@ static bool field_fft_size(int m) {
 }
 
 void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cudaStream_t st, const int *gate,
-                      int gate_mask) {
-    const FieldRec a = solve_rec(f, d, ex, ey);
+                      int gate_mask, float2 *exy) {
+    const FieldRec a = solve_rec(f, d, ex, ey, exy);
     switch (f.m) {
     case kDense: dense_kernel<<<1, 512, 0, st>>>(a, gate, gate_mask); break;
     case 64: launch_fft<64>(a, st, gate, gate_mask); break;
@@ -800,10 +804,10 @@ void field_solver_free(FieldSolver &f) {
 // the batch's choice) runs the passes of any grid; the bits do not depend on
 // it (an FFT's arithmetic is its own).
 
-bool field_records(const FieldSolver &f, const float *d, float *ex, float *ey, int tile, FieldRec rec[4]) {
+bool field_records(const FieldSolver &f, const float *d, float2 *exy, int tile, FieldRec rec[4]) {
     if ((f.m != kDense && 2 * fft_threads(f.m) > 8 * tile) || odd_part(f.m) != 1) return false;
     for (int k = 0; k < 4; ++k) {
-        rec[k] = solve_rec(f, d, ex, ey);
+        rec[k] = solve_rec(f, d, nullptr, nullptr, exy);
         rec[k].pass = std::min(k, 2);
     }
     rec[2].row_hi = rec[3].row_lo = f.m / 2;
