@@ -53,6 +53,10 @@ void launch_interleave(int n, const float *px, const float *py, float2 *xy, cuda
 // each, 4 per gather block at kGatherMaxBlocks, 2 per update block (at most
 // 8192 blocks).
 constexpr int kPartialDoubles = 4 * 8192 + 64;
+// Where the three launches' partials start (a trial's stay apart until its
+// gather folds the update's): the update's at 0
+constexpr int kWaPartials = 8192;
+constexpr int kGatherPartials = kWaPartials + 4 * 2432;
 // Blocks per bucket launch, grid-stride beyond (at 2M cells: 4096 blocks
 // 131 us for the WA stage, 2432 blocks 123 us, 1216 blocks 133 us)
 constexpr int kWaMaxBlocks = 2432;
@@ -170,6 +174,11 @@ struct GatherArgs {
     float *gxo, *gyo;
     DevScalars *sc;
     double *partials;       // 4 * grid
+    // GATHER_STEP: block partials the gather folds (counts of 0: folded by
+    // their own kernels): the position update's and the overflow's
+    const float *upd_partials;
+    const long long *rho_partials;
+    int n_upd, n_rho;
     unsigned int *counter;
     int mode;
     // GATHER_STEP / NODE_OUT, optional: the bin records of this point
@@ -234,6 +243,10 @@ void field_solver_free(FieldSolver &f);
 // exy: the field as (ex, ey) pairs here instead of in ex, ey (or null)
 void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cudaStream_t st,
                       const int *gate = nullptr, int gate_mask = 0, float2 *exy = nullptr);
+// The same from the fixed-point maps, with the density kernel's work (rho_kernel)
+// in its first pass; returns that pass's blocks, whose overflow sums (in
+// rho.partials) are the gather's to fold.
+int field_solve_maps(FieldSolver &f, const RhoArgs &rho, float2 *exy, cudaStream_t st);
 // Builds the TMA tensor maps of the tcgen05 path with (d_hi, d_lo) as the
 // density input; needs m a multiple of 128.
 int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo);

@@ -236,7 +236,7 @@ WaArgs wa_args(ap_handle *h, const float *px, const float *py, float gamma, int 
     a.gqx = h->d_gqx;
     a.gqy = h->d_gqy;
     a.n_grad = n_grad;
-    a.partials = h->d_partials;
+    a.partials = h->d_partials + kWaPartials;
     a.counter = h->d_counters + 0;
     a.out = out;
     a.mode = mode;
@@ -265,7 +265,7 @@ GatherArgs gather_args(ap_handle *h, int at, int mode) {
     a.pins = h->d_pins;
     a.charge = h->d_charge;
     a.sc = h->d_sc;
-    a.partials = h->d_partials;
+    a.partials = h->d_partials + kGatherPartials;
     a.counter = h->d_counters + 2;
     a.mode = mode;
     a.block_nodes = h->p.block_nodes;
@@ -304,6 +304,8 @@ GatherArgs loop_gather_args(ap_handle *h, bool pairs) {
     a.exy = pairs ? h->d_exy : nullptr;
     a.rec_bin = h->d_rec_bin;
     a.rec_ov = h->d_rec_ov;
+    a.upd_partials = reinterpret_cast<const float *>(h->d_partials);
+    a.rho_partials = h->d_partials_ll;
     return a;
 }
 
@@ -345,28 +347,32 @@ int join_wa(ap_handle *h, cudaStream_t st) {
     return AP_OK;
 }
 
-// The trial after its position update.
-int enqueue_after_update(ap_handle *h, cudaStream_t st) {
+// The trial after its position update, whose n_upd block partials the gather
+// folds.
+int enqueue_after_update(ap_handle *h, cudaStream_t st, int n_upd) {
     int r = fork_wa(h, st);
     if (r != AP_OK) return r;
     launch_movable_bins(h, loop_scatter_args(h), st);
-    launch_rho(rho_args(h, RHO_LOOP, nullptr), st);
-    if (h->surr) {
-        r = enqueue_field_surrogate(h, st, -1);
-        if (r != AP_OK) return r;
+    GatherArgs g = loop_gather_args(h, loop_pairs(h));
+    g.n_upd = n_upd;
+    if (loop_pairs(h)) {
+        // density and overflow within the solve's first pass; folded by the gather
+        g.n_rho = field_solve_maps(h->fs, rho_args(h, RHO_LOOP, nullptr), h->d_exy, st);
     } else {
-        r = run_field(h, h->p.field_solver, st, nullptr, 0, loop_pairs(h) ? h->d_exy : nullptr);
+        launch_rho(rho_args(h, RHO_LOOP, nullptr), st);
+        r = h->surr ? enqueue_field_surrogate(h, st, -1) : run_field(h, h->p.field_solver, st);
         if (r != AP_OK) return r;
     }
     r = join_wa(h, st);
     if (r != AP_OK) return r;
-    launch_gather(loop_gather_args(h, loop_pairs(h)), st);
+    launch_gather(g, st);
     return cudaGetLastError() == cudaSuccess ? AP_OK : AP_ERR_CUDA;
 }
 
 int enqueue_iteration(ap_handle *h, cudaStream_t st) {
-    launch_update(loop_scatter_args(h), st);
-    return enqueue_after_update(h, st);
+    ScatterArgs s = loop_scatter_args(h);
+    s.no_fold = 1;
+    return enqueue_after_update(h, st, launch_update(s, st));
 }
 
 // Density/overflow + WA + field at buffer `at` (no position update).
@@ -1464,11 +1470,11 @@ int ap_step_host(ap_handle *h, const float *x_in, const float *y_in, float *x_ou
                 sa.upd_lo = lo;
                 sa.upd_hi = hi;  // chunks are non-empty: nc > 1 only for n_mov >= 65536
                 sa.part_base = base;
-                sa.no_fold = k < nc - 1;
+                sa.no_fold = 1;
                 base += launch_update(sa, st);
             }
             CK(cudaEventRecord(h->ev_upd, st));
-            int r = enqueue_after_update(h, st);
+            int r = enqueue_after_update(h, st, base);
             if (r != AP_OK) return r;
             CK(cudaStreamWaitEvent(h->copy_stream, h->ev_upd, 0));
             CK(cudaMemcpyAsync(x_out, h->d_sx, sizeof(float) * h->n_nodes, cudaMemcpyDeviceToHost, h->copy_stream));

@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "ap_common.cuh"
+#include "ap_density.cuh"
 #include "ap_kernels.h"
 #include "ap_persist.cuh"
 
@@ -273,7 +274,7 @@ __device__ __forceinline__ void update_fold(const ScatterArgs &a, int nb) {
 
 __global__ void __launch_bounds__(kThreads) update_kernel(ScatterArgs a) {
     update_body<true>(a, grid_block());
-    if (a.no_fold) return;  // uniform: an earlier chunk of a chunked update
+    if (a.no_fold) return;  // uniform: an earlier chunk of a chunked update, or the gather folds
     // the partials of this launch and of the chunks before it (launched
     // earlier on the same stream, so complete)
     if (arrive_last(a.counter, gridDim.x)) update_fold(a, a.part_base + (int)gridDim.x);
@@ -560,48 +561,23 @@ __device__ __forceinline__ void rho_body(const RhoArgs &a, VBlock vb) {
     // thread and round, every load of the round issued before any store (the
     // kernel is bound by memory latency, not bandwidth)
     const int npairs = a.nbins >> 1;
-    longlong2 *mov2 = reinterpret_cast<longlong2 *>(a.mov_q);
-    const longlong2 *__restrict__ fs2 = reinterpret_cast<const longlong2 *>(a.fixs_q);
-    const longlong2 *__restrict__ fx2 = reinterpret_cast<const longlong2 *>(a.fix_q);
-    longlong2 *fl2 = reinterpret_cast<longlong2 *>(a.fill_q);  // filler cells, or null
     const int stride = vb.n * blockDim.x;
     for (int p0 = vb.id * blockDim.x + threadIdx.x; p0 < npairs; p0 += kRhoBatch * stride) {
-        longlong2 mv[kRhoBatch], fs[kRhoBatch], fx[kRhoBatch], fl[kRhoBatch];
+        BinPair b[kRhoBatch];
 #pragma unroll
-        for (int j = 0; j < kRhoBatch; ++j) {
-            const int p = p0 + j * stride;
-            fl[j] = make_longlong2(0, 0);
-            if (p < npairs) {
-                mv[j] = __ldcg(mov2 + p);
-                fs[j] = __ldg(fs2 + p);
-                fx[j] = __ldg(fx2 + p);
-                if (fl2) fl[j] = __ldcg(fl2 + p);
-            }
-        }
+        for (int j = 0; j < kRhoBatch; ++j)
+            if (p0 + j * stride < npairs) b[j] = load_pair(a, p0 + j * stride);
 #pragma unroll
         for (int j = 0; j < kRhoBatch; ++j) {
             const int p = p0 + j * stride;
             if (p >= npairs) break;
-            mov2[p] = make_longlong2(0, 0);
-            if (fl2) fl2[p] = make_longlong2(0, 0);
-            const long long m[2] = {mv[j].x, mv[j].y}, sq[2] = {fs[j].x, fs[j].y}, f[2] = {fx[j].x, fx[j].y};
-            const long long fil[2] = {fl[j].x, fl[j].y};
-            float d[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const long long tot = m[k] + sq[k];
-                const long long t = tot - a.cap_q;
-                over += t > 0 ? t : 0;
-                const long long ab = m[k] + f[k] - a.ab_q;
-                over_abs += ab > 0 ? ab : 0;
-                d[k] = ll2f_rn_bits(tot + fil[k]) * a.inv_ab_f - a.d_shift;
-            }
-            if (a.d_f32) reinterpret_cast<float2 *>(a.d_f32)[p] = make_float2(d[0], d[1]);
+            const float2 d = take_pair(a, p, b[j], over, over_abs);
+            if (a.d_f32) reinterpret_cast<float2 *>(a.d_f32)[p] = d;
             if (a.d_hi) {
-                const __nv_bfloat16 h0 = __float2bfloat16_rn(d[0]), h1 = __float2bfloat16_rn(d[1]);
+                const __nv_bfloat16 h0 = __float2bfloat16_rn(d.x), h1 = __float2bfloat16_rn(d.y);
                 reinterpret_cast<__nv_bfloat162 *>(a.d_hi)[p] = __halves2bfloat162(h0, h1);
                 reinterpret_cast<__nv_bfloat162 *>(a.d_lo)[p] = __floats2bfloat162_rn(
-                    d[0] - __bfloat162float(h0), d[1] - __bfloat162float(h1));
+                    d.x - __bfloat162float(h0), d.y - __bfloat162float(h1));
             }
         }
     }
@@ -611,6 +587,12 @@ __device__ __forceinline__ void rho_body(const RhoArgs &a, VBlock vb) {
         a.partials[2 * vb.id] = over;
         a.partials[2 * vb.id + 1] = over_abs;
     }
+}
+
+__device__ __forceinline__ void overflow_of(const DevScalars *sc, long long o, long long oa, double &tau,
+                                            double &tau_abs) {
+    tau = sc->mov_area_q > 0 ? (double)o / sc->mov_area_q : 0.0;
+    tau_abs = (double)oa * 0x1p-32;  // exact power-of-two scaling
 }
 
 // The overflow sums of partials [0, nb) into the device scalars, gamma of the
@@ -626,8 +608,8 @@ __device__ __forceinline__ void rho_fold(const RhoArgs &a, int nb) {
     oa = block_sum(oa, red);
     if (threadIdx.x == 0) {
         DevScalars *sc = a.sc;
-        const double tau = sc->mov_area_q > 0 ? (double)o / sc->mov_area_q : 0.0;
-        const double tau_abs = (double)oa * 0x1p-32;  // exact power-of-two scaling
+        double tau, tau_abs;
+        overflow_of(sc, o, oa, tau, tau_abs);
         if (a.out) {
             a.out[0] = tau;
             a.out[1] = tau_abs;
@@ -952,27 +934,122 @@ __device__ __forceinline__ void gather_body(const GatherArgs &a, VBlock vb) {
     }
 }
 
-// The sums of partials [0, nb) into the device scalars; in a loop trial the
-// accept / retry decision (one block).
+// kahan_strided's sum of n values, the loads of the first four all in flight
+struct Strided {
+    float v[4];
+    const float *p;
+    int n, step;
+    __device__ __forceinline__ void load(const float *partials, int count, int s) {
+        p = partials;
+        n = count;
+        step = s;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = threadIdx.x + u * kThreads;
+            v[u] = i < n ? __ldcg(p + (size_t)i * step) : 0.f;
+        }
+    }
+    __device__ __forceinline__ float sum() const {
+        float s = 0.f, c = 0.f;
+        auto add = [&](float x) {
+            const float y = x - c, t = s + y;
+            c = (t - s) - y;
+            s = t;
+        };
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (threadIdx.x + u * kThreads < n) add(v[u]);
+        for (int i = threadIdx.x + 4 * kThreads; i < n; i += kThreads) add(__ldcg(p + (size_t)i * step));
+        return s;
+    }
+};
+
+// A loop trial's end, in the gather's last block: the gather's own sum, the
+// position update's two and the overflow's two (their kernels leave the
+// block partials to this block, so that none of them ends in a fold the next
+// launch waits for), then the accept / retry decision.  The scalars are
+// worked on in shared memory: one load and one store of the whole block
+// instead of a chain of dependent accesses by one thread.
+__device__ __forceinline__ void step_fold(const GatherArgs &a, int nb) {
+    static_assert(sizeof(DevScalars) % 4 == 0, "whole words");
+    __shared__ __align__(8) DevScalars sc;
+    __shared__ double fsum[3][32];
+    __shared__ long long isum[2][32];
+    constexpr int words = (int)(sizeof(DevScalars) / 4);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (int)blockDim.x >> 5;
+    for (int t = tid; t < words; t += blockDim.x)
+        reinterpret_cast<int *>(&sc)[t] = __ldcg(reinterpret_cast<const int *>(a.sc) + t);
+    Strided s[3];
+    s[0].load(reinterpret_cast<const float *>(a.partials) + 1, nb, 4);
+    s[1].load(a.upd_partials, a.n_upd, 2);
+    s[2].load(a.upd_partials + 1, a.n_upd, 2);
+    long long o = 0, oa = 0;
+    for (int i = tid; i < a.n_rho; i += blockDim.x) {
+        o += __ldcg(a.rho_partials + 2 * i);
+        oa += __ldcg(a.rho_partials + 2 * i + 1);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float v = warp_sum(s[k].sum());
+        if (lane == 0) fsum[k][wid] = (double)v;
+    }
+    o = warp_sum(o);
+    oa = warp_sum(oa);
+    if (lane == 0) {
+        isum[0][wid] = o;
+        isum[1][wid] = oa;
+    }
+    __syncthreads();
+    if (wid == 0) {
+        double d[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d[k] = warp_sum(lane < nw ? fsum[k][lane] : 0.0);
+        o = warp_sum(lane < nw ? isum[0][lane] : 0ll);
+        oa = warp_sum(lane < nw ? isum[1][lane] : 0ll);
+        if (lane == 0) {
+            if (a.n_upd) {
+                sc.t_du = d[1];
+                sc.t_dv2 = d[2];
+            }
+            if (a.n_rho) {
+                overflow_of(&sc, o, oa, sc.t_tau, sc.t_tau_abs);
+                sc.gamma_next = gamma_of(&sc, sc.t_tau);
+                sc.field_mode = kFieldExact;
+            }
+            // the next evaluation's WA smoothing: this trial's gamma(tau),
+            // whether the trial is accepted or not
+            sc.gamma = sc.gamma_next;
+            finish_trial(&sc, sc.t_dv2, d[0]);
+            publish_f32(&sc);
+            *a.counter = 0u;
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < words; t += blockDim.x)
+        reinterpret_cast<int *>(a.sc)[t] = reinterpret_cast<const int *>(&sc)[t];
+}
+
+// The sums of partials [0, nb) of the initial evaluations into the device
+// scalars (one block).
 __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
     __shared__ double red[64];
+    if (a.mode == GATHER_STEP) {  // uniform
+        step_fold(a, nb);
+        return;
+    }
     const bool is_max = a.mode == GATHER_INIT_GRAD;
     const float *pf = reinterpret_cast<const float *>(a.partials);
-    const double t0 = a.mode == GATHER_STEP
-                          ? 0.0
-                          : block_sum_f(kahan_strided(pf + 0, threadIdx.x, nb, blockDim.x, 4), red);
+    const double t0 = block_sum_f(kahan_strided(pf + 0, threadIdx.x, nb, blockDim.x, 4), red);
     const double t1 = block_sum_f(kahan_strided(pf + 1, threadIdx.x, nb, blockDim.x, 4), red);
-    double t2 = 0.0, t3 = 0.0;
-    if (a.mode == GATHER_STEP) {
-        // one sum: the others are the initial evaluation's
-    } else if (is_max) {
+    double t2;
+    if (is_max) {
         float m = 0.f;
         for (int k = threadIdx.x; k < nb; k += blockDim.x) m = fmaxf(m, __ldcg(pf + 4 * k + 2));
         t2 = block_max_f(m, red);
     } else {
         t2 = block_sum_f(kahan_strided(pf + 2, threadIdx.x, nb, blockDim.x, 4), red);
     }
-    if (a.mode != GATHER_STEP) t3 = block_sum_f(kahan_strided(pf + 3, threadIdx.x, nb, blockDim.x, 4), red);
+    const double t3 = block_sum_f(kahan_strided(pf + 3, threadIdx.x, nb, blockDim.x, 4), red);
     if (threadIdx.x == 0) {
         DevScalars *sc = a.sc;
         if (a.mode == GATHER_INIT_NORMS) {
@@ -981,7 +1058,7 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
             sc->lambda = t3 > 0.0 ? sc->init_density_weight * t2 / t3 : sc->init_density_weight;
         } else if (a.mode == GATHER_INIT_GRAD) {
             sc->gmax = t2;
-        } else if (a.mode == GATHER_INIT_PREV) {
+        } else {
             // first predicted step from v_0 and the probe point v_{-1}
             sc->sum_dv2 = t0;
             sc->sum_dg2 = t1;
@@ -990,11 +1067,6 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
             sc->a_next = (1.0 + sqrt(5.0)) / 2.0;
             sc->mom = 0.0;
             if (!isfinite(sc->alpha)) sc->status = 9;
-        } else {
-            // the next evaluation's WA smoothing: this trial's gamma(tau),
-            // whether the trial is accepted or not
-            sc->gamma = sc->gamma_next;
-            finish_trial(sc, sc->t_dv2, t1);
         }
         publish_f32(sc);
         *a.counter = 0u;

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "../../include/aieplace.h"
+#include "ap_density.cuh"
 #include "ap_kernels.h"
 
 namespace ap {
@@ -299,19 +300,76 @@ __device__ __forceinline__ float2 merge_cos(float re, float im, float2 h) {
     return make_float2(0.5f * fmaf(h.x, re, __fmul_rn(h.y, im)), 0.5f * fmaf(h.x, im, -__fmul_rn(h.y, re)));
 }
 
-// P1: block vb transforms rows 2 f, 2 f + 1, f = vb S .. vb S + S - 1.
+// The overflow sums of a block, through warp sums in `red`; the caller has a
+// barrier between the two halves.
+template <int NT>
+__device__ __forceinline__ void put_overflow(long long over, long long over_abs, long long (*red)[2]) {
+    over = warp_sum(over);
+    over_abs = warp_sum(over_abs);
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5][0] = over;
+        red[threadIdx.x >> 5][1] = over_abs;
+    }
+}
+template <int NT>
+__device__ __forceinline__ void get_overflow(const RhoArgs &rho, int vb, const long long (*red)[2]) {
+    if (threadIdx.x < 2) {
+        long long s = 0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) s += red[w][threadIdx.x];
+        rho.partials[2 * vb + threadIdx.x] = s;
+    }
+}
+
+// P1 from the fixed-point maps: the block's 2 S rows of densities into its
+// slots (row 2 f of slot f the real part), the maps cleared, the overflow
+// summed -- rho_kernel's work, without the map's round trip and its launch.
 template <int M, int NT>
-__device__ __forceinline__ void fft_rows(const FieldRec &a, int vb, float2 *sm) {
+__device__ __forceinline__ void rows_density(const RhoArgs &rho, int vb, float2 *sm) {
+    constexpr int S = fft_slots(M, NT), SL = fft_slot(M), N = fft_points(M);
+    constexpr int B = M <= 1024 ? 4 : 2;  // pairs in flight
+    static_assert(N * NT == 2 * S * (M / 2) && N % B == 0 && (M / 2) % S == 0, "the pairs fill the block");
+    __shared__ long long red[NT / 32][2];
+    float *d = reinterpret_cast<float *>(sm);
+    long long over = 0, over_abs = 0;
+#pragma unroll
+    for (int it = 0; it < N; it += B) {
+        BinPair b[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) b[u] = load_pair(rho, vb * (N * NT) + (it + u) * NT + (int)threadIdx.x);
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int at = (it + u) * NT + (int)threadIdx.x, row = at / (M / 2), c = at % (M / 2);
+            const float2 v = take_pair(rho, vb * (N * NT) + at, b[u], over, over_abs);
+            float *z = d + 2 * (row >> 1) * SL + (row & 1);  // bins 2 c, 2 c + 1: elements c, M - 1 - c
+            z[2 * fft_pad(c)] = v.x;
+            z[2 * fft_pad(M - 1 - c)] = v.y;
+        }
+    }
+    put_overflow<NT>(over, over_abs, red);
+    __syncthreads();
+    get_overflow<NT>(rho, vb, red);
+}
+
+// P1: block vb transforms rows 2 f, 2 f + 1, f = vb S .. vb S + S - 1.  MAPS:
+// from the fixed-point maps `rho`.
+template <int M, int NT, bool MAPS = false>
+__device__ __forceinline__ void fft_rows(const FieldRec &a, int vb, float2 *sm, const RhoArgs *rho = nullptr) {
     constexpr int TPF = fft_threads(M), E = fft_points(M), S = fft_slots(M, NT), SL = fft_slot(M);
     static_assert(S >= 2 && S % 2 == 0, "whole tiles of four rows per block");
     const int slot = (int)threadIdx.x / TPF, j = (int)threadIdx.x % TPF;
     const int f = vb * S + slot;
     float2 x[E];
-    const float *r0 = a.d + (size_t)(2 * f) * M, *r1 = r0 + M;
+    if constexpr (MAPS) {
+        rows_density<M, NT>(*rho, vb, sm);
+        slot_load<M>(x, sm + slot * SL, j);
+    } else {
+        const float *r0 = a.d + (size_t)(2 * f) * M, *r1 = r0 + M;
 #pragma unroll
-    for (int q = 0; q < E; ++q) {
-        const int n = j + q * TPF, y = n < M / 2 ? 2 * n : 2 * (M - 1 - n) + 1;
-        x[q] = f < M / 2 ? make_float2(__ldg(r0 + y), __ldg(r1 + y)) : make_float2(0.f, 0.f);
+        for (int q = 0; q < E; ++q) {
+            const int n = j + q * TPF, y = n < M / 2 ? 2 * n : 2 * (M - 1 - n) + 1;
+            x[q] = f < M / 2 ? make_float2(__ldg(r0 + y), __ldg(r1 + y)) : make_float2(0.f, 0.f);
+        }
     }
     fft_stage<M, false, 0>(x, sm + slot * SL, j, a.tab);
     __syncthreads();
@@ -517,9 +575,20 @@ __device__ __forceinline__ void dense_dot(const float (*A)[kDenseLd], const floa
     }
 }
 
-template <int NT>  // 256 or 512 threads
-__device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm) {
+// 256 or 512 threads; MAPS (512): from the fixed-point maps `rho`
+template <int NT, bool MAPS = false>
+__device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, const RhoArgs *rho = nullptr) {
     constexpr int M = kDense;
+    __shared__ long long red[NT / 32][2];
+    if constexpr (MAPS) {
+        static_assert(NT == M * M / 2, "a pair of bins per thread");
+        long long over = 0, over_abs = 0;
+        const int p = (int)threadIdx.x;
+        const float2 d = take_pair(*rho, p, load_pair(*rho, p), over, over_abs);
+        sm.b[0][2 * p / M][2 * p % M] = d.x;
+        sm.b[0][2 * p / M][2 * p % M + 1] = d.y;
+        put_overflow<NT>(over, over_abs, red);
+    }
     const float *tab = reinterpret_cast<const float *>(a.tab);
     for (int t = threadIdx.x; t < M * M; t += NT) {
         const int k = t / M, i = t % M;
@@ -527,9 +596,10 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm) {
         sm.c[k][i] = c;
         sm.ct[i][k] = c;
         sm.st[i][k] = s;
-        sm.b[0][k][i] = __ldg(a.d + t);
+        if constexpr (!MAPS) sm.b[0][k][i] = __ldg(a.d + t);
     }
     __syncthreads();
+    if constexpr (MAPS) get_overflow<NT>(*rho, 0, red);
     // 256 threads a product; the two products of S3 and of S4 side by side
     // (512 threads) or in turn
     const int t = threadIdx.x & 255, z = threadIdx.x >> 8, i = t >> 4, j = t & 15;
@@ -598,6 +668,19 @@ __global__ void __launch_bounds__(NT, odd_part(M) == 1 && M <= 2048 ? 1024 / NT 
     if (PASS == 2) fft_fields<M, NT>(a, blockIdx.x, fft_sm);
 }
 
+// (up to 1024 bins its blocks are resident at once with 512 threads an SM: 128 registers, no spills)
+template <int M, int NT>
+__global__ void __launch_bounds__(NT, (M <= 1024 ? 512 : 1024) / NT) fft_maps_kernel(FieldRec a, RhoArgs rho) {
+    extern __shared__ __align__(16) float2 fft_sm[];
+    grid_release();
+    fft_rows<M, NT, true>(a, blockIdx.x, fft_sm, &rho);
+}
+
+__global__ void __launch_bounds__(512) dense_maps_kernel(FieldRec a, RhoArgs rho) {
+    __shared__ __align__(16) DenseSmem sm;
+    dense_solve<512, true>(a, sm, &rho);
+}
+
 __global__ void __launch_bounds__(512) dense_kernel(FieldRec a, const int *gate, int mask) {
     __shared__ __align__(16) DenseSmem sm;
     if (gated_off(gate, mask)) return;
@@ -614,15 +697,26 @@ constexpr int fft_blocks(int m, int nt, int pass, int rows) {
 // at least.
 constexpr int fft_block_threads(int m) { return std::max(32, 2 * fft_threads(m)); }
 
+// rho: the first pass from the fixed-point maps (or null); returns its blocks
 template <int M>
-void launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask) {
+int launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask, const RhoArgs *rho = nullptr) {
     constexpr int NT = fft_block_threads(M), SM = fft_smem(M, NT);
     if constexpr (SM > 48 * 1024) {  // a no-op after the first call
         cudaFuncSetAttribute(fft_kernel<M, NT, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
         cudaFuncSetAttribute(fft_kernel<M, NT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
         cudaFuncSetAttribute(fft_kernel<M, NT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
     }
-    fft_kernel<M, NT, 0><<<fft_blocks(M, NT, 0, M), NT, SM, st>>>(a, gate, mask);
+    constexpr int blocks = fft_blocks(M, NT, 0, M);
+    bool maps = false;
+    if constexpr (odd_part(M) == 1) {
+        if (rho) {
+            maps = true;
+            if constexpr (SM > 48 * 1024)
+                cudaFuncSetAttribute(fft_maps_kernel<M, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
+            fft_maps_kernel<M, NT><<<blocks, NT, SM, st>>>(a, *rho);
+        }
+    }
+    if (!maps) fft_kernel<M, NT, 0><<<blocks, NT, SM, st>>>(a, gate, mask);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -636,6 +730,7 @@ void launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask) {
     cudaLaunchKernelEx(&cfg, fft_kernel<M, NT, 1>, a, gate, mask);
     cfg.gridDim = dim3(fft_blocks(M, NT, 2, M));
     cudaLaunchKernelEx(&cfg, fft_kernel<M, NT, 2>, a, gate, mask);
+    return blocks;
 }
 
 // a solve's arguments: tables, scratch, all rows
@@ -744,6 +839,20 @@ void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cuda
     case 1024: launch_fft<1024>(a, st, gate, gate_mask); break;
     case 2048: launch_fft<2048>(a, st, gate, gate_mask); break;
     case 4096: launch_fft<4096>(a, st, gate, gate_mask); break;
+    }
+}
+
+int field_solve_maps(FieldSolver &f, const RhoArgs &rho, float2 *exy, cudaStream_t st) {
+    const FieldRec a = solve_rec(f, nullptr, nullptr, nullptr, exy);
+    switch (f.m) {
+    case kDense: dense_maps_kernel<<<1, 512, 0, st>>>(a, rho); return 1;
+    case 64: return launch_fft<64>(a, st, nullptr, 0, &rho);
+    case 128: return launch_fft<128>(a, st, nullptr, 0, &rho);
+    case 256: return launch_fft<256>(a, st, nullptr, 0, &rho);
+    case 512: return launch_fft<512>(a, st, nullptr, 0, &rho);
+    case 1024: return launch_fft<1024>(a, st, nullptr, 0, &rho);
+    case 2048: return launch_fft<2048>(a, st, nullptr, 0, &rho);
+    default: return launch_fft<4096>(a, st, nullptr, 0, &rho);
     }
 }
 
