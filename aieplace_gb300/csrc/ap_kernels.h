@@ -44,7 +44,8 @@ struct WaArgs {
     int mode;
 };
 // launches the four bucket kernels (after filling a.xy from a.px, a.py in
-// the modes other than WA_LOOP); the last one (warp per net) folds the sums
+// the modes other than WA_LOOP), or for small netlists all of them as one;
+// the last one (warp per net) folds the sums
 void launch_wirelength(const WaArgs &a, cudaStream_t st);
 // xy[i] = (px[i], py[i]), i < n
 void launch_interleave(int n, const float *px, const float *py, float2 *xy, cudaStream_t st);

@@ -435,6 +435,25 @@ __global__ void __launch_bounds__(kThreads, 4) wa_large_kernel(WaArgs a) {
     if (arrive_last(a.counter, gridDim.x)) wa_fold(a, a.small_blocks + (int)gridDim.x);
 }
 
+// The four launches in one, by block range: where all their blocks are
+// resident at once.  At its largest bucket's registers it holds fewer blocks an
+// SM, and past one wave that costs more than three launches (an iteration
+// with the four / with the one: 576 cells 27.1 / 25.1 us, 5k 31.6 / 27.3, 60k
+// 36.0 / 35.4; 200k, 1582 blocks, 72.2 / 75.2; 2M 210 / 254).
+__global__ void __launch_bounds__(kThreads, 3) wa_all_kernel(WaArgs a) {
+    int b = (int)blockIdx.x;
+    if (b < a.bucket_blocks[0]) {
+        wa_small_body<2, 0>(a, VBlock{b, a.bucket_blocks[0]});
+    } else if ((b -= a.bucket_blocks[0]) < a.bucket_blocks[1]) {
+        wa_small_body<4, 1>(a, VBlock{b, a.bucket_blocks[1]});
+    } else if ((b -= a.bucket_blocks[1]) < a.bucket_blocks[2]) {
+        wa_small_body<8, 2>(a, VBlock{b, a.bucket_blocks[2]});
+    } else {
+        wa_large_body(a, VBlock{b - a.bucket_blocks[2], (int)gridDim.x - a.small_blocks});
+    }
+    if (arrive_last(a.counter, gridDim.x)) wa_fold(a, (int)gridDim.x);
+}
+
 int wa_plan(WaArgs &a) {
     const int per = a.block_nets > kThreads ? a.block_nets : kThreads;
     auto grid = [per](int items) {
@@ -470,7 +489,13 @@ void launch_interleave(int n, const float *px, const float *py, float2 *xy, cuda
 void launch_wirelength(const WaArgs &a0, cudaStream_t st) {
     WaArgs a = a0;
     if (a.mode != WA_LOOP) launch_interleave(a.n_nodes, a.px, a.py, a.xy, st);
-    const int large = wa_plan(a) - a.small_blocks;
+    const int all = wa_plan(a), large = all - a.small_blocks;
+    static int wave = 0;
+    if (wave <= 0) wave = wave_of((const void *)wa_all_kernel, kThreads, 456);
+    if (all <= wave) {
+        wa_all_kernel<<<all, kThreads, 0, st>>>(a);
+        return;
+    }
     wa_small_kernel<2, 0><<<a.bucket_blocks[0], kThreads, 0, st>>>(a);
     wa_small_kernel<4, 1><<<a.bucket_blocks[1], kThreads, 0, st>>>(a);
     wa_small_kernel<8, 2><<<a.bucket_blocks[2], kThreads, 0, st>>>(a);
