@@ -35,6 +35,56 @@ struct AxisTerms {
 // instructions and a branch per call here
 __device__ __forceinline__ float rcp(float b) { return __fdividef(1.f, b); }
 
+// Both axes at once: two IEEE FP32 operations an instruction (the WA kernels
+// are bound by instruction issue).  exp(x) = 2^(x log2 e), results below 2^-126
+// taken as 0: next to the extreme pin's 1 they change no sum, and no gradient
+// in its fixed point.  The stage at 2M cells 108 -> 100.5 us, at 60k 31 -> 28.
+__device__ __forceinline__ ull pair_bits(float2 a) { return ((ull)__float_as_uint(a.y) << 32) | __float_as_uint(a.x); }
+__device__ __forceinline__ float2 bits_pair(ull v) {
+    return make_float2(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    ull r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    ull r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    ull r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 exp2_pair(float2 a) {
+    const float2 t = mul2(a, both(1.44269504088896341f));
+    float2 r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(t.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(t.y));
+    return r;
+}
+
+// A net's constants of both axes, for its pins' gradients
+struct PairTerms {
+    float2 ibp, ibm;    // 1/b+, 1/b-
+    float2 nwp, nwm;    // -(WA+ - x_max), -(WA- - x_min)
+    __device__ __forceinline__ PairTerms(float2 bp, float2 bm, float2 cp, float2 cm) {
+        ibp = make_float2(rcp(bp.x), rcp(bp.y));
+        ibm = make_float2(rcp(bm.x), rcp(bm.y));
+        nwp = neg2(mul2(cp, ibp));
+        nwm = neg2(mul2(cm, ibm));
+    }
+    // a+/b+ (1 + (x - WA+)/g) - a-/b- (1 - (x - WA-)/g)
+    __device__ __forceinline__ float2 grad(float2 ep, float2 em, float2 dp, float2 dm, float2 ig, float2 nig) const {
+        const float2 tp = fma2(add2(dp, nwp), ig, both(1.f)), tm = fma2(add2(dm, nwm), nig, both(1.f));
+        return fma2(mul2(ep, ibp), tp, neg2(mul2(mul2(em, ibm), tm)));
+    }
+};
+
 // one pin's gradient into its node's accumulators; `raw` is the pin_node entry
 __device__ __forceinline__ void add_grad(ull *gq, ull *gqx, ull *gqy, int raw, float gx, float gy) {
     const int n = raw & kPinNode;
@@ -99,7 +149,7 @@ __device__ __forceinline__ void net_group(const WaArgs &a, int s, int d, int l, 
                                           const float2 *xy, float inv_g, float &hpf, float &waf) {
     bool v[P];
     int nd[P];
-    float c[P][2];
+    float2 c[P];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         const int j = l + p * G;
@@ -107,53 +157,49 @@ __device__ __forceinline__ void net_group(const WaArgs &a, int s, int d, int l, 
         // a slot past the net's end repeats its last pin: the extrema are
         // unchanged and no load waits on a branch (its terms are zeroed below)
         nd[p] = __ldg(a.pin_node + s + min(j, d - 1));  // raw entry (heavy flag)
-        const float2 q = __ldg(xy + (nd[p] & kPinNode));
-        c[p][0] = q.x;
-        c[p][1] = q.y;
+        c[p] = __ldg(xy + (nd[p] & kPinNode));
     }
     float m4[4] = {-3.0e38f, -3.0e38f, -3.0e38f, -3.0e38f};  // max x, max y, -min x, -min y
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-        m4[0] = fmaxf(m4[0], c[p][0]);
-        m4[1] = fmaxf(m4[1], c[p][1]);
-        m4[2] = fmaxf(m4[2], -c[p][0]);
-        m4[3] = fmaxf(m4[3], -c[p][1]);
+        m4[0] = fmaxf(m4[0], c[p].x);
+        m4[1] = fmaxf(m4[1], c[p].y);
+        m4[2] = fmaxf(m4[2], -c[p].x);
+        m4[3] = fmaxf(m4[3], -c[p].y);
     }
     group_max4<G>(m4, l, mask, base);
     const float mx[2] = {m4[0], m4[1]}, mn[2] = {-m4[2], -m4[3]};
-    float ep[P][2], em[P][2], s8[8];
+    // the shifted coordinates are formed again for the gradients (two
+    // instructions a pin, against registers that hold four blocks an SM)
+    const float2 ig = both(inv_g), nig = both(-inv_g);
+    const float2 nmx = make_float2(-mx[0], -mx[1]), nmn = make_float2(-mn[0], -mn[1]);
+    float2 ep[P], em[P], bp = both(0.f), bm = both(0.f), cp = both(0.f), cm = both(0.f);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s8[k] = 0.f;
-#pragma unroll
-    for (int ax = 0; ax < 2; ++ax)
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const float dp = c[p][ax] - mx[ax], dm = c[p][ax] - mn[ax];
-            ep[p][ax] = v[p] ? __expf(dp * inv_g) : 0.f;
-            em[p][ax] = v[p] ? __expf(-dm * inv_g) : 0.f;
-            s8[4 * ax + 0] += ep[p][ax];
-            s8[4 * ax + 1] += em[p][ax];
-            s8[4 * ax + 2] += ep[p][ax] * dp;
-            s8[4 * ax + 3] += em[p][ax] * dm;
-        }
-    group_sum8<G>(s8, l, mask, base);
-    float g[P][2], wa_net = 0.f;
-#pragma unroll
-    for (int ax = 0; ax < 2; ++ax) {
-        const float ibp = rcp(s8[4 * ax + 0]), ibm = rcp(s8[4 * ax + 1]);
-        const float wp = s8[4 * ax + 2] * ibp, wm = s8[4 * ax + 3] * ibm;
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const float dp = c[p][ax] - mx[ax], dm = c[p][ax] - mn[ax];
-            g[p][ax] = ep[p][ax] * ibp * (1.f + (dp - wp) * inv_g) - em[p][ax] * ibm * (1.f - (dm - wm) * inv_g);
-        }
-        wa_net += (mx[ax] - mn[ax]) + wp - wm;
+    for (int p = 0; p < P; ++p) {
+        const float2 dp = add2(c[p], nmx), dm = add2(c[p], nmn);
+        ep[p] = exp2_pair(mul2(dp, ig));
+        em[p] = exp2_pair(mul2(dm, nig));
+        if (!v[p]) ep[p] = em[p] = both(0.f);
+        bp = add2(bp, ep[p]);
+        bm = add2(bm, em[p]);
+        cp = fma2(ep[p], dp, cp);
+        cm = fma2(em[p], dm, cm);
     }
+    float s8[8] = {bp.x, bm.x, cp.x, cm.x, bp.y, bm.y, cp.y, cm.y};
+    group_sum8<G>(s8, l, mask, base);
+    const PairTerms t(make_float2(s8[0], s8[4]), make_float2(s8[1], s8[5]), make_float2(s8[2], s8[6]),
+                      make_float2(s8[3], s8[7]));
 #pragma unroll
-    for (int p = 0; p < P; ++p)
-        if (v[p] && (nd[p] & kPinNode) < a.n_grad) add_grad(a.gq, a.gqx, a.gqy, nd[p], g[p][0], g[p][1]);
+    for (int p = 0; p < P; ++p) {
+        if (!v[p] || (nd[p] & kPinNode) >= a.n_grad) continue;
+        const float2 g = t.grad(ep[p], em[p], add2(c[p], nmx), add2(c[p], nmn), ig, nig);
+        add_grad(a.gq, a.gqx, a.gqy, nd[p], g.x, g.y);
+    }
     if (l == 0) {
         hpf += (mx[0] - mn[0]) + (mx[1] - mn[1]);
+        float wa_net = 0.f;
+        wa_net += (mx[0] - mn[0]) - t.nwp.x + t.nwm.x;
+        wa_net += (mx[1] - mn[1]) - t.nwp.y + t.nwm.y;
         waf += wa_net;
     }
 }
@@ -179,57 +225,43 @@ __device__ __forceinline__ void net_thread(const int *__restrict__ pins, int d, 
                                            float inv_g, ull *gq, ull *gqx, ull *gqy, int n_grad, float &hp_acc,
                                            float &wa_acc) {
     int node[D];
-    float xs[D], ys[D];
+    float2 c[D];
     float xmx = -3.0e38f, xmn = 3.0e38f, ymx = -3.0e38f, ymn = 3.0e38f;
 #pragma unroll
     for (int j = 0; j < D; ++j) {
         if (j < d) {
             node[j] = __ldg(pins + j);  // raw entry (heavy flag)
-            const float2 q = __ldg(xy + (node[j] & kPinNode));
-            xs[j] = q.x;
-            ys[j] = q.y;
-            xmx = fmaxf(xmx, xs[j]);
-            xmn = fminf(xmn, xs[j]);
-            ymx = fmaxf(ymx, ys[j]);
-            ymn = fminf(ymn, ys[j]);
+            c[j] = __ldg(xy + (node[j] & kPinNode));
+            xmx = fmaxf(xmx, c[j].x);
+            xmn = fminf(xmn, c[j].x);
+            ymx = fmaxf(ymx, c[j].y);
+            ymn = fminf(ymn, c[j].y);
         }
     }
-    float gxs[D];
+    const float2 ig = both(inv_g), nig = both(-inv_g);
+    const float2 nmx = make_float2(-xmx, -ymx), nmn = make_float2(-xmn, -ymn);
+    float2 ep[D], em[D], bp = both(0.f), bm = both(0.f), cp = both(0.f), cm = both(0.f);
 #pragma unroll
-    for (int j = 0; j < D; ++j) gxs[j] = 0.f;
-    float wa_net = 0.f;
-#pragma unroll
-    for (int axis = 0; axis < 2; ++axis) {
-        const float cmx = axis ? ymx : xmx, cmn = axis ? ymn : xmn;
-        float ep[D], em[D];
-        float bp = 0.f, bm = 0.f, cp = 0.f, cm = 0.f;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-            if (j < d) {
-                const float c = axis ? ys[j] : xs[j];
-                const float dp = c - cmx, dm = c - cmn;
-                ep[j] = __expf(dp * inv_g);
-                em[j] = __expf(-dm * inv_g);
-                bp += ep[j];
-                bm += em[j];
-                cp += ep[j] * dp;
-                cm += em[j] * dm;
-            }
+    for (int j = 0; j < D; ++j) {
+        if (j < d) {
+            const float2 dp = add2(c[j], nmx), dm = add2(c[j], nmn);
+            ep[j] = exp2_pair(mul2(dp, ig));
+            em[j] = exp2_pair(mul2(dm, nig));
+            bp = add2(bp, ep[j]);
+            bm = add2(bm, em[j]);
+            cp = fma2(ep[j], dp, cp);
+            cm = fma2(em[j], dm, cm);
         }
-        const float ibp = rcp(bp), ibm = rcp(bm), wp = cp * ibp, wm = cm * ibm;
-        wa_net += (cmx - cmn) + wp - wm;
+    }
+    const PairTerms t(bp, bm, cp, cm);
+    float wa_net = 0.f;
+    wa_net += (xmx - xmn) - t.nwp.x + t.nwm.x;
+    wa_net += (ymx - ymn) - t.nwp.y + t.nwm.y;
 #pragma unroll
-        for (int j = 0; j < D; ++j) {
-            if (j < d) {
-                const float c = axis ? ys[j] : xs[j];
-                const float g = ep[j] * ibp * (1.f + ((c - cmx) - wp) * inv_g) -
-                                em[j] * ibm * (1.f - ((c - cmn) - wm) * inv_g);
-                if (axis == 0) {
-                    gxs[j] = g;
-                } else if ((node[j] & kPinNode) < n_grad) {
-                    add_grad(gq, gqx, gqy, node[j], gxs[j], g);
-                }
-            }
+    for (int j = 0; j < D; ++j) {
+        if (j < d && (node[j] & kPinNode) < n_grad) {
+            const float2 g = t.grad(ep[j], em[j], add2(c[j], nmx), add2(c[j], nmn), ig, nig);
+            add_grad(gq, gqx, gqy, node[j], g.x, g.y);
         }
     }
     hp_acc += (xmx - xmn) + (ymx - ymn);
