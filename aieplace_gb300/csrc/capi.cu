@@ -1111,13 +1111,16 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(cudaMallocHost((void **)&h->h_sc, sizeof(DevScalars)));
     A(cudaMallocHost((void **)&h->h_out, sizeof(double) * 8));
     A(cudaMallocHost((void **)&h->h_status, 2 * sizeof(unsigned int)));
-    // the WA launches run beside the density chain (scatter -> rho -> field)
-    // at the same priority: with the chain's stream at the highest priority a
-    // 2M-cell trial took 1.5% longer (its blocks kept the WA blocks waiting
-    // where both would have shared the SMs)
+    // the WA launches run beside the density chain (scatter -> field), whose
+    // blocks they share the SMs with; they are the longer branch at 2M cells
+    // and go first there (an iteration with the WA stream at the chain's
+    // priority / above it: 200k cells 51.8 / 51.8 us, 2M 201.4 / 196.8; the chain's
+    // above the WA's: 1.5% longer than equal)
+    int p_low = 0, p_high = 0;
+    A(cudaDeviceGetStreamPriorityRange(&p_low, &p_high));
     A(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
-    A(cudaStreamCreateWithFlags(&h->wa_stream, cudaStreamNonBlocking));
+    A(cudaStreamCreateWithPriority(&h->wa_stream, cudaStreamNonBlocking, p_high));
     A(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
     A(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     A(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));

@@ -468,6 +468,15 @@ int wave_of(const void *kernel, int threads, int fallback, int dyn_smem) {
     return fallback;
 }
 
+// a wave of at most `per` blocks an SM
+static int at_most_per_sm(int wave, int per) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+        return std::min(wave, per * sms);
+    return wave;
+}
+
 __global__ void size_q_kernel(int n, const float *__restrict__ w, const float *__restrict__ h, int2 *out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const long long wq = to_q(w[i]), hq = to_q(h[i]);
@@ -504,12 +513,15 @@ int launch_update(const ScatterArgs &a, cudaStream_t st) {
 }
 
 int scatter_grid(int n, int block_nodes) {
-    // one wave of resident blocks, each a contiguous range of nodes (fewer
-    // blocks: fewer tile flushes onto the dense core's bins)
+    // two of the three blocks that fit an SM, each a contiguous range of nodes
+    // (fewer blocks: fewer tile flushes onto the dense core's bins): the third
+    // would take the registers and shared memory that the WA launches beside it
+    // need (an iteration with three / two an SM: 200k cells 53.2 / 51.7 us, 2M
+    // 205.5 / 199.5)
     static int wave = 0;
     if (wave <= 0) {
         cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem);
-        wave = wave_of((const void *)scatter_kernel, kScatterThreads, 304, kScatterSmem);
+        wave = at_most_per_sm(wave_of((const void *)scatter_kernel, kScatterThreads, 304, kScatterSmem), 2);
     }
     const int per = block_nodes > kScatterThreads ? block_nodes : kScatterThreads;
     int blocks = (n + per - 1) / per;
@@ -739,7 +751,7 @@ __device__ void finish_trial(DevScalars *sc, double dv2, double dg2) {
 }
 
 // MODE: GATHER_STEP, or -1 for the mode in the arguments (a loop trial's gather
-// has one sum and few arrays, and its registers suffice for four blocks an SM).
+// has one sum and few arrays).
 // PAIRS: the field comes as (ex, ey) pairs, one load a bin: the stage
 // 43.0 -> 42.7 us at 2M cells, 21.9 -> 18.4 at 200k, 14.1 -> 12.9 at 20k.
 template <int MODE, bool PAIRS>
@@ -1073,8 +1085,9 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
     }
 }
 
+// (a loop trial's: five blocks an SM, 42.3 -> 38.9 us at 2M cells against four)
 template <int MODE, bool PAIRS>
-__global__ void __launch_bounds__(kThreads, 4) gather_kernel(GatherArgs a) {
+__global__ void __launch_bounds__(kThreads, MODE == GATHER_STEP ? 5 : 4) gather_kernel(GatherArgs a) {
     gather_body<MODE, PAIRS>(a, grid_block());
     if (a.mode == GATHER_FORCE_ONLY || a.mode == GATHER_NODE_OUT) return;
     if (arrive_last(a.counter, gridDim.x)) gather_fold(a, gridDim.x);
@@ -1222,13 +1235,8 @@ int persist_density_wave(int stage) {
         // beside the scatter and need shared memory and warp slots too
         if (!waves[1]) {
             cudaFuncSetAttribute(persist_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem);
-            int dev = 0, sms = 0;
-            const int full = wave_of((const void *)persist_scatter_kernel, kScatterThreads, 304, kScatterSmem);
-            if (cudaGetDevice(&dev) == cudaSuccess &&
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-                waves[1] = std::min(full, 2 * sms);
-            else
-                waves[1] = full;
+            waves[1] = at_most_per_sm(
+                wave_of((const void *)persist_scatter_kernel, kScatterThreads, 304, kScatterSmem), 2);
         }
         return waves[1];
     case PS_RHO:
