@@ -261,6 +261,29 @@ __device__ __forceinline__ float i32_to_float(int q) {
     return q < 4194304 ? i2f_small(q) : i64_to_float((long long)q);
 }
 
+// Two IEEE FP32 operations in one instruction.
+__device__ __forceinline__ ull pair_bits(float2 a) { return ((ull)__float_as_uint(a.y) << 32) | __float_as_uint(a.x); }
+__device__ __forceinline__ float2 bits_pair(ull v) {
+    return make_float2(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    ull r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    ull r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    ull r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
+    return bits_pair(r);
+}
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -64,9 +64,7 @@ __device__ __forceinline__ float bilinear_up(const float *c, int R, int f, int X
 // ---- pooling and network input ------------------------------------------
 
 // coarse[I][J] = mean of the f x f fine bins; the fine density is FP32
-// (d_f32) or the BF16 hi/lo split of the tensor-core solver (hi + lo).  The
-// result goes to `coarse` (FP32) or, for the tensor-core coarse solve, to
-// its own hi/lo split (c_hi, c_lo).
+// (d_f32) or the BF16 hi/lo split of the tensor-core solver (hi + lo).
 __global__ void pool_kernel(int M, int f, const float *d_f32, const __nv_bfloat16 *d_hi,
                             const __nv_bfloat16 *d_lo, float *coarse, const int *gate, int mask) {
     if (!gate_open(gate, mask)) return;
@@ -268,121 +266,6 @@ __global__ void __launch_bounds__(256) conv_fwd_kernel(int B, int R, int cin, in
     }
 }
 
-// Inference forward of the (K0, 1, 1, 1) architecture in one launch: the
-// arithmetic of four conv_fwd_kernel launches in the same order (bias first,
-// then input channel, kx, ky; ReLU on the hidden layers), so the output is
-// bit-identical, without the three hidden maps in global memory.  Block: an
-// 8 x 32 pixel tile, one pixel per thread (two pixels a thread measured
-// slower: 233 registers left one block per SM); shared memory holds the
-// input tile with its halo and every layer's weights as [input][kMaxCh] rows
-// (one float4 load feeds four output channels).
-struct FusedNet {
-    int cin0, width, cout;
-    size_t w_off[kSurrLayers], b_off[kSurrLayers];
-};
-
-constexpr int kFuseTX = 8, kFuseTY = 32;
-
-__host__ __device__ constexpr int fused_halo(int k) { return (kFuseTX + k - 1) * (kFuseTY + k - 1); }
-
-template <int K0>
-__global__ void __launch_bounds__(256, 2) net_fwd_fused_kernel(int R, FusedNet fn, const float *x0,
-                                                                const float *params, float *y, const int *gate,
-                                                                int mask) {
-    if (!gate_open(gate, mask)) return;
-    extern __shared__ float4 smem4[];
-    constexpr int KK = K0 * K0, H = K0 / 2, HX = kFuseTX + K0 - 1, HY = kFuseTY + K0 - 1;
-    const int cin0 = fn.cin0, width = fn.width, cout = fn.cout;
-    float *w0 = reinterpret_cast<float *>(smem4);      // [cin0 KK][kMaxCh]
-    float *wh = w0 + cin0 * KK * kMaxCh;               // 3 x [kMaxCh][kMaxCh] (layers 1-3)
-    float *bs = wh + 3 * kMaxCh * kMaxCh;              // 4 x [kMaxCh]
-    float *xin = bs + 4 * kMaxCh;                      // [cin0][HX][HY]
-    const int b = blockIdx.z, X0 = blockIdx.y * kFuseTX, Y0 = blockIdx.x * kFuseTY, RR = R * R;
-    // staging by asynchronous copies (zero fill for unused slots and the
-    // halo outside the map): the loads of the whole loop are in flight together
-    for (int t = threadIdx.x; t < cin0 * KK * kMaxCh; t += blockDim.x) {
-        const int co = t % kMaxCh, r = t / kMaxCh, ci = r / KK, kk = r - ci * KK;
-        const bool ok = co < width;
-        cp_async4(w0 + t, params + (ok ? fn.w_off[0] + ((size_t)co * cin0 + ci) * KK + kk : 0), ok);
-    }
-    for (int t = threadIdx.x; t < 3 * kMaxCh * kMaxCh; t += blockDim.x) {
-        const int l = 1 + t / (kMaxCh * kMaxCh), r = t % (kMaxCh * kMaxCh), ci = r / kMaxCh, co = r % kMaxCh;
-        const int cin = width, co_n = l == kSurrLayers - 1 ? cout : width;
-        const size_t wo = l == 1 ? fn.w_off[1] : l == 2 ? fn.w_off[2] : fn.w_off[3];
-        const bool ok = co < co_n && ci < cin;
-        cp_async4(wh + t, params + (ok ? wo + (size_t)co * cin + ci : 0), ok);
-    }
-    for (int t = threadIdx.x; t < 4 * kMaxCh; t += blockDim.x) {
-        const int l = t / kMaxCh, co = t % kMaxCh, co_n = l == kSurrLayers - 1 ? cout : width;
-        const size_t bo = l == 0 ? fn.b_off[0] : l == 1 ? fn.b_off[1] : l == 2 ? fn.b_off[2] : fn.b_off[3];
-        const bool ok = co < co_n;
-        cp_async4(bs + t, params + (ok ? bo + co : 0), ok);
-    }
-    const float *xb = x0 + (size_t)b * cin0 * RR;
-    for (int t = threadIdx.x; t < cin0 * HX * HY; t += blockDim.x) {
-        const int ci = t / (HX * HY), r = t - ci * (HX * HY), hx = r / HY, hy = r - hx * HY;
-        const int xx = X0 + hx - H, yy = Y0 + hy - H;
-        const bool ok = xx >= 0 && xx < R && yy >= 0 && yy < R;
-        cp_async4(xin + t, xb + (ok ? (size_t)ci * RR + xx * R + yy : 0), ok);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const int lx = threadIdx.x / kFuseTY, ly = threadIdx.x % kFuseTY;  // rows lx and lx + 8
-    float a0[kMaxCh], h0[kMaxCh];
-#pragma unroll
-    for (int c = 0; c < kMaxCh; ++c) a0[c] = bs[c];
-    const float4 *w04 = reinterpret_cast<const float4 *>(w0);
-    for (int ci = 0; ci < cin0; ++ci) {
-        const float *xc = xin + ci * (HX * HY);
-#pragma unroll
-        for (int kx = 0; kx < K0; ++kx)
-#pragma unroll
-            for (int ky = 0; ky < K0; ++ky) {
-                const float v0 = xc[(lx + kx) * HY + ly + ky];
-                const float4 *w4 = w04 + (ci * KK + kx * K0 + ky) * (kMaxCh / 4);
-#pragma unroll
-                for (int j = 0; j < kMaxCh / 4; ++j) {
-                    const float4 w = w4[j];
-                    a0[4 * j] += v0 * w.x;
-                    a0[4 * j + 1] += v0 * w.y;
-                    a0[4 * j + 2] += v0 * w.z;
-                    a0[4 * j + 3] += v0 * w.w;
-                }
-            }
-    }
-#pragma unroll
-    for (int l = 1; l < kSurrLayers; ++l) {
-#pragma unroll
-        for (int c = 0; c < kMaxCh; ++c) {
-            h0[c] = fmaxf(a0[c], 0.f);  // every layer before the last has a ReLU
-            a0[c] = bs[l * kMaxCh + c];
-        }
-        const float4 *w4l = reinterpret_cast<const float4 *>(wh + (l - 1) * kMaxCh * kMaxCh);
-#pragma unroll
-        for (int ci = 0; ci < kMaxCh; ++ci) {
-            if (ci < width) {
-#pragma unroll
-                for (int j = 0; j < kMaxCh / 4; ++j) {
-                    const float4 w = w4l[ci * (kMaxCh / 4) + j];
-                    a0[4 * j] += h0[ci] * w.x;
-                    a0[4 * j + 1] += h0[ci] * w.y;
-                    a0[4 * j + 2] += h0[ci] * w.z;
-                    a0[4 * j + 3] += h0[ci] * w.w;
-                }
-            }
-        }
-    }
-    const int xg = X0 + lx, yg = Y0 + ly;
-    if (yg < R) {
-        float *yb = y + (size_t)b * cout * RR;
-#pragma unroll
-        for (int c = 0; c < kMaxCh; ++c)
-            if (c < cout) {
-                yb[(size_t)c * RR + xg * R + yg] = a0[c];
-            }
-    }
-}
-
 // dIn[b][ci][x][y] = sum_co sum_k W[co][ci][k] g[b][co][x - kx + H][y - ky + H],
 // g = dOut, masked by out > 0 when the layer has a ReLU.  Weights in shared
 // memory as [cout][K*K][kMaxCh] (input channel fastest).
@@ -495,6 +378,385 @@ __global__ void reduce_tiles_kernel(int n_tiles, int n, const float *partial, fl
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         float s = 0.f;
         for (int t = 0; t < n_tiles; ++t) s += partial[(size_t)t * n + j];
+        grad[j] = s;
+    }
+}
+
+// ---- the (K0, 1, 1, 1) architecture by tiles of pixels ------------------------
+// A block of 256 threads takes a kTile x kTile tile of one map through all
+// layers: past the first a pixel's activations depend on that pixel alone, so
+// they stay in shared memory, [channel][kPixLd].  Every layer is a product of
+// 256 pixels, its inputs and kMaxCh output channels, and a thread holds eight
+// pixels (a half row) x four channels of it: per input two vector loads of
+// pixels and one of weights for 32 products.  (A pixel a thread with all its
+// channels read eight weight vectors, the same for every lane, for as many
+// products: shared memory was the bound, 50 us for a 256 x 256 map of 18 inputs
+// against 38.6 under ncu, of which 16 are the products at the FP32 rate.)  The sums run as in conv_fwd_kernel -- bias, then input
+// channel, kx, ky -- so the outputs are those of the per-layer kernels bit for
+// bit.
+struct FusedNet {
+    int cin0, width, cout;
+    size_t w_off[kSurrLayers], b_off[kSurrLayers];
+};
+
+constexpr int kPix = kTile * kTile;
+constexpr int kPixLd = kPix + 4;  // rows of a layer: 16-byte aligned, four banks apart
+constexpr int kRowLd = kTile + 4;  // rows of the input patch (kTile + K0 - 1 of them)
+constexpr int kWLd = kMaxCh + 4;   // rows of weights
+
+struct TileThread {
+    int cg, p0, px, y0;  // channels 4 cg .., pixels p0 .. p0 + 7: row px, columns y0 ..
+    __device__ __forceinline__ TileThread() {
+        const int lane = threadIdx.x & 31, pg = (threadIdx.x >> 5) * 4 + (lane & 3);
+        cg = lane >> 2;
+        p0 = 8 * pg;
+        px = pg >> 1;
+        y0 = 8 * (pg & 1);
+    }
+};
+
+// [channel][pixel pair] sums of a thread
+struct TileSums {
+    float2 a[4][4];
+    __device__ __forceinline__ void bias(const float *bs, int cg) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[c][q] = both(bs[4 * cg + c]);
+    }
+    __device__ __forceinline__ void add(const float2 (&v)[4], float4 w) {
+        const float ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[c][q] = fma2(v[q], both(ww[c]), a[c][q]);
+    }
+    // += over inputs i < n: in[i][pixel] w[i][channel]
+    __device__ __forceinline__ void layer(const float *in, const float *w, int n, const TileThread &t) {
+        const float *ip = in + t.p0, *wp = w + 4 * t.cg;
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) {
+            const float4 u = *reinterpret_cast<const float4 *>(ip + i * kPixLd);
+            const float4 v = *reinterpret_cast<const float4 *>(ip + i * kPixLd + 4);
+            const float2 p[4] = {make_float2(u.x, u.y), make_float2(u.z, u.w), make_float2(v.x, v.y),
+                                 make_float2(v.z, v.w)};
+            add(p, *reinterpret_cast<const float4 *>(wp + i * kWLd));
+        }
+    }
+    // the first layer from the input patch [ci][row][kRowLd]
+    template <int K0>
+    __device__ __forceinline__ void first(const float *xin, const float *w, int cin, const TileThread &t) {
+        constexpr int P = kTile + K0 - 1;
+        for (int ci = 0; ci < cin; ++ci)
+#pragma unroll
+            for (int kx = 0; kx < K0; ++kx) {
+                const float *r = xin + (ci * P + t.px + kx) * kRowLd + t.y0;
+                const float4 u = *reinterpret_cast<const float4 *>(r), v = *reinterpret_cast<const float4 *>(r + 4);
+                float x[10] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, 0.f, 0.f};
+                if (K0 > 1) {
+                    const float2 e = *reinterpret_cast<const float2 *>(r + 8);
+                    x[8] = e.x;
+                    x[9] = e.y;
+                }
+#pragma unroll
+                for (int ky = 0; ky < K0; ++ky) {
+                    const float2 p[4] = {make_float2(x[ky], x[ky + 1]), make_float2(x[ky + 2], x[ky + 3]),
+                                         make_float2(x[ky + 4], x[ky + 5]), make_float2(x[ky + 6], x[ky + 7])};
+                    add(p, *reinterpret_cast<const float4 *>(w + ((ci * K0 + kx) * K0 + ky) * kWLd + 4 * t.cg));
+                }
+            }
+    }
+    // f(value, channel of four, pixel of eight) into rows of `out`
+    template <class F>
+    __device__ __forceinline__ void store(float *out, const TileThread &t, F &&f) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4 *>(out + (4 * t.cg + c) * kPixLd + t.p0 + 4 * q) =
+                    make_float4(f(a[c][2 * q].x, c, 4 * q), f(a[c][2 * q].y, c, 4 * q + 1),
+                                f(a[c][2 * q + 1].x, c, 4 * q + 2), f(a[c][2 * q + 1].y, c, 4 * q + 3));
+    }
+};
+
+// Shared memory of a tile (floats): the weights as [input][kWLd] rows of
+// channels, the biases, the input patch; `wt`: layers 1-3 again as [output] rows
+struct TileNet {
+    float *w0, *wh, *wt, *bs, *xin;
+    template <int K0>
+    __device__ __forceinline__ float *carve(float *p, int cin0, bool train) {
+        w0 = p;
+        wh = w0 + cin0 * K0 * K0 * kWLd;
+        wt = wh + 3 * kMaxCh * kWLd;
+        bs = wt + (train ? 3 * kMaxCh * kWLd : 0);
+        xin = bs + 4 * kMaxCh;
+        return xin + cin0 * (kTile + K0 - 1) * kRowLd;
+    }
+};
+__host__ __device__ constexpr int tile_net_floats(int cin0, int k0, bool train) {
+    return (cin0 * k0 * k0 + (train ? 6 : 3) * kMaxCh) * kWLd + 4 * kMaxCh + cin0 * (kTile + k0 - 1) * kRowLd;
+}
+
+// Staging by asynchronous copies (zero fill for unused slots and the halo
+// outside the map): the loads of every loop are in flight together, a warp to
+// a row as it is stored.
+template <int K0>
+__device__ __forceinline__ void stage_tile(const TileNet &m, const FusedNet &fn, const float *params, const float *xb,
+                                           int R, int X0, int Y0, bool train) {
+    constexpr int KK = K0 * K0, H = K0 / 2, P = kTile + K0 - 1;
+    const int cin0 = fn.cin0, width = fn.width, cout = fn.cout, RR = R * R, n0 = cin0 * KK;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int row = warp; row < cin0 * P; row += 8) {
+        const int ci = row / P, xx = X0 + row - ci * P - H, yy = Y0 + lane - H;
+        const bool ok = xx >= 0 && xx < R && yy >= 0 && yy < R;
+        if (lane < P) cp_async4(m.xin + row * kRowLd + lane, xb + (ok ? (size_t)ci * RR + xx * R + yy : 0), ok);
+    }
+    for (int co = warp; co < kMaxCh; co += 8)
+        for (int r = lane; r < n0; r += 32)
+            cp_async4(m.w0 + r * kWLd + co, params + (co < width ? fn.w_off[0] + (size_t)co * n0 + r : 0), co < width);
+    for (int row = warp; row < 3 * kMaxCh; row += 8) {
+        const int l = 1 + row / kMaxCh, co = row % kMaxCh, ci = lane, co_n = l == kSurrLayers - 1 ? cout : width;
+        const size_t wo = l == 1 ? fn.w_off[1] : l == 2 ? fn.w_off[2] : fn.w_off[3];
+        const bool ok = co < co_n && ci < width;
+        const float *src = params + (ok ? wo + (size_t)co * width + ci : 0);
+        cp_async4(m.wh + ((l - 1) * kMaxCh + ci) * kWLd + co, src, ok);
+        if (train) cp_async4(m.wt + ((l - 1) * kMaxCh + co) * kWLd + ci, src, ok);
+    }
+    if (warp < 4) {
+        const int l = warp, co_n = l == kSurrLayers - 1 ? cout : width;
+        const size_t bo = l == 0 ? fn.b_off[0] : l == 1 ? fn.b_off[1] : l == 2 ? fn.b_off[2] : fn.b_off[3];
+        cp_async4(m.bs + l * kMaxCh + lane, params + (lane < co_n ? bo + lane : 0), lane < co_n);
+    }
+}
+
+// All layers: the hidden maps into hs (layer l's at hs + l step; step 0: one
+// buffer in turn), the outputs left in s.
+template <int K0>
+__device__ __forceinline__ void tile_forward(const TileNet &m, const FusedNet &fn, float *hs, int step,
+                                             const TileThread &t, TileSums &s) {
+    s.bias(m.bs, t.cg);
+    s.first<K0>(m.xin, m.w0, fn.cin0, t);
+#pragma unroll 1
+    for (int l = 1; l < kSurrLayers; ++l) {
+        float *h = hs + (l - 1) * step;
+        __syncthreads();  // one buffer: every thread has read the layer before
+        s.store(h, t, [](float v, int, int) { return fmaxf(v, 0.f); });
+        __syncthreads();
+        s.bias(m.bs + l * kMaxCh, t.cg);
+        s.layer(h, m.wh + (l - 1) * kMaxCh * kWLd, fn.width, t);
+    }
+}
+
+template <int K0>
+__global__ void __launch_bounds__(256, 2) net_fwd_fused_kernel(int R, FusedNet fn, const float *x0,
+                                                                const float *params, float *y, const int *gate,
+                                                                int mask) {
+    if (!gate_open(gate, mask)) return;
+    extern __shared__ float4 smem4[];
+    TileNet m;
+    float *hs = m.carve<K0>(reinterpret_cast<float *>(smem4), fn.cin0, false);
+    const int b = blockIdx.z, X0 = blockIdx.y * kTile, Y0 = blockIdx.x * kTile, RR = R * R;
+    stage_tile<K0>(m, fn, params, x0 + (size_t)b * fn.cin0 * RR, R, X0, Y0, false);
+    cp_async_wait_all();
+    __syncthreads();
+    const TileThread t;
+    TileSums s;
+    tile_forward<K0>(m, fn, hs, 0, t, s);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (4 * t.cg + c < fn.cout) {
+            float4 *o = reinterpret_cast<float4 *>(y + ((size_t)b * fn.cout + 4 * t.cg + c) * RR + (X0 + t.px) * R +
+                                                   Y0 + t.y0);
+            o[0] = make_float4(s.a[c][0].x, s.a[c][0].y, s.a[c][1].x, s.a[c][1].y);
+            o[1] = make_float4(s.a[c][2].x, s.a[c][2].y, s.a[c][3].x, s.a[c][3].y);
+        }
+}
+
+// Training pass: forward, loss and every gradient of the tile; only the weight
+// gradients' sums over the tile (partial[tile][n_params]) and the squared
+// error leave the block.  Sums within a tile run as in the per-layer kernels,
+// whose 14 launches of 6-27 us each waited for their own loads (a gradient of 8
+// maps of 64 x 64: 250 us a call, 99 in two launches).
+template <int K0>
+__global__ void __launch_bounds__(256, 1) net_train_kernel(int B, int R, int margin, FusedNet fn, const float *x0,
+                                                           const float *target, const float *map_w,
+                                                           const float *params, int n_params, float *partial,
+                                                           float *loss_partial) {
+    extern __shared__ float4 smem4[];
+    constexpr int KK = K0 * K0, P = kTile + K0 - 1, kHid = kMaxCh * kPixLd;
+    const int cin0 = fn.cin0, width = fn.width, cout = fn.cout;
+    float *gs = reinterpret_cast<float *>(smem4);  // gradient w.r.t. the layer's output
+    float *hs = gs + kHid;                         // three hidden maps
+    TileNet m;
+    m.carve<K0>(hs + 3 * kHid, cin0, true);
+    __shared__ float red[32];
+    const int tiles = R / kTile, tile = blockIdx.x, b = tile / (tiles * tiles);
+    const int tr = tile - b * tiles * tiles, X0 = (tr / tiles) * kTile, Y0 = (tr % tiles) * kTile;
+    const int RR = R * R, tid = threadIdx.x;
+    stage_tile<K0>(m, fn, params, x0 + (size_t)b * cin0 * RR, R, X0, Y0, true);
+    const TileThread t;
+    const int xg = X0 + t.px, yg = Y0 + t.y0;
+    float4 tv[4][2];  // the targets, loaded while the copies are in flight
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            tv[c][q] = 4 * t.cg + c < cout ? __ldg(reinterpret_cast<const float4 *>(
+                                                 target + ((size_t)b * cout + 4 * t.cg + c) * RR + xg * R + yg + 4 * q))
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+    cp_async_wait_all();
+    __syncthreads();
+    TileSums s;
+    tile_forward<K0>(m, fn, hs, kHid, t, s);
+    // loss and its gradient (mse_kernel)
+    const int inner = R - 2 * margin;
+    const float inv_n = 1.f / ((float)B * cout * inner * inner), wb = map_w ? map_w[b] : 1.f;
+    float sq = 0.f;
+    s.store(gs, t, [&](float v, int c, int p) {
+        const float4 q = tv[c][p >> 2];
+        const float tt = (p & 3) == 0 ? q.x : (p & 3) == 1 ? q.y : (p & 3) == 2 ? q.z : q.w;
+        const bool in = 4 * t.cg + c < cout && xg >= margin && xg < R - margin && yg + p >= margin && yg + p < R - margin;
+        const float d = in ? v - tt : 0.f;
+        sq += wb * d * d;
+        return 2.f * wb * d * inv_n;
+    });
+    const float bsum = block_sum_ff(sq, red);
+    if (tid == 0) loss_partial[tile] = bsum;
+    __syncthreads();
+    // backward, last layer first: its weight gradients from gs, then gs for the
+    // layer before
+    float *out = partial + (size_t)tile * n_params;
+#pragma unroll 1
+    for (int l = kSurrLayers - 1; l >= 0; --l) {
+        const int co_n = l == kSurrLayers - 1 ? cout : width;
+        const size_t wo = l == 0 ? fn.w_off[0] : l == 1 ? fn.w_off[1] : l == 2 ? fn.w_off[2] : fn.w_off[3];
+        const size_t bo = l == 0 ? fn.b_off[0] : l == 1 ? fn.b_off[1] : l == 2 ? fn.b_off[2] : fn.b_off[3];
+        const float *h = hs + (l - 1) * kHid;  // the layer's input (l > 0)
+        if (l > 0) {
+            // 2 x 2 weights a thread: outputs co, co + 1, inputs ci, ci + 16
+            const int co = 2 * (tid >> 4), ci = tid & 15;
+            if (co < co_n) {
+                float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+                for (int p = 0; p < kPix; p += 4) {
+                    float4 g[2], v[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        g[k] = *reinterpret_cast<const float4 *>(gs + (co + k) * kPixLd + p);
+                        v[k] = *reinterpret_cast<const float4 *>(h + (ci + 16 * k) * kPixLd + p);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            float r = acc[k][i];
+                            r = fmaf(g[k].x, v[i].x, r);
+                            r = fmaf(g[k].y, v[i].y, r);
+                            r = fmaf(g[k].z, v[i].z, r);
+                            acc[k][i] = fmaf(g[k].w, v[i].w, r);
+                        }
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        if (co + k < co_n && ci + 16 * i < width)
+                            out[wo + (size_t)(co + k) * width + ci + 16 * i] = acc[k][i];
+            }
+        } else {
+            // a thread: input channel, kx; outputs co, co + 8, ..; every ky
+            for (int w = tid; w < cin0 * K0 * 8; w += 256) {
+                const int co = w & 7, kx = (w >> 3) % K0, ci = (w >> 3) / K0;
+                float acc[4][K0];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int k = 0; k < K0; ++k) acc[c][k] = 0.f;
+#pragma unroll 1
+                for (int r = 0; r < kTile; ++r) {
+                    float x[kRowLd];
+#pragma unroll
+                    for (int q = 0; q < kRowLd / 4; ++q) {
+                        const float4 v = *reinterpret_cast<const float4 *>(m.xin + (ci * P + r + kx) * kRowLd + 4 * q);
+                        x[4 * q] = v.x;
+                        x[4 * q + 1] = v.y;
+                        x[4 * q + 2] = v.z;
+                        x[4 * q + 3] = v.w;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int q = 0; q < kTile / 4; ++q) {
+                            const float4 g =
+                                *reinterpret_cast<const float4 *>(gs + (co + 8 * c) * kPixLd + r * kTile + 4 * q);
+#pragma unroll
+                            for (int k = 0; k < K0; ++k) {
+                                float a = acc[c][k];
+                                a = fmaf(g.x, x[4 * q + k], a);
+                                a = fmaf(g.y, x[4 * q + k + 1], a);
+                                a = fmaf(g.z, x[4 * q + k + 2], a);
+                                acc[c][k] = fmaf(g.w, x[4 * q + k + 3], a);
+                            }
+                        }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int k = 0; k < K0; ++k)
+                        if (co + 8 * c < co_n)
+                            out[wo + ((size_t)(co + 8 * c) * cin0 + ci) * KK + kx * K0 + k] = acc[c][k];
+            }
+        }
+        if (tid >= 224 && tid - 224 < co_n) {  // biases, by the last warp
+            float a = 0.f;
+#pragma unroll 8
+            for (int p = 0; p < kPix; p += 4) {
+                const float4 g = *reinterpret_cast<const float4 *>(gs + (tid - 224) * kPixLd + p);
+                a += g.x;
+                a += g.y;
+                a += g.z;
+                a += g.w;
+            }
+            out[bo + tid - 224] = a;
+        }
+        if (l == 0) break;
+        // gradient w.r.t. the layer's input, through its ReLU
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s.a[c][q] = both(0.f);
+        s.layer(gs, m.wt + (l - 1) * kMaxCh * kWLd, co_n, t);
+        __syncthreads();
+        s.store(gs, t, [&](float v, int c, int p) {
+            return h[(4 * t.cg + c) * kPixLd + t.p0 + p] > 0.f ? v : 0.f;
+        });
+        __syncthreads();
+    }
+}
+
+// grad[j] = sum over tiles of partial[tile][j]: eight runs of tiles a
+// parameter, a warp each, added in their order; the last block: the loss
+__global__ void __launch_bounds__(256) train_reduce_kernel(int n_tiles, int n, const float *partial, float *grad,
+                                                           const float *loss_partial, float inv_n, float *loss) {
+    __shared__ double red[32];
+    __shared__ float part[8][32];
+    if (blockIdx.x == gridDim.x - 1) {
+        const double t = block_sum_f(kahan_strided(loss_partial, threadIdx.x, n_tiles, blockDim.x, 1), red);
+        if (threadIdx.x == 0) *loss = (float)(t * (double)inv_n);
+        return;
+    }
+    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+    const int per = (n_tiles + 7) / 8, t1 = min(n_tiles, (run + 1) * per);
+    float s = 0.f;
+    if (j < n)
+#pragma unroll 8
+        for (int t = run * per; t < t1; ++t) s += __ldg(partial + (size_t)t * n + j);
+    part[run][lane] = s;
+    __syncthreads();
+    if (run == 0 && j < n) {
+        s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += part[k][lane];
         grad[j] = s;
     }
 }
@@ -687,22 +949,28 @@ void conv_bwd(const SurrLayer &L, int B, int R, const float *in, const float *ou
 }
 
 size_t fused_smem(int cin0, int k0) {
-    return ((size_t)cin0 * k0 * k0 * kMaxCh + 3 * kMaxCh * kMaxCh + 4 * kMaxCh +
-            (size_t)cin0 * sg::fused_halo(k0)) *
-           sizeof(float);
+    return ((size_t)sg::tile_net_floats(cin0, k0, false) + kMaxCh * sg::kPixLd) * sizeof(float);
 }
+size_t train_smem(int cin0, int k0) {
+    return ((size_t)sg::tile_net_floats(cin0, k0, true) + 4 * kMaxCh * sg::kPixLd) * sizeof(float);
+}
+constexpr int kMaxCin0 = 18;  // f^2 + 2, f <= 4
 
 bool g_attrs_set = false;
 void set_kernel_attrs() {
     if (g_attrs_set) return;
     cudaFuncSetAttribute(sg::net_fwd_fused_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)fused_smem(kMaxCh, 3));
+                         (int)fused_smem(kMaxCin0, 3));
     cudaFuncSetAttribute(sg::net_fwd_fused_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)fused_smem(kMaxCh, 1));
+                         (int)fused_smem(kMaxCin0, 1));
     cudaFuncSetAttribute(sg::conv_bwd_weight_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)wgrad_smem(3));
     cudaFuncSetAttribute(sg::conv_bwd_weight_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)wgrad_smem(1));
+    cudaFuncSetAttribute(sg::net_train_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)train_smem(kMaxCin0, 3));
+    cudaFuncSetAttribute(sg::net_train_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)train_smem(kMaxCin0, 1));
     g_attrs_set = true;
 }
 
@@ -712,20 +980,30 @@ void net_forward(const SurrNet &net, int B, int R, float *const a[kSurrLayers + 
     for (int l = 0; l < kSurrLayers; ++l) conv_fwd(net.L[l], B, R, a[l], net.d_params, a[l + 1], st, gate, mask);
 }
 
+// Whether every layer after the first is 1 x 1 (the hidden maps of a pixel
+// depend on that pixel alone), and the fused kernels' view of the net.
+bool fusable(const SurrNet &net) {
+    bool fuse = true;
+    for (int l = 1; l < kSurrLayers; ++l) fuse = fuse && net.L[l].k == 1;
+    return fuse;
+}
+sg::FusedNet fused_net(const SurrNet &net) {
+    sg::FusedNet fn{net.cin0, net.width, net.cout, {}, {}};
+    for (int l = 0; l < kSurrLayers; ++l) {
+        fn.w_off[l] = net.L[l].w_off;
+        fn.b_off[l] = net.L[l].b_off;
+    }
+    return fn;
+}
+
 // Inference forward x -> y: one fused launch when every layer after the first
 // is 1 x 1 (the hidden maps stay in registers), else the per-layer kernels
 // through the scratch maps a[1..3].  Both give the same bits.
 void net_infer(const SurrNet &net, int B, int R, const float *x, float *const a[kSurrLayers + 1], float *y,
                cudaStream_t st, const int *gate = nullptr, int mask = 0) {
-    bool fuse = true;
-    for (int l = 1; l < kSurrLayers; ++l) fuse = fuse && net.L[l].k == 1;
-    if (fuse) {
-        sg::FusedNet fn{net.cin0, net.width, net.cout, {}, {}};
-        for (int l = 0; l < kSurrLayers; ++l) {
-            fn.w_off[l] = net.L[l].w_off;
-            fn.b_off[l] = net.L[l].b_off;
-        }
-        const dim3 g((R + sg::kFuseTY - 1) / sg::kFuseTY, R / sg::kFuseTX, B);
+    if (fusable(net)) {
+        const sg::FusedNet fn = fused_net(net);
+        const dim3 g(R / kTile, R / kTile, B);
         if (net.L[0].k == 3)
             sg::net_fwd_fused_kernel<3><<<g, 256, fused_smem(net.cin0, 3), st>>>(R, fn, x, net.d_params, y, gate,
                                                                                   mask);
@@ -884,7 +1162,8 @@ int ensure_scratch(ap_surrogate *s, int B, int R) {
     ok = ok && ap::dmalloc(&s->d_g[0], (size_t)B * kMaxCh * RR) && ap::dmalloc(&s->d_g[1], (size_t)B * kMaxCh * RR);
     const size_t tiles = (size_t)B * (R / kTile) * (R / kTile);
     ok = ok && ap::dmalloc(&s->d_tb, (size_t)B * n.cout * RR) &&
-         ap::dmalloc(&s->d_wpart, tiles * (kMaxCh * kMaxCh * 9 + kMaxCh)) && ap::dmalloc(&s->d_lpart, 2 * ap::kBlocks) &&
+         ap::dmalloc(&s->d_wpart, tiles * (size_t)std::max(kMaxCh * kMaxCh * 9 + kMaxCh, n.n_params)) &&
+         ap::dmalloc(&s->d_lpart, std::max(2 * (size_t)ap::kBlocks, tiles)) &&
          ap::dmalloc(&s->d_loss, 2) && ap::dmalloc(&s->d_sel, 3 * (size_t)B) && ap::dmalloc(&s->d_cnt, 4) &&
          ap::dmalloc(&s->d_w, B);
     if (!ok || cudaMemset(s->d_cnt, 0, 4 * sizeof(unsigned int)) != cudaSuccess) {
@@ -901,12 +1180,25 @@ int ensure_scratch(ap_surrogate *s, int B, int R) {
 void train_pass(ap_surrogate *s, int B, int R, int margin, bool relative, cudaStream_t st) {
     ap::SurrNet &net = s->net;
     float *const *a = s->d_a;
+    if (relative) ap::sg::rel_weight_kernel<<<B, 256, 0, st>>>(net.cout, R, margin, s->d_tb, s->d_w);
+    const float *map_w = relative ? s->d_w : nullptr;
+    if (ap::fusable(net)) {
+        const int tiles = B * (R / kTile) * (R / kTile), n = net.n_params, inner = R - 2 * margin;
+        const size_t smem = ap::train_smem(net.cin0, net.L[0].k);
+        if (net.L[0].k == 3)
+            ap::sg::net_train_kernel<3><<<tiles, 256, smem, st>>>(B, R, margin, ap::fused_net(net), a[0], s->d_tb, map_w,
+                                                                   net.d_params, n, s->d_wpart, s->d_lpart);
+        else
+            ap::sg::net_train_kernel<1><<<tiles, 256, smem, st>>>(B, R, margin, ap::fused_net(net), a[0], s->d_tb, map_w,
+                                                                   net.d_params, n, s->d_wpart, s->d_lpart);
+        ap::sg::train_reduce_kernel<<<(n + 31) / 32 + 1, 256, 0, st>>>(
+            tiles, n, s->d_wpart, net.d_grad, s->d_lpart, 1.f / ((float)B * net.cout * inner * inner), s->d_loss);
+        return;
+    }
     ap::net_forward(net, B, R, a, st);
     const size_t ny = (size_t)B * net.cout * R * R;
-    if (relative) ap::sg::rel_weight_kernel<<<B, 256, 0, st>>>(net.cout, R, margin, s->d_tb, s->d_w);
-    ap::sg::mse_kernel<<<ap::grid_for(ny), 256, 0, st>>>(B, net.cout, R, margin, a[kSurrLayers], s->d_tb,
-                                                         relative ? s->d_w : nullptr, s->d_g[0], s->d_lpart,
-                                                         s->d_cnt, s->d_loss);
+    ap::sg::mse_kernel<<<ap::grid_for(ny), 256, 0, st>>>(B, net.cout, R, margin, a[kSurrLayers], s->d_tb, map_w,
+                                                         s->d_g[0], s->d_lpart, s->d_cnt, s->d_loss);
     int cur = 0;
     for (int l = kSurrLayers - 1; l >= 0; --l) {
         float *din = l > 0 ? s->d_g[1 - cur] : nullptr;

@@ -39,27 +39,6 @@ __device__ __forceinline__ float rcp(float b) { return __fdividef(1.f, b); }
 // are bound by instruction issue).  exp(x) = 2^(x log2 e), results below 2^-126
 // taken as 0: next to the extreme pin's 1 they change no sum, and no gradient
 // in its fixed point.  The stage at 2M cells 108 -> 100.5 us, at 60k 31 -> 28.
-__device__ __forceinline__ ull pair_bits(float2 a) { return ((ull)__float_as_uint(a.y) << 32) | __float_as_uint(a.x); }
-__device__ __forceinline__ float2 bits_pair(ull v) {
-    return make_float2(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    ull r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
-    return bits_pair(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    ull r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
-    return bits_pair(r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    ull r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
-    return bits_pair(r);
-}
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 exp2_pair(float2 a) {
     const float2 t = mul2(a, both(1.44269504088896341f));
     float2 r;
