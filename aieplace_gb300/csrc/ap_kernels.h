@@ -198,6 +198,10 @@ void launch_perturb(int n_mov, const float *vx, const float *vy, const float *gx
                     float *ox, float *oy, const double *gmax, float coef_bw, float die_w, float die_h,
                     const float *w, const float *h, cudaStream_t st);
 
+// ---- host arrays --------------------------------------------------------------
+// device array -> the caller's memory, whose untouched pages it touches first
+cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t st);
+
 // ---- field solve ------------------------------------------------------------
 // Spectral solver state for an m x m grid (square, m a power of two, 32..4096).
 constexpr int kTcCandidates = 5;  // tensor-core solve variants the autotuner times

@@ -1317,7 +1317,8 @@ int ap_surrogate_forward(ap_surrogate *s, const float *x, int32_t batch, int32_t
     CKS(cudaMemcpy(s->d_a[0], x, sizeof(float) * batch * s->net.cin0 * RR, cudaMemcpyHostToDevice));
     ap::net_infer(s->net, batch, res, s->d_a[0], s->d_a, s->d_a[kSurrLayers], 0);
     CKS(cudaGetLastError());
-    CKS(cudaMemcpy(y, s->d_a[kSurrLayers], sizeof(float) * batch * s->net.cout * RR, cudaMemcpyDeviceToHost));
+    CKS(ap::copy_out(y, s->d_a[kSurrLayers], sizeof(float) * batch * s->net.cout * RR, 0));
+    CKS(cudaStreamSynchronize(0));
     return AP_OK;
 }
 
