@@ -39,6 +39,8 @@ struct WaArgs {
     double *partials;      // 2 per block over all bucket launches
     unsigned int *counter;
     int small_blocks;      // blocks of the three thread-per-net launches together
+    int all_blocks;        // and of all four
+    int bucket;            // batched form: the launch this record is of (0, 1, 2; 3: the larger nets)
     int block_nets;        // nets (lanes of the larger nets) per block, at least (<= 256: one per thread)
     double *out;           // [2]: HPWL, WA
     int mode;
@@ -264,11 +266,8 @@ int field_solver_clear_status(FieldSolver &f);
 void launch_split_bf16(int n, const float *src, __nv_bfloat16 *hi, __nv_bfloat16 *lo, cudaStream_t st);
 
 // ---- batched form: persistent launches (ap_persist.cuh) ----------------------
-// the persistent launches of one trial step; PS_WA is the WA launch of the
-// nets of more than 8 pins (it folds the sums), PS_WA2/4/8 those of the
-// thread-per-net buckets (2, 3-4 and 5-8 pins)
-enum { PS_UPDATE = 0, PS_SCATTER = 1, PS_RHO = 2, PS_WA = 3, PS_FIELD = 4, PS_GATHER = 5,
-       PS_WA2 = 6, PS_WA4 = 7, PS_WA8 = 8, PS_COUNT = 9 };
+// the persistent launches of one trial step
+enum { PS_UPDATE = 0, PS_SCATTER = 1, PS_RHO = 2, PS_WA = 3, PS_FIELD = 4, PS_GATHER = 5, PS_COUNT = 6 };
 
 // resident blocks of `kernel` on the whole GPU (dyn_smem bytes of dynamic
 // shared memory per block), or `fallback`
@@ -276,7 +275,6 @@ int wave_of(const void *kernel, int threads, int fallback, int dyn_smem = 0);
 // the grids the launchers give an instance's own launches (a persistent
 // record of the same instance runs the same blocks)
 int update_grid(const ScatterArgs &a);
-int scatter_grid(int n, int block_nodes);
 // whether the bin adds of n nodes over `blocks` blocks may use 32-bit tile slots
 bool tile32_exact(const Grid &g, int n, int blocks);
 int rho_grid(int nbins);
@@ -308,10 +306,10 @@ int field_rec_blocks(const FieldRec &r, int tile);
 // one persistent launch of a stage over the records `recs` (device memory)
 // with the grid persist_*_wave() (one wave of resident blocks)
 int persist_density_wave(int stage);
-int persist_wa_wave(int bucket);  // 0, 1, 2: the thread-per-net buckets; 3: the larger nets
+int persist_wa_wave();
 int persist_field_wave(int tile, int m);  // m: the largest grid of the launch
 void launch_persist_density(int stage, const PersistQueue &q, const void *recs, cudaStream_t st);
-void launch_persist_wa(int bucket, const PersistQueue &q, const WaArgs *recs, cudaStream_t st);
+void launch_persist_wa(const PersistQueue &q, const WaArgs *recs, cudaStream_t st);
 void launch_persist_field(const PersistQueue &q, const FieldRec *recs, int tile, int m, cudaStream_t st);
 
 }  // namespace ap

@@ -8,7 +8,7 @@
 // r holds items [start[r], start[r + 1])), and its resident blocks pull
 // items off a device queue (an atomic head) until the space is exhausted,
 // so instances of uneven size share the GPU without per-instance grids, and
-// the graph of a trial step holds nine kernel nodes instead of a dozen per
+// the graph of a trial step holds six kernel nodes instead of a dozen per
 // instance.  A record's blocks run the same body the
 // instance's own launch runs (VBlock{id, n} for blockIdx.x / gridDim.x), so
 // each instance's results are the same bit for bit as its own launches'.

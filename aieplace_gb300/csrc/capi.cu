@@ -1969,9 +1969,9 @@ struct PersistPlan {
     int *d_dep = nullptr;
     // queue heads and the field stage's done counters, laid out so that each
     // launch zeroes the counters of the launch before it on its stream as
-    // one range: [0] gather, [1] update, [2] scatter, [3] rho, [4..7] the
-    // four WA launches, [8] field, [9 ..) field done counters (the gather
-    // follows the field and the WA launches)
+    // one range: [0] gather, [1] update, [2] scatter, [3] rho, [4] WA, [5]
+    // field, [6 ..) field done counters (the gather follows the field and the
+    // WA launch)
     unsigned int *d_cnt = nullptr;
     int field_tile = 32;  // blocks of the field launch have 8 field_tile threads (32 or 64)
     int field_m = 0;      // the largest grid of the field launch
@@ -2032,18 +2032,12 @@ bool persist_supported(const ap_batch *b) {
     return true;
 }
 
-constexpr int kFieldDone = 9;  // first field done counter in PersistPlan::d_cnt
+constexpr int kFieldDone = 6;  // first field done counter in PersistPlan::d_cnt
 
 int stage_wave(int k) {
     switch (k) {
-    case PS_WA2:
-        return persist_wa_wave(0);
-    case PS_WA4:
-        return persist_wa_wave(1);
-    case PS_WA8:
-        return persist_wa_wave(2);
     case PS_WA:
-        return persist_wa_wave(3);
+        return persist_wa_wave();
     case PS_FIELD:
         return persist_field_wave(32, 512);  // not asked for: a field item is one block
     default:
@@ -2089,11 +2083,25 @@ int upload_stage(PersistPlan &pp, int k, const std::vector<T> &recs, const std::
 // launches would run it (enqueue_iteration).
 int plan_build(ap_batch *b, PersistPlan &pp) {
     plan_free(pp);
+    // Bin adds and density sums are exact integers however they are cut.  The
+    // bin adds take items small enough that those of 32 instances fill the
+    // resident blocks twice over and let the WA launch's blocks in between
+    // (a step of 32 instances of 5k-150k cells at overflow 0.97 / 0.05, items of
+    // 512, 1024, 2048 nodes, one round of equal items: 271 / 312, 264 / 316, 276 /
+    // 334, 271 / 380 us); the density sums one round of resident blocks (26 ->
+    // 22 us a stage).
+    long long rb = 0;
+    for (size_t i = 0; i < b->inst.size(); ++i)
+        if (b->active[i]) rb += rho_grid(b->inst[i]->p.bins_x * b->inst[i]->p.bins_y);
+    const int rw = std::max(1, stage_wave(PS_RHO));
+    const int rounds = (int)std::max(1ll, (rb + rw - 1) / rw);
+    constexpr int kItemNodes = 1024;
+    auto bins_blocks = [](int n) { return std::max(1, (n + kItemNodes - 1) / kItemNodes); };
     std::vector<ScatterArgs> upd, sct;
     std::vector<RhoArgs> rho;
     std::vector<WaArgs> wa;
     std::vector<GatherArgs> gat;
-    std::vector<int> bu, bs, br, bg, bw[4];
+    std::vector<int> bu, bs, br, bg, bw;
     std::vector<FieldRec> fld[4];
     for (size_t i = 0; i < b->inst.size(); ++i) {
         if (!b->active[i]) continue;
@@ -2107,7 +2115,7 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
         s.hi = h->n_real;
         s.rho_q = h->d_mov_q;
         if (s.hi > s.lo) {
-            bs.push_back(scatter_grid(s.hi - s.lo, s.block_nodes));
+            bs.push_back(bins_blocks(s.hi - s.lo));
             s.tile32 = tile32_exact(s.g, s.hi - s.lo, bs.back()) ? 1 : 0;
             sct.push_back(s);
         }
@@ -2115,17 +2123,15 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
             s.lo = h->n_real;
             s.hi = h->n_mov;
             s.rho_q = h->d_fill_q;
-            bs.push_back(scatter_grid(s.hi - s.lo, s.block_nodes));
+            bs.push_back(bins_blocks(s.hi - s.lo));
             s.tile32 = tile32_exact(s.g, s.hi - s.lo, bs.back()) ? 1 : 0;
             sct.push_back(s);
         }
         const RhoArgs ra = rho_args(h, RHO_LOOP, nullptr);
         rho.push_back(ra);
-        br.push_back(rho_grid(ra.nbins));
+        br.push_back((rho_grid(ra.nbins) + rounds - 1) / rounds);
         WaArgs wr = wa_args(h, h->d_px[0], h->d_py[0], 0.f, h->n_mov, WA_LOOP, nullptr);
-        const int all = wa_plan(wr);
-        for (int k = 0; k < 3; ++k) bw[k].push_back(wr.bucket_blocks[k]);
-        bw[3].push_back(all - wr.small_blocks);
+        wa_plan(wr);
         wa.push_back(wr);
         FieldRec fr[4];
         if (!field_records(h->fs, h->d_dens, h->d_exy, pp.field_tile, fr)) return AP_ERR_UNSUPPORTED;
@@ -2144,13 +2150,18 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
             bf.push_back(field_rec_blocks(fld[k][i], pp.field_tile));
             dep.push_back(k == 0 ? -1 : std::min(k - 1, 1) * ni + i);  // both halves of P3 wait for P2
         }
+    // the WA launches' records, those of the longest blocks first
+    std::vector<WaArgs> wall;
+    for (int k : {3, 2, 0, 1})
+        for (const WaArgs &w : wa) {
+            wall.push_back(w);
+            wall.back().bucket = k;
+            bw.push_back(k < 3 ? w.bucket_blocks[k] : w.all_blocks - w.small_blocks);
+        }
     int r = upload_stage(pp, PS_UPDATE, upd, bu);
     if (r == AP_OK) r = upload_stage(pp, PS_SCATTER, sct, bs);
     if (r == AP_OK) r = upload_stage(pp, PS_RHO, rho, br);
-    if (r == AP_OK) r = upload_stage(pp, PS_WA2, wa, bw[0]);
-    if (r == AP_OK) r = upload_stage(pp, PS_WA4, wa, bw[1]);
-    if (r == AP_OK) r = upload_stage(pp, PS_WA8, wa, bw[2]);
-    if (r == AP_OK) r = upload_stage(pp, PS_WA, wa, bw[3]);
+    if (r == AP_OK) r = upload_stage(pp, PS_WA, wall, bw);
     if (r == AP_OK) r = upload_stage(pp, PS_FIELD, fall, bf);
     if (r == AP_OK) r = upload_stage(pp, PS_GATHER, gat, bg);
     if (r != AP_OK) return r;
@@ -2169,7 +2180,7 @@ PersistQueue plan_queue(const ap_batch *b, int k, int reset_lo, int reset_n) {
     q.n_rec = pp.n_rec[k];
     q.chunk = pp.chunk[k];
     // PS_* -> counter slot (PersistPlan::d_cnt)
-    static const int head_slot[PS_COUNT] = {1, 2, 3, 7, 8, 0, 4, 5, 6};
+    static const int head_slot[PS_COUNT] = {1, 2, 3, 4, 5, 0};
     q.head = pp.d_cnt + head_slot[k];
     q.status = b->d_status;
     q.wait_ns = b->wait_ns;
@@ -2194,27 +2205,18 @@ int batch_sync(ap_batch *b) {
     return AP_OK;
 }
 
-// The four WA launches of a trial (stream `st`): the thread-per-net buckets,
-// then the larger nets, whose records fold the sums.
-void enqueue_persist_wa(ap_batch *b, cudaStream_t st) {
-    const PersistPlan &pp = b->plan;
-    const int stage[4] = {PS_WA2, PS_WA4, PS_WA8, PS_WA};
-    for (int k = 0; k < 4; ++k)
-        launch_persist_wa(k, plan_queue(b, stage[k], 0, 0), static_cast<const WaArgs *>(pp.d_recs[stage[k]]), st);
-}
-
-// The gather zeroes the counters of the field and the WA launches.
+// The gather zeroes the counters of the field and the WA launch.
 int gather_reset_n(const PersistPlan &pp) { return kFieldDone - 4 + pp.n_rec[PS_FIELD]; }
 
-// One trial step of every active instance as nine persistent launches: the
-// position update; the four WA launches on a second stream beside scatter ->
+// One trial step of every active instance as six persistent launches: the
+// position update; the WA launch on a second stream beside scatter ->
 // density/overflow -> field; the gather with each instance's accept / retry.
 int enqueue_persist(ap_batch *b, cudaStream_t st) {
     const PersistPlan &pp = b->plan;
     launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.d_recs[PS_UPDATE], st);
     CK(cudaEventRecord(b->wa_fork, st));
     CK(cudaStreamWaitEvent(b->wa_stream, b->wa_fork, 0));
-    enqueue_persist_wa(b, b->wa_stream);
+    launch_persist_wa(plan_queue(b, PS_WA, 0, 0), static_cast<const WaArgs *>(pp.d_recs[PS_WA]), b->wa_stream);
     CK(cudaEventRecord(b->wa_join, b->wa_stream));
     launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.d_recs[PS_SCATTER], st);
     launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.d_recs[PS_RHO], st);
@@ -2240,7 +2242,7 @@ int persist_profile(ap_batch *b, int n_trials, float *ms) {
         CK(cudaEventRecord(ev[0], st));
         launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.d_recs[PS_UPDATE], st);
         CK(cudaEventRecord(ev[1], st));
-        enqueue_persist_wa(b, st);
+        launch_persist_wa(plan_queue(b, PS_WA, 0, 0), static_cast<const WaArgs *>(pp.d_recs[PS_WA]), st);
         CK(cudaEventRecord(ev[2], st));
         launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.d_recs[PS_SCATTER], st);
         CK(cudaEventRecord(ev[3], st));
@@ -2434,12 +2436,10 @@ int ap_batch_get_info(ap_batch *b, ap_batch_info *info) {
     info->field_tile = b->tuned_tile;
     info->field_tune_ms[0] = b->tune_ms[0];
     info->field_tune_ms[1] = b->tune_ms[1];
-    for (int k = 0; k < 6; ++k) {  // the WA entry: the launch of the larger nets; its items: all four launches'
-        info->records[k] = b->plan.n_rec[k];
+    for (int k = 0; k < 6; ++k) {
+        info->records[k] = b->plan.n_rec[k] / (k == PS_WA ? 4 : 1);  // WA: four degree ranges an instance
         info->item_blocks[k] = b->plan.chunk[k];
-        info->items[k] = b->plan.items[k] + (k == PS_WA ? b->plan.items[PS_WA2] + b->plan.items[PS_WA4] +
-                                                              b->plan.items[PS_WA8]
-                                                        : 0);
+        info->items[k] = b->plan.items[k];
     }
     return AP_OK;
 }

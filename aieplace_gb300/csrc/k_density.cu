@@ -512,7 +512,7 @@ int launch_update(const ScatterArgs &a, cudaStream_t st) {
     return ub;
 }
 
-int scatter_grid(int n, int block_nodes) {
+static int scatter_grid(int n, int block_nodes) {
     // two of the three blocks that fit an SM, each a contiguous range of nodes
     // (fewer blocks: fewer tile flushes onto the dense core's bins): the third
     // would take the registers and shared memory that the WA launches beside it
@@ -1195,11 +1195,11 @@ __global__ void numerics_selftest_kernel(long long n, ull seed, int *mism) {
 }
 
 // ---- persistent launches of the batched form ------------------------------
-// Each record is one instance's launch of the stage (its arguments and its
-// grid as the launchers above would size it); the per-instance sums fold in
-// the record's last block, as in the instance's own launch.
+// Each record is one instance's launch of the stage: its arguments, and where
+// sums depend on it the grid that the launchers above give it (plan_build); an
+// instance's sums fold in its last block, as in its own launch.
 
-__global__ void __launch_bounds__(kThreads) persist_update_kernel(PersistQueue q, const ScatterArgs *recs) {
+__global__ void __launch_bounds__(kThreads, 5) persist_update_kernel(PersistQueue q, const ScatterArgs *recs) {
     persist_loop(q, recs, [](const ScatterArgs &a, VBlock vb, int) {
         update_body<false>(a, vb);
         if (arrive_last(a.counter, vb.n)) update_fold(a, vb.n);
@@ -1217,7 +1217,7 @@ __global__ void __launch_bounds__(kThreads) persist_rho_kernel(PersistQueue q, c
     });
 }
 
-__global__ void __launch_bounds__(kThreads, 4) persist_gather_kernel(PersistQueue q, const GatherArgs *recs) {
+__global__ void __launch_bounds__(kThreads, 5) persist_gather_kernel(PersistQueue q, const GatherArgs *recs) {
     persist_loop(q, recs, [](const GatherArgs &a, VBlock vb, int) {
         gather_body<GATHER_STEP, true>(a, vb);
         if (arrive_last(a.counter, vb.n)) gather_fold(a, vb.n);
@@ -1231,12 +1231,9 @@ int persist_density_wave(int stage) {
         if (!waves[0]) waves[0] = wave_of((const void *)persist_update_kernel, kThreads, 1216);
         return waves[0];
     case PS_SCATTER:
-        // two blocks per SM, not the three that fit: the WA launches run
-        // beside the scatter and need shared memory and warp slots too
         if (!waves[1]) {
             cudaFuncSetAttribute(persist_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem);
-            waves[1] = at_most_per_sm(
-                wave_of((const void *)persist_scatter_kernel, kScatterThreads, 304, kScatterSmem), 2);
+            waves[1] = wave_of((const void *)persist_scatter_kernel, kScatterThreads, 304, kScatterSmem);
         }
         return waves[1];
     case PS_RHO:

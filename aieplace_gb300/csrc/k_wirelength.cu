@@ -480,7 +480,8 @@ int wa_plan(WaArgs &a) {
         large += a.bucket_blocks[b];
     }
     a.small_blocks = a.bucket_blocks[0] + a.bucket_blocks[1] + a.bucket_blocks[2];
-    return a.small_blocks + large;
+    a.all_blocks = a.small_blocks + large;
+    return a.all_blocks;
 }
 
 // Positions (px, py) of all nodes -> the interleaved copy the WA kernels read.
@@ -513,49 +514,29 @@ void launch_wirelength(const WaArgs &a0, cudaStream_t st) {
     wa_large_kernel<<<large, kThreads, 0, st>>>(a);
 }
 
-// The batched form: the four bucket launches of every instance as four
-// persistent launches (one record per instance each; registers sized per
-// bucket as in the instance's own launches); the last one folds each
-// instance's sums in the record's last block, after the other three ended.
-template <int D, int B>
-__global__ void __launch_bounds__(kThreads, D == 8 ? 3 : 4) persist_wa_small_kernel(PersistQueue q, const WaArgs *recs) {
-    persist_loop(q, recs, [](const WaArgs &a, VBlock vb, int) { wa_small_body<D, B>(a, vb); });
-}
-
-__global__ void __launch_bounds__(kThreads, 4) persist_wa_large_kernel(PersistQueue q, const WaArgs *recs) {
+// The batched form: the four bucket launches of every instance as records of
+// one persistent launch (WaArgs::bucket), so that the buckets with few blocks
+// fill the GPU together; an instance's sums fold in the last of all its blocks.
+// (As four launches one after the other, the 3-4- and 5-8-pin nets on a third
+// and a tenth of the resident blocks: 186 us for 32 instances, 126 in one.)
+__global__ void __launch_bounds__(kThreads, 3) persist_wa_kernel(PersistQueue q, const WaArgs *recs) {
     persist_loop(q, recs, [](const WaArgs &a, VBlock vb, int) {
-        wa_large_body(a, vb);
-        if (arrive_last(a.counter, vb.n)) wa_fold(a, a.small_blocks + vb.n);
+        if (a.bucket == 0) wa_small_body<2, 0>(a, vb);
+        else if (a.bucket == 1) wa_small_body<4, 1>(a, vb);
+        else if (a.bucket == 2) wa_small_body<8, 2>(a, vb);
+        else wa_large_body(a, vb);
+        if (arrive_last(a.counter, a.all_blocks)) wa_fold(a, a.all_blocks);
     });
 }
 
-int persist_wa_wave(int bucket) {
-    static int waves[4] = {0, 0, 0, 0};
-    if (bucket < 0 || bucket > 3) return 0;
-    if (!waves[bucket]) {
-        const void *k[4] = {(const void *)persist_wa_small_kernel<2, 0>, (const void *)persist_wa_small_kernel<4, 1>,
-                            (const void *)persist_wa_small_kernel<8, 2>, (const void *)persist_wa_large_kernel};
-        waves[bucket] = wave_of(k[bucket], kThreads, 1216);
-    }
-    return waves[bucket];
+int persist_wa_wave() {
+    static int wave = 0;
+    if (!wave) wave = wave_of((const void *)persist_wa_kernel, kThreads, 456);
+    return wave;
 }
 
-void launch_persist_wa(int bucket, const PersistQueue &q, const WaArgs *recs, cudaStream_t st) {
-    const int w = persist_wa_wave(bucket);
-    switch (bucket) {
-    case 0:
-        persist_wa_small_kernel<2, 0><<<w, kThreads, 0, st>>>(q, recs);
-        break;
-    case 1:
-        persist_wa_small_kernel<4, 1><<<w, kThreads, 0, st>>>(q, recs);
-        break;
-    case 2:
-        persist_wa_small_kernel<8, 2><<<w, kThreads, 0, st>>>(q, recs);
-        break;
-    default:
-        persist_wa_large_kernel<<<w, kThreads, 0, st>>>(q, recs);
-        break;
-    }
+void launch_persist_wa(const PersistQueue &q, const WaArgs *recs, cudaStream_t st) {
+    persist_wa_kernel<<<persist_wa_wave(), kThreads, 0, st>>>(q, recs);
 }
 
 }  // namespace ap

@@ -219,7 +219,7 @@ class Placer:
 
 class BatchPlacer:
     """Independent placements stepped together (ap_create_batch): one CUDA
-    graph launch advances one trial step of every active instance, as nine
+    graph launch advances one trial step of every active instance, as six
     persistent launches over all instances ("persistent", the default where
     it serves every instance) or as every instance's own launches in
     parallel branches ("graph")."""

@@ -276,7 +276,7 @@ def profile_mode(args):
 def batch_mode(args):
     """Batched form: n instances (cell counts LogUniform[5k, 150k], bins 128..512)
     stepped together.  Reports instance-iterations per second over K graph
-    launches for the persistent form (nine persistent launches per trial step
+    launches for the persistent form (six persistent launches per trial step
     over all instances, FP32 field, the default), for the graph of
     per-instance branches with the FP32 field and with the BF16x3 tensor-core
     field, the wall time until every instance is below 10% overflow, and the

@@ -304,8 +304,8 @@ int ap_restore(ap_handle *h, const void *buf, size_t bytes);
  * design per run (Placer::run, AIEplace.cpp:44-76); small designs cannot fill
  * a GB300 alone, so a batch advances every active instance by one trial step
  * per launch of one CUDA graph, in one of two forms:
- *   AP_BATCH_PERSISTENT  nine persistent kernels per trial step, one per stage
- *                        (position update, four WA launches by net degree, bin
+ *   AP_BATCH_PERSISTENT  six persistent kernels per trial step, one per stage
+ *                        (position update, WA gradient, bin
  *                        scatter, density/overflow, field solve, gather), each
  *                        over all instances: its resident blocks pull
  *                        (instance, block)
