@@ -380,6 +380,28 @@ struct VBlock {
 };
 __device__ __forceinline__ VBlock grid_block() { return VBlock{(int)blockIdx.x, (int)gridDim.x}; }
 
+// Programmatic dependents: the blocks of a launch made with launch_dependent
+// start while the launch before it on the stream drains, and wait for its
+// results in grid_wait(); grid_release() lets the next launch's blocks start.
+// No-ops in and after ordinary launches.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... Args>
+inline void launch_dependent(void (*kernel)(P...), int blocks, int threads, int smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Last-block detection for grid-wide reductions without waiting: every block
 // publishes its partials, the block that arrives last of `blocks` reduces
 // them in block order (so the result does not depend on scheduling) and

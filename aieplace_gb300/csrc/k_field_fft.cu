@@ -649,10 +649,7 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, co
 }
 
 // ---- launches of one solve ----------------------------------------------------
-// P2 and P3 are programmatic dependents of the pass before: their blocks
-// start while it drains and wait for its results here.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// P2 and P3 are programmatic dependents of the pass before.
 
 // run only if gate is null or (1 << *gate) & mask
 __device__ __forceinline__ bool gated_off(const int *gate, int mask) { return gate && !((1 << *gate) & mask); }
@@ -717,19 +714,8 @@ int launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask, co
         }
     }
     if (!maps) fft_kernel<M, NT, 0><<<blocks, NT, SM, st>>>(a, gate, mask);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = SM;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(fft_blocks(M, NT, 1, M));
-    cudaLaunchKernelEx(&cfg, fft_kernel<M, NT, 1>, a, gate, mask);
-    cfg.gridDim = dim3(fft_blocks(M, NT, 2, M));
-    cudaLaunchKernelEx(&cfg, fft_kernel<M, NT, 2>, a, gate, mask);
+    launch_dependent(fft_kernel<M, NT, 1>, fft_blocks(M, NT, 1, M), NT, SM, st, a, gate, mask);
+    launch_dependent(fft_kernel<M, NT, 2>, fft_blocks(M, NT, 2, M), NT, SM, st, a, gate, mask);
     return blocks;
 }
 

@@ -1,0 +1,51 @@
+"""The bin adds as a dependent launch of the position update.
+
+A loop trial's bin adds start while its update drains where they take at most
+a block an SM (152), and as an ordinary launch beyond.  The batched form's
+stages are ordinary launches of the same sums, so a batch of one gives the
+same bits: at the last size of the first rule, the first of the second, with
+filler cells (two launches of bin adds in a row) and at a single block.
+"""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BLOCK_NODES = 2048  # the batched form's grid policy
+LINE = 152 * BLOCK_NODES
+
+
+@pytest.fixture(scope="module")
+def ap():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from aieplace_gb300 import build
+
+    build.build()
+    import aieplace_gb300
+
+    return aieplace_gb300
+
+
+@pytest.mark.parametrize("cells,bins,fillers", [(200, 32, 0), (LINE, 256, 0), (LINE + 1, 256, 0), (LINE - 1, 256, 1)])
+def test_dependent_bin_adds_match_ordinary_launches(ap, cells, bins, fillers):
+    nl = ap.synth.generate(dict(num_cells=cells, num_nets=cells, num_macros=0, num_pads=24, unit_cells=1, degree_mix=0,
+                                locality=0.0, window=64, target_density=0.9,
+                                die_side=float(math.ceil(math.sqrt(cells / 0.8))), bins=bins), seed=3)
+    with ap.BatchPlacer([nl], filler_cells=fillers) as b:
+        b.initialize_placement(seed=7, sigma=1.0)
+        b.step(16)
+        bx, by = b.positions(0)
+        bs = b.stats(0)
+    with ap.Placer(nl, block_nodes=BLOCK_NODES, filler_cells=fillers) as p:
+        p.initialize_placement(seed=7, sigma=1.0)
+        p.step_async(16)
+        x, y = p.positions()
+        s = p.stats()
+    np.testing.assert_array_equal(bx, x)
+    np.testing.assert_array_equal(by, y)
+    assert bs["hpwl"] == s["hpwl"] and bs["overflow"] == s["overflow"]
