@@ -688,13 +688,30 @@ int rho_grid(int nbins) {
 
 void launch_rho(const RhoArgs &a, cudaStream_t st) { rho_kernel<<<rho_grid(a.nbins), kThreads, 0, st>>>(a); }
 
+// What the accept / retry decision of one trial needs, each part worked out by
+// a warp of its own (step_fold): in FP32 where the oracle's bounds allow (FP64
+// sqrt and pow cost microseconds on this part's narrow FP64 pipe).
+struct StepParts {
+    double du, dv2, dg2;        // |u_new - u|^2, |v_new - v|^2, |g_new - g|^2
+    float ahat;                 // re-predicted step sqrt(dv2 / dg2)
+    int finite;
+    double tau, tau_abs, gamma; // the trial's overflow, the next evaluation's smoothing
+    float f_gamma;
+    double lambda;              // density weight after an accepted trial
+    float f_lambda;
+    float a_next[2], mom[2];    // momentum without [0] and with [1] a restart
+    double least;               // steps below this are retried
+    unsigned long long t_ns;    // device clock
+    int accepted;               // finish_trial's result
+};
+
 // The trajectory record of the trial just decided (trial number sc->evals - 1).
-__device__ void log_trial(DevScalars *sc, int accepted) {
+__device__ void log_trial(const DevScalars *sc, const StepParts &p) {
     if (!sc->traj) return;
     TrajRec r;
     r.eval = sc->evals - 1;
     r.iteration = sc->iteration;
-    r.accepted = accepted;
+    r.accepted = p.accepted;
     r.field_mode = sc->field_mode;
     r.hpwl = sc->t_hpwl;
     r.overflow = sc->t_tau;
@@ -703,47 +720,13 @@ __device__ void log_trial(DevScalars *sc, int accepted) {
     r.alpha = sc->alpha;
     r.gamma = sc->gamma;
     r.surr_err = sc->surr_err;
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    r.t_ns = t;
+    r.t_ns = p.t_ns;
     sc->traj[(unsigned)r.eval % (unsigned)sc->traj_cap] = r;
 }
 
-// Accept / retry decision of one trial (one thread).  Mirrors or_step in the
-// oracle: backtracking while the re-predicted step falls below 0.95 of the
-// step tried; on acceptance the momentum restart test, the density-penalty
-// update (RePlAce: mu = mu_max^(1 - dHPWL/ref) in [mu_min, mu_max]) and the
-// momentum coefficients of the next iteration.
-__device__ void finish_trial(DevScalars *sc, double dv2, double dg2) {
-    sc->sum_dv2 = dv2;
-    sc->sum_dg2 = dg2;
-    sc->evals += 1;
-    // step and momentum arithmetic in FP32 (single thread; FP64 sqrt/pow here
-    // cost microseconds per trial on the narrow FP64 pipe)
-    const double ahat = dg2 > 0.0 ? (double)(sqrtf((float)dv2) / sqrtf((float)dg2)) : 0.0;
-    if (!isfinite(ahat) || !isfinite(dv2) || !isfinite(dg2)) {
-        sc->status = 9;
-        log_trial(sc, -1);
-        return;
-    }
-    if (ahat <= 0.95 * sc->alpha && sc->backtracks < sc->max_backtracks) {
-        sc->alpha = ahat;
-        sc->backtracks += 1;
-        log_trial(sc, 0);
-        return;
-    }
-    bool restart = false;
-    if (sc->restart_mode == 2) restart = true;
-    if (sc->restart_mode == 3) restart = sc->t_du < sc->du_prev;
-    if (sc->restart_mode == 4) restart = sc->t_tau > sc->tau_prev;
-    sc->du_prev = sc->t_du;
-    sc->tau_prev = sc->t_tau;
-    sc->alpha = ahat;
-    sc->a_k = restart ? 1.0 : sc->a_next;
-    if (restart && sc->restart_mode != 2) sc->restarts += 1;
-    const float ak = (float)sc->a_k, an = 0.5f * (1.0f + sqrtf(4.0f * ak * ak + 1.0f));
-    sc->a_next = (double)an;
-    sc->mom = (double)((ak - 1.0f) / an);
+// The density weight after an accepted trial (RePlAce: mu = mu_max^(1 -
+// dHPWL/ref) in [mu_min, mu_max]).
+__device__ __forceinline__ double lambda_of(const DevScalars *sc) {
     const float pc = (float)(sc->t_hpwl - sc->hpwl_prev) / (float)sc->ref_dh;
     const float mmax = (float)sc->mu_max, mmin = (float)sc->mu_min;
     float mu = pc < 0.0f ? mmax : exp2f(log2f(mmax) * (1.0f - pc));
@@ -751,7 +734,44 @@ __device__ void finish_trial(DevScalars *sc, double dv2, double dg2) {
     // capped where the density term dominates completely: keeps the FP32
     // products finite when the target overflow is out of reach (lambda would
     // otherwise grow 5% per iteration until it overflows)
-    sc->lambda = fmin(sc->lambda * mu, kLambdaMax);
+    return fmin(sc->lambda * mu, kLambdaMax);
+}
+
+// Accept / retry decision of one trial (one thread): 1, 0, or -1 where the
+// trial is not finite.  Mirrors or_step in the oracle: backtracking while the
+// re-predicted step falls below 0.95 of the step tried; on acceptance the
+// momentum restart test, the density weight and the momentum coefficients of
+// the next iteration.  The FP32 copies (publish_f32) go along: ahat and mom are
+// floats.
+__device__ __forceinline__ int finish_trial(DevScalars *sc, const StepParts &p) {
+    sc->sum_dv2 = p.dv2;
+    sc->sum_dg2 = p.dg2;
+    sc->evals += 1;
+    if (!p.finite) {
+        sc->status = 9;
+        return -1;
+    }
+    const double ahat = (double)p.ahat;
+    const bool retry = ahat <= p.least && sc->backtracks < sc->max_backtracks;
+    sc->alpha = ahat;
+    sc->f_alpha = p.ahat;
+    if (retry) {
+        sc->backtracks += 1;
+        return 0;
+    }
+    bool restart = false;
+    if (sc->restart_mode == 2) restart = true;
+    if (sc->restart_mode == 3) restart = sc->t_du < sc->du_prev;
+    if (sc->restart_mode == 4) restart = sc->t_tau > sc->tau_prev;
+    sc->du_prev = sc->t_du;
+    sc->tau_prev = sc->t_tau;
+    sc->a_k = restart ? 1.0 : sc->a_next;
+    if (restart && sc->restart_mode != 2) sc->restarts += 1;
+    sc->a_next = (double)p.a_next[restart ? 1 : 0];
+    sc->f_mom = p.mom[restart ? 1 : 0];
+    sc->mom = (double)sc->f_mom;
+    sc->lambda = p.lambda;
+    sc->f_lambda = p.f_lambda;
     sc->hpwl_prev = sc->t_hpwl;
     sc->hpwl = sc->t_hpwl;
     sc->wa = sc->t_wa;
@@ -760,7 +780,7 @@ __device__ void finish_trial(DevScalars *sc, double dv2, double dg2) {
     sc->backtracks = 0;
     sc->cur = 1 - sc->cur;
     sc->iteration += 1;
-    log_trial(sc, 1);
+    return 1;
 }
 
 // MODE: GATHER_STEP, or -1 for the mode in the arguments (a loop trial's gather
@@ -992,66 +1012,132 @@ struct Strided {
 // A loop trial's end, in the gather's last block: the gather's own sum, the
 // position update's two and the overflow's two (their kernels leave the
 // block partials to this block, so that none of them ends in a fold the next
-// launch waits for), then the accept / retry decision.  The scalars are
-// worked on in shared memory: one load and one store of the whole block
-// instead of a chain of dependent accesses by one thread.
+// launch waits for), then the accept / retry decision.
+// Nothing runs beside it, so its latency is the trial's: the scalars are
+// worked on in shared memory (one load and one store of the whole block), the
+// three FP64 sums share one warp's adds (an FP64 instruction of a warp holds
+// the pipe for tens of cycles), and what the decision needs is worked out by a
+// warp each.  (By one thread, after three FP64 sums of their own, the fold
+// took 4.9 us; a trial with it / as here: 576 cells 23.4 / 19.4 us, 20k 27.4 /
+// 24.9, 60k 32.5 / 30.5, 200k 52.8 / 50.9.)
 __device__ __forceinline__ void step_fold(const GatherArgs &a, int nb) {
-    static_assert(sizeof(DevScalars) % 4 == 0, "whole words");
+    static_assert(sizeof(DevScalars) % 4 == 0 && sizeof(DevScalars) / 4 <= kThreads, "a word a thread");
+    static_assert(kThreads == 256, "eight warps' sums");
     __shared__ __align__(8) DevScalars sc;
-    __shared__ double fsum[3][32];
-    __shared__ long long isum[2][32];
+    __shared__ StepParts part;
+    __shared__ float fsum[3][8];
+    __shared__ long long isum[2][8];
     constexpr int words = (int)(sizeof(DevScalars) / 4);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (int)blockDim.x >> 5;
-    for (int t = tid; t < words; t += blockDim.x)
-        reinterpret_cast<int *>(&sc)[t] = __ldcg(reinterpret_cast<const int *>(a.sc) + t);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int word = tid < words ? __ldcg(reinterpret_cast<const int *>(a.sc) + tid) : 0;
+    longlong2 ov[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        ov[u] = tid + u * kThreads < a.n_rho
+                    ? __ldcg(reinterpret_cast<const longlong2 *>(a.rho_partials) + tid + u * kThreads)
+                    : make_longlong2(0ll, 0ll);
     Strided s[3];
     s[0].load(reinterpret_cast<const float *>(a.partials) + 1, nb, 4);
     s[1].load(a.upd_partials, a.n_upd, 2);
     s[2].load(a.upd_partials + 1, a.n_upd, 2);
-    long long o = 0, oa = 0;
-    for (int i = tid; i < a.n_rho; i += blockDim.x) {
+    if (tid < words) reinterpret_cast<int *>(&sc)[tid] = word;
+    long long o = ov[0].x + ov[1].x, oa = ov[0].y + ov[1].y;
+    for (int i = tid + 2 * kThreads; i < a.n_rho; i += kThreads) {
         o += __ldcg(a.rho_partials + 2 * i);
         oa += __ldcg(a.rho_partials + 2 * i + 1);
     }
+    float v[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float v = warp_sum(s[k].sum());
-        if (lane == 0) fsum[k][wid] = (double)v;
-    }
+    for (int k = 0; k < 3; ++k) v[k] = s[k].sum();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = warp_sum(v[k]);
     o = warp_sum(o);
     oa = warp_sum(oa);
     if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) fsum[k][wid] = v[k];
         isum[0][wid] = o;
         isum[1][wid] = oa;
     }
     __syncthreads();
-    if (wid == 0) {
-        double d[3];
+    switch (wid) {
+    case 0: {
+        // sum k in lanes 8k .. 8k + 7, in the order of a warp's sum of eight
+        double d = lane < 24 ? (double)fsum[lane >> 3][lane & 7] : 0.0;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) d[k] = warp_sum(lane < nw ? fsum[k][lane] : 0.0);
-        o = warp_sum(lane < nw ? isum[0][lane] : 0ll);
-        oa = warp_sum(lane < nw ? isum[1][lane] : 0ll);
+        for (int t = 4; t > 0; t >>= 1) d += __shfl_xor_sync(0xffffffffu, d, t);
+        if (lane == 16 && !a.n_upd) d = sc.t_dv2;  // the update's own kernel folded it
+        const float root = sqrtf((float)d), root_dv = __shfl_sync(0xffffffffu, root, 16);
+        const bool fin = __all_sync(0xffffffffu, isfinite(d) || (lane != 0 && lane != 16));
         if (lane == 0) {
-            if (a.n_upd) {
-                sc.t_du = d[1];
-                sc.t_dv2 = d[2];
-            }
-            if (a.n_rho) {
-                overflow_of(&sc, o, oa, sc.t_tau, sc.t_tau_abs);
-                sc.gamma_next = gamma_of(&sc, sc.t_tau);
-                sc.field_mode = kFieldExact;
-            }
-            // the next evaluation's WA smoothing: this trial's gamma(tau),
-            // whether the trial is accepted or not
-            sc.gamma = sc.gamma_next;
-            finish_trial(&sc, sc.t_dv2, d[0]);
-            publish_f32(&sc);
-            *a.counter = 0u;
+            const float ahat = d > 0.0 ? root_dv / root : 0.f;
+            part.dg2 = d;
+            part.ahat = ahat;
+            part.finite = fin && isfinite(ahat);
         }
+        if (lane == 8) part.du = a.n_upd ? d : sc.t_du;
+        if (lane == 16) part.dv2 = d;
+        break;
+    }
+    case 1:
+        o = lane < 8 ? isum[0][lane] : 0ll;
+        oa = lane < 8 ? isum[1][lane] : 0ll;
+#pragma unroll
+        for (int t = 4; t > 0; t >>= 1) {
+            o += __shfl_xor_sync(0xffffffffu, o, t);
+            oa += __shfl_xor_sync(0xffffffffu, oa, t);
+        }
+        if (lane == 0) {
+            double tau = sc.t_tau, tau_abs = sc.t_tau_abs, gamma = sc.gamma_next;
+            if (a.n_rho) {
+                overflow_of(&sc, o, oa, tau, tau_abs);
+                gamma = gamma_of(&sc, tau);
+            }
+            part.tau = tau;
+            part.tau_abs = tau_abs;
+            part.gamma = gamma;
+            part.f_gamma = (float)gamma;
+        }
+        break;
+    case 2:
+        if (lane == 0) {
+            part.lambda = lambda_of(&sc);
+            part.f_lambda = (float)part.lambda;
+        }
+        break;
+    case 3:
+        if (lane < 2) {
+            const float ak = lane ? 1.0f : (float)sc.a_next, an = 0.5f * (1.0f + sqrtf(4.0f * ak * ak + 1.0f));
+            part.a_next[lane] = an;
+            part.mom[lane] = (ak - 1.0f) / an;
+        }
+        break;
+    case 4:
+        if (lane == 0) {
+            part.least = 0.95 * sc.alpha;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(part.t_ns));
+        }
+        break;
+    default:
+        break;
     }
     __syncthreads();
-    for (int t = tid; t < words; t += blockDim.x)
-        reinterpret_cast<int *>(a.sc)[t] = reinterpret_cast<const int *>(&sc)[t];
+    if (tid == 0) {
+        sc.t_du = part.du;
+        sc.t_dv2 = part.dv2;
+        sc.t_tau = part.tau;
+        sc.t_tau_abs = part.tau_abs;
+        if (a.n_rho) sc.field_mode = kFieldExact;
+        // the next evaluation's WA smoothing: this trial's gamma(tau),
+        // whether the trial is accepted or not
+        sc.gamma = sc.gamma_next = part.gamma;
+        sc.f_gamma = part.f_gamma;
+        part.accepted = finish_trial(&sc, part);
+        *a.counter = 0u;
+    }
+    __syncthreads();
+    if (tid < words) reinterpret_cast<int *>(a.sc)[tid] = reinterpret_cast<const int *>(&sc)[tid];
+    if (tid == kThreads - 32) log_trial(&sc, part);
 }
 
 // The sums of partials [0, nb) of the initial evaluations into the device
