@@ -382,8 +382,11 @@ __device__ __forceinline__ VBlock grid_block() { return VBlock{(int)blockIdx.x, 
 
 // Programmatic dependents: the blocks of a launch made with launch_dependent
 // start while the launch before it on the stream drains, and wait for its
-// results in grid_wait(); grid_release() lets the next launch's blocks start.
-// No-ops in and after ordinary launches.
+// results in grid_wait(); grid_release() lets the next launch's blocks start
+// earlier still.  No-ops in and after ordinary launches.  Outside a graph the
+// boundary between two ordinary launches is rounded up to 2.05 us on this part
+// (kernels of 0.4 - 2.2 us of work follow each other every 4.1 us, dependent
+// ones every work + 0.6 us); in a graph it is 0.5 us, 0.3 us for dependents.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -413,9 +416,12 @@ __device__ __forceinline__ bool arrive_last(unsigned int *counter, int blocks) {
         __threadfence();
         const unsigned int t = atomicAdd(counter, 1u);
         last = (t == (unsigned int)blocks - 1u);
+        // after the add, by the thread that made it: the barrier passes what it
+        // has seen on to the block (a fence of every thread would wait for the
+        // stores of all of them)
+        if (last) __threadfence();
     }
     __syncthreads();
-    if (last) __threadfence();
     return last;
 }
 

@@ -274,6 +274,7 @@ __device__ __forceinline__ void update_fold(const ScatterArgs &a, int nb) {
 
 __global__ void __launch_bounds__(kThreads) update_kernel(ScatterArgs a) {
     grid_release();
+    grid_wait();
     update_body<true>(a, grid_block());
     if (a.no_fold) return;  // uniform: an earlier chunk of a chunked update, or the gather folds
     // the partials of this launch and of the chunks before it (launched
@@ -316,19 +317,36 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs &a, VBlock vb) {
     const int per = (n + vb.n - 1) / vb.n;
     const int r_lo = min(n, vb.id * per), r_hi = min(n, r_lo + per);
     const int tid = threadIdx.x, lane = tid & 31;
+    // a node's raw inputs (update mode: its record; plain mode: x, y, w, h as
+    // bits), loaded two iterations ahead: the loads of the next two nodes are
+    // in flight while this one is added, those of the first two while the tile
+    // is placed
+    auto load_raw = [&](int i, int &rb, int4 &ro) {
+        rb = kRecNone;
+        ro = make_int4(0, 0, 0, 0);
+        if (i >= r_hi) return;
+        const int node = a.lo + i;
+        if (a.update) {
+            rb = __ldg(a.rec_bin + node);
+            ro = __ldg(a.rec_ov + node);
+        } else {
+            rb = 0;
+            ro = make_int4(__float_as_int(__ldg(a.px + node)), __float_as_int(__ldg(a.py + node)),
+                           __float_as_int(__ldg(a.w + node)), __float_as_int(__ldg(a.h + node)));
+        }
+    };
+    int next_b[2];  // two nodes ahead
+    int4 next_o[2];
+    load_raw(r_lo + tid, next_b[0], next_o[0]);
+    load_raw(r_lo + tid + kScatterThreads, next_b[1], next_o[1]);
     // 1. a sample of the range, its first kScatterThreads nodes (one per
     //    thread, kept in registers): their mean base bin places the tiles
-    int sb = kRecNone;
-    if (r_lo + tid < r_hi) {
-        const int node = a.lo + r_lo + tid;
-        if (a.update) {
-            sb = __ldg(a.rec_bin + node);
-        } else {
-            int c0, c1, r0, r1;
-            sb = make_rec(g, __ldg(a.px + node), __ldg(a.py + node), __ldg(a.w + node), __ldg(a.h + node), c0, c1,
-                          r0, r1)
-                     .bin;
-        }
+    int sb = next_b[0];
+    if (!a.update && r_lo + tid < r_hi) {
+        int c0, c1, r0, r1;
+        sb = make_rec(g, __int_as_float(next_o[0].x), __int_as_float(next_o[0].y), __int_as_float(next_o[0].z),
+                      __int_as_float(next_o[0].w), c0, c1, r0, r1)
+                 .bin;
     }
     const bool valid = sb >= 0;
     const int scol = valid ? rec_c0(sb) : 0, srow = valid ? rec_r0(sb) : 0;
@@ -398,27 +416,6 @@ __device__ __forceinline__ void scatter_body(const ScatterArgs &a, VBlock vb) {
         }
     };
     int had = 0;  // this thread added to the tile
-    // a node's raw inputs (update mode: its record; plain mode: x, y, w, h as
-    // bits), loaded two iterations ahead: the loads of the next two nodes are
-    // in flight while this one is added
-    auto load_raw = [&](int i, int &rb, int4 &ro) {
-        rb = kRecNone;
-        ro = make_int4(0, 0, 0, 0);
-        if (i >= r_hi) return;
-        const int node = a.lo + i;
-        if (a.update) {
-            rb = __ldg(a.rec_bin + node);
-            ro = __ldg(a.rec_ov + node);
-        } else {
-            rb = 0;
-            ro = make_int4(__float_as_int(__ldg(a.px + node)), __float_as_int(__ldg(a.py + node)),
-                           __float_as_int(__ldg(a.w + node)), __float_as_int(__ldg(a.h + node)));
-        }
-    };
-    int next_b[2];  // two nodes ahead
-    int4 next_o[2];
-    load_raw(r_lo + tid, next_b[0], next_o[0]);
-    load_raw(r_lo + tid + kScatterThreads, next_b[1], next_o[1]);
     for (int base = r_lo; base < r_hi; base += kScatterThreads) {
         const int i = base + tid;
         const int node = a.lo + i;
@@ -512,7 +509,7 @@ int update_grid(const ScatterArgs &a) {
 int launch_update(const ScatterArgs &a, cudaStream_t st) {
     if (!a.update || a.n_mov <= 0) return 0;
     const int ub = update_grid(a);
-    update_kernel<<<ub, kThreads, 0, st>>>(a);
+    launch_dependent(update_kernel, ub, kThreads, 0, st, a);
     return ub;
 }
 
@@ -1187,6 +1184,7 @@ __device__ __forceinline__ void gather_fold(const GatherArgs &a, int nb) {
 // (a loop trial's: five blocks an SM, 42.3 -> 38.9 us at 2M cells against four)
 template <int MODE, bool PAIRS>
 __global__ void __launch_bounds__(kThreads, MODE == GATHER_STEP ? 5 : 4) gather_kernel(GatherArgs a) {
+    grid_wait();
     gather_body<MODE, PAIRS>(a, grid_block());
     if (a.mode == GATHER_FORCE_ONLY || a.mode == GATHER_NODE_OUT) return;
     if (arrive_last(a.counter, gridDim.x)) gather_fold(a, gridDim.x);
@@ -1208,8 +1206,10 @@ int gather_grid(int n_mov, int block_nodes) {
 
 void launch_gather(const GatherArgs &a, cudaStream_t st) {
     const int blocks = gather_grid(a.n_mov, a.block_nodes);
+    // (a trial with this launch and the update's ordinary / dependent: 576 cells
+    // 19.8 / 19.4 us, 5k 22.7 / 22.2, 60k 30.7 / 30.2, 200k 50.5 / 50.1)
     if (a.mode == GATHER_STEP && a.exy)
-        gather_kernel<GATHER_STEP, true><<<blocks, kThreads, 0, st>>>(a);
+        launch_dependent(gather_kernel<GATHER_STEP, true>, blocks, kThreads, 0, st, a);
     else
         gather_kernel<-1, false><<<blocks, kThreads, 0, st>>>(a);
 }

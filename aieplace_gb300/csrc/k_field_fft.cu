@@ -580,6 +580,23 @@ template <int NT, bool MAPS = false>
 __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, const RhoArgs *rho = nullptr) {
     constexpr int M = kDense;
     __shared__ long long red[NT / 32][2];
+    // 256 threads a product; the two products of S3 and of S4 side by side
+    // (512 threads) or in turn
+    const int t = threadIdx.x & 255, z = threadIdx.x >> 8, i = t >> 4, j = t & 15;
+    // every load up front (a 576-cell trial 21.0 -> 20.4 us)
+    const float *tab = reinterpret_cast<const float *>(a.tab);
+    constexpr int N = M * M / NT;
+    float tc[N], ts[N], wx[2], wy[2];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        tc[n] = __ldg(tab + threadIdx.x + n * NT);
+        ts[n] = __ldg(tab + M * M + threadIdx.x + n * NT);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        wx[r] = __ldg(a.wx + i + 16 * r);
+        wy[r] = __ldg(a.wy + j + 16 * r);
+    }
     if constexpr (MAPS) {
         static_assert(NT == M * M / 2, "a pair of bins per thread");
         long long over = 0, over_abs = 0;
@@ -589,20 +606,16 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, co
         sm.b[0][2 * p / M][2 * p % M + 1] = d.y;
         put_overflow<NT>(over, over_abs, red);
     }
-    const float *tab = reinterpret_cast<const float *>(a.tab);
-    for (int t = threadIdx.x; t < M * M; t += NT) {
-        const int k = t / M, i = t % M;
-        const float c = __ldg(tab + t), s = __ldg(tab + M * M + t);
-        sm.c[k][i] = c;
-        sm.ct[i][k] = c;
-        sm.st[i][k] = s;
-        if constexpr (!MAPS) sm.b[0][k][i] = __ldg(a.d + t);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        const int e = (int)threadIdx.x + n * NT, k = e / M, x = e % M;
+        sm.c[k][x] = tc[n];
+        sm.ct[x][k] = tc[n];
+        sm.st[x][k] = ts[n];
+        if constexpr (!MAPS) sm.b[0][k][x] = __ldg(a.d + e);
     }
     __syncthreads();
     if constexpr (MAPS) get_overflow<NT>(*rho, 0, red);
-    // 256 threads a product; the two products of S3 and of S4 side by side
-    // (512 threads) or in turn
-    const int t = threadIdx.x & 255, z = threadIdx.x >> 8, i = t >> 4, j = t & 15;
     float acc[2][2];
     auto put = [&](float (*D)[kDenseLd]) {
 #pragma unroll
@@ -622,7 +635,7 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, co
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int u = i + 16 * r, v = j + 16 * q;
-                const float2 p = spectral(acc[r][q], a.scale, u, v, __ldg(a.wx + u), __ldg(a.wy + v));
+                const float2 p = spectral(acc[r][q], a.scale, u, v, wx[r], wy[q]);
                 sm.b[2][u][v] = p.x;
                 sm.b[3][u][v] = p.y;
             }
@@ -649,7 +662,9 @@ __device__ __forceinline__ void dense_solve(const FieldRec &a, DenseSmem &sm, co
 }
 
 // ---- launches of one solve ----------------------------------------------------
-// P2 and P3 are programmatic dependents of the pass before.
+// The passes are programmatic dependents of the launch before (a solve in the
+// caller's buffers 12.3 -> 9.8 us at 96 bins, 6.2 -> 4.0 at 32 against an
+// ordinary first launch); a loop trial's first pass only at few bins.
 
 // run only if gate is null or (1 << *gate) & mask
 __device__ __forceinline__ bool gated_off(const int *gate, int mask) { return gate && !((1 << *gate) & mask); }
@@ -658,7 +673,7 @@ template <int M, int NT, int PASS>
 __global__ void __launch_bounds__(NT, odd_part(M) == 1 && M <= 2048 ? 1024 / NT : 1) fft_kernel(FieldRec a, const int *gate, int mask) {
     extern __shared__ __align__(16) float2 fft_sm[];
     if (PASS < 2) grid_release();
-    if (PASS > 0) grid_wait();
+    grid_wait();
     if (gated_off(gate, mask)) return;
     if (PASS == 0) fft_rows<M, NT>(a, blockIdx.x, fft_sm);
     if (PASS == 1) fft_columns<M, NT>(a, blockIdx.x, fft_sm);
@@ -670,16 +685,19 @@ template <int M, int NT>
 __global__ void __launch_bounds__(NT, (M <= 1024 ? 512 : 1024) / NT) fft_maps_kernel(FieldRec a, RhoArgs rho) {
     extern __shared__ __align__(16) float2 fft_sm[];
     grid_release();
+    grid_wait();
     fft_rows<M, NT, true>(a, blockIdx.x, fft_sm, &rho);
 }
 
 __global__ void __launch_bounds__(512) dense_maps_kernel(FieldRec a, RhoArgs rho) {
     __shared__ __align__(16) DenseSmem sm;
+    grid_wait();
     dense_solve<512, true>(a, sm, &rho);
 }
 
 __global__ void __launch_bounds__(512) dense_kernel(FieldRec a, const int *gate, int mask) {
     __shared__ __align__(16) DenseSmem sm;
+    grid_wait();
     if (gated_off(gate, mask)) return;
     dense_solve<512>(a, sm);
 }
@@ -710,10 +728,16 @@ int launch_fft(const FieldRec &a, cudaStream_t st, const int *gate, int mask, co
             maps = true;
             if constexpr (SM > 48 * 1024)
                 cudaFuncSetAttribute(fft_maps_kernel<M, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
-            fft_maps_kernel<M, NT><<<blocks, NT, SM, st>>>(a, *rho);
+            // beyond 128 bins its blocks would take SMs while the WA launch is
+            // still starting (an iteration without / with: 20k cells on 128
+            // bins 25.0 / 24.5 us, 100k on 256 33.7 / 34.4)
+            if constexpr (M <= 128)
+                launch_dependent(fft_maps_kernel<M, NT>, blocks, NT, SM, st, a, *rho);
+            else
+                fft_maps_kernel<M, NT><<<blocks, NT, SM, st>>>(a, *rho);
         }
     }
-    if (!maps) fft_kernel<M, NT, 0><<<blocks, NT, SM, st>>>(a, gate, mask);
+    if (!maps) launch_dependent(fft_kernel<M, NT, 0>, blocks, NT, SM, st, a, gate, mask);
     launch_dependent(fft_kernel<M, NT, 1>, fft_blocks(M, NT, 1, M), NT, SM, st, a, gate, mask);
     launch_dependent(fft_kernel<M, NT, 2>, fft_blocks(M, NT, 2, M), NT, SM, st, a, gate, mask);
     return blocks;
@@ -813,7 +837,7 @@ void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cuda
                       int gate_mask, float2 *exy) {
     const FieldRec a = solve_rec(f, d, ex, ey, exy);
     switch (f.m) {
-    case kDense: dense_kernel<<<1, 512, 0, st>>>(a, gate, gate_mask); break;
+    case kDense: launch_dependent(dense_kernel, 1, 512, 0, st, a, gate, gate_mask); break;
     case 64: launch_fft<64>(a, st, gate, gate_mask); break;
     case 96: launch_fft<96>(a, st, gate, gate_mask); break;
     case 128: launch_fft<128>(a, st, gate, gate_mask); break;
@@ -831,7 +855,7 @@ void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cuda
 int field_solve_maps(FieldSolver &f, const RhoArgs &rho, float2 *exy, cudaStream_t st) {
     const FieldRec a = solve_rec(f, nullptr, nullptr, nullptr, exy);
     switch (f.m) {
-    case kDense: dense_maps_kernel<<<1, 512, 0, st>>>(a, rho); return 1;
+    case kDense: launch_dependent(dense_maps_kernel, 1, 512, 0, st, a, rho); return 1;
     case 64: return launch_fft<64>(a, st, nullptr, 0, &rho);
     case 128: return launch_fft<128>(a, st, nullptr, 0, &rho);
     case 256: return launch_fft<256>(a, st, nullptr, 0, &rho);

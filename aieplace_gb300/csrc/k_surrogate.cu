@@ -738,6 +738,7 @@ __global__ void __launch_bounds__(256, 1) net_train_kernel(int B, int R, int mar
 // parameter, a warp each, added in their order; the last block: the loss
 __global__ void __launch_bounds__(256) train_reduce_kernel(int n_tiles, int n, const float *partial, float *grad,
                                                            const float *loss_partial, float inv_n, float *loss) {
+    grid_wait();
     __shared__ double red[32];
     __shared__ float part[8][32];
     if (blockIdx.x == gridDim.x - 1) {
@@ -1191,8 +1192,8 @@ void train_pass(ap_surrogate *s, int B, int R, int margin, bool relative, cudaSt
         else
             ap::sg::net_train_kernel<1><<<tiles, 256, smem, st>>>(B, R, margin, ap::fused_net(net), a[0], s->d_tb, map_w,
                                                                    net.d_params, n, s->d_wpart, s->d_lpart);
-        ap::sg::train_reduce_kernel<<<(n + 31) / 32 + 1, 256, 0, st>>>(
-            tiles, n, s->d_wpart, net.d_grad, s->d_lpart, 1.f / ((float)B * net.cout * inner * inner), s->d_loss);
+        ap::launch_dependent(ap::sg::train_reduce_kernel, (n + 31) / 32 + 1, 256, 0, st, tiles, n, s->d_wpart,
+                             net.d_grad, s->d_lpart, 1.f / ((float)B * net.cout * inner * inner), s->d_loss);
         return;
     }
     ap::net_forward(net, B, R, a, st);

@@ -1,10 +1,12 @@
-"""The bin adds as a dependent launch of the position update.
+"""The dependent launches of a loop trial.
 
-A loop trial's bin adds start while its update drains where they take at most
-a block an SM (152), and as an ordinary launch beyond.  The batched form's
-stages are ordinary launches of the same sums, so a batch of one gives the
-same bits: at the last size of the first rule, the first of the second, with
-filler cells (two launches of bin adds in a row) and at a single block.
+A trial's position update and gather start while the launch before them
+drains, its bin adds where they take at most a block an SM (152), the field's
+first pass up to 128 bins; all wait for that launch's results.  The batched
+form's stages are ordinary launches of the same sums, so a batch of one gives
+the same bits: at the last size of the bin adds' rule and the first beyond,
+on both sides of the field's, with filler cells (two launches of bin adds in a
+row), at a single block, in graphs and launched one by one.
 """
 import math
 
@@ -31,8 +33,10 @@ def ap():
     return aieplace_gb300
 
 
-@pytest.mark.parametrize("cells,bins,fillers", [(200, 32, 0), (LINE, 256, 0), (LINE + 1, 256, 0), (LINE - 1, 256, 1)])
-def test_dependent_bin_adds_match_ordinary_launches(ap, cells, bins, fillers):
+@pytest.mark.parametrize("graph", [1, 0])
+@pytest.mark.parametrize("cells,bins,fillers", [(200, 32, 0), (3000, 64, 1), (20_000, 128, 0), (LINE, 256, 0),
+                                                (LINE + 1, 256, 0), (LINE - 1, 256, 1)])
+def test_dependent_launches_match_ordinary_ones(ap, cells, bins, fillers, graph):
     nl = ap.synth.generate(dict(num_cells=cells, num_nets=cells, num_macros=0, num_pads=24, unit_cells=1, degree_mix=0,
                                 locality=0.0, window=64, target_density=0.9,
                                 die_side=float(math.ceil(math.sqrt(cells / 0.8))), bins=bins), seed=3)
@@ -41,7 +45,7 @@ def test_dependent_bin_adds_match_ordinary_launches(ap, cells, bins, fillers):
         b.step(16)
         bx, by = b.positions(0)
         bs = b.stats(0)
-    with ap.Placer(nl, block_nodes=BLOCK_NODES, filler_cells=fillers) as p:
+    with ap.Placer(nl, block_nodes=BLOCK_NODES, filler_cells=fillers, use_graph=graph) as p:
         p.initialize_placement(seed=7, sigma=1.0)
         p.step_async(16)
         x, y = p.positions()
