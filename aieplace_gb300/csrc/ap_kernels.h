@@ -279,6 +279,8 @@ int update_grid(const ScatterArgs &a);
 bool tile32_exact(const Grid &g, int n, int blocks);
 int rho_grid(int nbins);
 int gather_grid(int n_mov, int block_nodes);
+// whether the WA launches are the longer of a trial's two branches
+bool wa_longer(int n_nets);
 // fills bucket_blocks and small_blocks as launch_wirelength does; returns
 // the blocks of all four bucket launches
 int wa_plan(WaArgs &a);

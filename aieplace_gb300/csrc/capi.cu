@@ -1133,15 +1133,13 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(cudaMallocHost((void **)&h->h_out, sizeof(double) * 8));
     A(cudaMallocHost((void **)&h->h_status, 2 * sizeof(unsigned int)));
     // the WA launches run beside the density chain (scatter -> field), whose
-    // blocks they share the SMs with; they are the longer branch at 2M cells
-    // and go first there (an iteration with the WA stream at the chain's
-    // priority / above it: 200k cells 51.8 / 51.8 us, 2M 201.4 / 196.8; the chain's
-    // above the WA's: 1.5% longer than equal)
+    // blocks they share the SMs with: the chain goes first where it is the longer
+    // branch (wa_longer)
     int p_low = 0, p_high = 0;
     A(cudaDeviceGetStreamPriorityRange(&p_low, &p_high));
-    A(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+    A(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, wa_longer(h->n_nets) ? p_low : p_high));
     h->own_stream = true;
-    A(cudaStreamCreateWithPriority(&h->wa_stream, cudaStreamNonBlocking, p_high));
+    A(cudaStreamCreateWithPriority(&h->wa_stream, cudaStreamNonBlocking, p_low));
     A(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
     A(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     A(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));

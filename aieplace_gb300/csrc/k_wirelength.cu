@@ -311,8 +311,16 @@ __device__ __forceinline__ void wa_small_body(const WaArgs &a, VBlock vb) {
     }
 }
 
+// The launches of several do not read one another's results: each is a
+// programmatic dependent that starts in the slots that the last blocks of the
+// one before leave free, and waits for it only at its end, so that the
+// end of the last is the end of all (2M cells: the stage 100 -> 85 us).
 template <int D, int B>
-__global__ void __launch_bounds__(kThreads) wa_small_kernel(WaArgs a) { wa_small_body<D, B>(a, grid_block()); }
+__global__ void __launch_bounds__(kThreads) wa_small_kernel(WaArgs a) {
+    grid_release();
+    wa_small_body<D, B>(a, grid_block());
+    grid_wait();
+}
 
 // General path of one net of any degree by a warp: three passes over the pins
 // (extrema; sums; gradients), pins lane, lane + 32, ...
@@ -440,9 +448,10 @@ __device__ __forceinline__ void wa_fold(const WaArgs &a, int nb) {
 }
 
 // The last of the four launches: it folds the partials of all of them (the
-// three before it ran earlier on the same stream).
+// three before it have ended behind grid_wait).
 __global__ void __launch_bounds__(kThreads, 4) wa_large_kernel(WaArgs a) {
     wa_large_body(a, grid_block());
+    grid_wait();
     if (arrive_last(a.counter, gridDim.x)) wa_fold(a, a.small_blocks + (int)gridDim.x);
 }
 
@@ -498,6 +507,17 @@ void launch_interleave(int n, const float *px, const float *py, float2 *xy, cuda
     interleave_kernel<<<blocks, kThreads, 0, st>>>(n, px, py, xy);
 }
 
+// Up to here the density chain is the longer branch of a trial: its stream goes
+// first (ap_create) and the larger nets' launch, which would fill what the
+// chain needs, waits for the three before it.  Beyond, the branches have equal
+// priority and all four launches follow one another without a gap.  (A trial,
+// the first form / the second / four ordinary launches going first, started at
+// the centre and spread: 100k cells 31.8, 30.6 / 33.0, 32.3 / 33.5, 32.0 us;
+// 350k 86.6, 54.9 / 88.0, 60.1 / 92.4, 56.7; 500k 91.6, 64.9 / 89.6, 71.0 /
+// 94.4, 67.5; 700k 127.8, 118.9 / 119.8, 114.7 / 123.5, 119.4; 2M 245.7, 201.8 /
+// 191.5, 188.6 / 194.6, 192.4.)
+bool wa_longer(int n_nets) { return n_nets > 600000; }
+
 void launch_wirelength(const WaArgs &a0, cudaStream_t st) {
     WaArgs a = a0;
     if (a.mode != WA_LOOP) launch_interleave(a.n_nodes, a.px, a.py, a.xy, st);
@@ -509,9 +529,12 @@ void launch_wirelength(const WaArgs &a0, cudaStream_t st) {
         return;
     }
     wa_small_kernel<2, 0><<<a.bucket_blocks[0], kThreads, 0, st>>>(a);
-    wa_small_kernel<4, 1><<<a.bucket_blocks[1], kThreads, 0, st>>>(a);
-    wa_small_kernel<8, 2><<<a.bucket_blocks[2], kThreads, 0, st>>>(a);
-    wa_large_kernel<<<large, kThreads, 0, st>>>(a);
+    launch_dependent(wa_small_kernel<4, 1>, a.bucket_blocks[1], kThreads, 0, st, a);
+    launch_dependent(wa_small_kernel<8, 2>, a.bucket_blocks[2], kThreads, 0, st, a);
+    if (wa_longer(a.n_nets))
+        launch_dependent(wa_large_kernel, large, kThreads, 0, st, a);
+    else
+        wa_large_kernel<<<large, kThreads, 0, st>>>(a);
 }
 
 // The batched form: the four bucket launches of every instance as records of

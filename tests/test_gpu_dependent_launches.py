@@ -7,6 +7,10 @@ form's stages are ordinary launches of the same sums, so a batch of one gives
 the same bits: at the last size of the bin adds' rule and the first beyond,
 on both sides of the field's, with filler cells (two launches of bin adds in a
 row), at a single block, in graphs and launched one by one.
+
+The wirelength launches of one call wait for one another only at their ends (three of
+the four up to 600k nets, all four beyond); one launch of the same nets gives
+the same gradient bit for bit.
 """
 import math
 
@@ -53,3 +57,23 @@ def test_dependent_launches_match_ordinary_ones(ap, cells, bins, fillers, graph)
     np.testing.assert_array_equal(bx, x)
     np.testing.assert_array_equal(by, y)
     assert bs["hpwl"] == s["hpwl"] and bs["overflow"] == s["overflow"]
+
+
+@pytest.mark.parametrize("cells", [LINE, 2 * LINE])
+def test_overlapping_wirelength_launches_match_one(ap, cells):
+    nl = ap.synth.generate(dict(ap.synth.batch_specs(1, seed=1, lo=cells, hi=cells)[0], bins=512), seed=5)
+    rng = np.random.default_rng(2)
+    n = len(nl["node_w"])
+    die = nl["die"]
+    x = rng.uniform(0, die[2] * 0.99, n).astype(np.float32)
+    y = rng.uniform(0, die[3] * 0.99, n).astype(np.float32)
+    gamma = 2.0 * float(die[2]) / 512
+    with ap.Placer(nl, bins=512, block_nodes=8192) as one, ap.Placer(nl, bins=512) as four:
+        gx, gy, wa, hpwl = one.compute_all_partials(x, y, gamma)
+        for _ in range(4):
+            r = four.compute_all_partials(x, y, gamma)
+            np.testing.assert_array_equal(r[0], gx)
+            np.testing.assert_array_equal(r[1], gy)
+            # FP32 sums of positive terms: at most 32 a thread and 8 levels of
+            # a block's tree, each to 2^-24; compensated beyond
+            assert abs(r[2] / wa - 1) < 2 * 40 * 2.0 ** -24 and abs(r[3] / hpwl - 1) < 2 * 40 * 2.0 ** -24
