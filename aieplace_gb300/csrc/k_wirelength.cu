@@ -57,9 +57,9 @@ struct PairTerms {
         nwp = neg2(mul2(cp, ibp));
         nwm = neg2(mul2(cm, ibm));
     }
-    // a+/b+ (1 + (x - WA+)/g) - a-/b- (1 - (x - WA-)/g)
-    __device__ __forceinline__ float2 grad(float2 ep, float2 em, float2 dp, float2 dm, float2 ig, float2 nig) const {
-        const float2 tp = fma2(add2(dp, nwp), ig, both(1.f)), tm = fma2(add2(dm, nwm), nig, both(1.f));
+    // a+/b+ (1 + (x - WA+)/g) - a-/b- (1 - (x - WA-)/g) of sp = x - WA+, sm = x - WA-
+    __device__ __forceinline__ float2 grad(float2 ep, float2 em, float2 sp, float2 sm, float2 ig, float2 nig) const {
+        const float2 tp = fma2(sp, ig, both(1.f)), tm = fma2(sm, nig, both(1.f));
         return fma2(mul2(ep, ibp), tp, neg2(mul2(mul2(em, ibm), tm)));
     }
 };
@@ -168,10 +168,14 @@ __device__ __forceinline__ void net_group(const WaArgs &a, int s, int d, int l, 
     group_sum8<G>(s8, l, mask, base);
     const PairTerms t(make_float2(s8[0], s8[4]), make_float2(s8[1], s8[5]), make_float2(s8[2], s8[6]),
                       make_float2(s8[3], s8[7]));
+    const float2 ncp = make_float2(-s8[2], -s8[6]), ncm = make_float2(-s8[3], -s8[7]);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         if (!v[p] || (nd[p] & kPinNode) >= a.n_grad) continue;
-        const float2 g = t.grad(ep[p], em[p], add2(c[p], nmx), add2(c[p], nmn), ig, nig);
+        // x - WA+- fused with the quotient (by hand: left to the compiler it
+        // changed the last bit of some gradients with the code around it)
+        const float2 g = t.grad(ep[p], em[p], fma2(ncp, t.ibp, add2(c[p], nmx)), fma2(ncm, t.ibm, add2(c[p], nmn)), ig,
+                                nig);
         add_grad(a.gq, a.gqx, a.gqy, nd[p], g.x, g.y);
     }
     if (l == 0) {
@@ -239,7 +243,8 @@ __device__ __forceinline__ void net_thread(const int *__restrict__ pins, int d, 
 #pragma unroll
     for (int j = 0; j < D; ++j) {
         if (j < d && (node[j] & kPinNode) < n_grad) {
-            const float2 g = t.grad(ep[j], em[j], add2(c[j], nmx), add2(c[j], nmn), ig, nig);
+            const float2 g =
+                t.grad(ep[j], em[j], add2(add2(c[j], nmx), t.nwp), add2(add2(c[j], nmn), t.nwm), ig, nig);
             add_grad(gq, gqx, gqy, node[j], g.x, g.y);
         }
     }
