@@ -1,17 +1,22 @@
 // Density map, overflow, field gather and the Nesterov position update.
 //
+// update_kernel    the position update that produces the evaluation point
+//                  (Nesterov), and every node's bin record there.
 // scatter_kernel   Placer::computeOverlaps -> Grid::computeBinOverlaps
 //                  (vck5000/host/src/AIEplace.cpp:937-967, Grid.cpp:38-110,
-//                  Bin.h:78-121) as int64 fixed-point atomics, fused with the
-//                  position update that produces the evaluation point.
+//                  Bin.h:78-121) as int64 fixed-point adds of the records.
 // rho_kernel       Grid::getRho / computeTotalOverflow (Grid.cpp:112-151):
 //                  fixed-point map -> density per bin for the solver, overflow
 //                  in exact integer sums; clears the map for the next pass.
+//                  (A loop trial does this within the field solve's first
+//                  pass, k_field_fft.cu, unless a surrogate or the tensor-core
+//                  solve reads the density.)
 // gather_kernel    Placer::nudgeNode (AIEplace.cpp:1004-1046): overlap-weighted
 //                  field per node, combined with the wirelength gradient and
-//                  preconditioned; FP64 norms re-predict the Lipschitz step and
-//                  decide whether the trial is accepted (ePlace) -- the
-//                  reference moves by a fixed learning rate instead.
+//                  preconditioned; its last block folds the trial's sums,
+//                  re-predicts the Lipschitz step and decides whether the trial
+//                  is accepted (ePlace) -- the reference moves by a fixed
+//                  learning rate instead.
 #include <math.h>
 
 #include <algorithm>
@@ -61,7 +66,8 @@ __device__ __forceinline__ double block_max_f(float v, double *smem) {
 //   * else half or more in the window (ranges of kWinMinNodes or more): the window
 //     in shared memory, kWinC copies;
 //   * else no tile.
-// Nodes inside the tile add to it (red.shared.add.u64), the rest straight to
+// Nodes inside the tile add to it (two 32-bit red.shared adds where their sums
+// are exact, else red.shared.add.u64), the rest straight to
 // the map (red.global.add); at the end each tile bin's copies are summed and
 // the non-zero bins added to the map once.  Copy k of bin e sits at
 // [k t^2 + e].  All sums are integers, so the map is the same bit for bit

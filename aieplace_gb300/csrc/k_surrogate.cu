@@ -16,10 +16,13 @@
 // long-range part of the Poisson field (a few 3x3 convolutions cannot); the
 // network learns the fine-resolution residual.
 //
-// Tensors are [C][X][Y] with Y contiguous, like the bin maps (x-major).  Conv
-// kernels are FP32 SIMT: direct convolution with zero padding, one output
-// pixel per thread and all output channels in registers; the weight gradient
-// is reduced over pixel tiles in a fixed order (deterministic).
+// Tensors are [C][X][Y] with Y contiguous, like the bin maps (x-major).  The
+// convolutions are FP32 SIMT, direct, with zero padding.  Nets whose layers
+// after the first are 1 x 1 run by pixel tiles: inference in one launch, a
+// training pass in one and a reduction, 8 pixels x 4 channels a thread.  Other
+// nets run layer by layer, one output pixel per thread and all output channels
+// in registers.  Weight gradients are reduced over pixel tiles in a fixed order
+// (deterministic).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
