@@ -168,6 +168,13 @@ __device__ __forceinline__ void net_group(const WaArgs &a, int s, int d, int l, 
     group_sum8<G>(s8, l, mask, base);
     const PairTerms t(make_float2(s8[0], s8[4]), make_float2(s8[1], s8[5]), make_float2(s8[2], s8[6]),
                       make_float2(s8[3], s8[7]));
+    if (l == 0) {
+        hpf += (mx[0] - mn[0]) + (mx[1] - mn[1]);
+        float wa_net = 0.f;
+        wa_net += (mx[0] - mn[0]) - t.nwp.x + t.nwm.x;
+        wa_net += (mx[1] - mn[1]) - t.nwp.y + t.nwm.y;
+        waf += wa_net;
+    }
     const float2 ncp = make_float2(-s8[2], -s8[6]), ncm = make_float2(-s8[3], -s8[7]);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
@@ -177,13 +184,6 @@ __device__ __forceinline__ void net_group(const WaArgs &a, int s, int d, int l, 
         const float2 g = t.grad(ep[p], em[p], fma2(ncp, t.ibp, add2(c[p], nmx)), fma2(ncm, t.ibm, add2(c[p], nmn)), ig,
                                 nig);
         add_grad(a.gq, a.gqx, a.gqy, nd[p], g.x, g.y);
-    }
-    if (l == 0) {
-        hpf += (mx[0] - mn[0]) + (mx[1] - mn[1]);
-        float wa_net = 0.f;
-        wa_net += (mx[0] - mn[0]) - t.nwp.x + t.nwm.x;
-        wa_net += (mx[1] - mn[1]) - t.nwp.y + t.nwm.y;
-        waf += wa_net;
     }
 }
 
