@@ -130,8 +130,9 @@ struct ap_handle {
     cudaEvent_t ev_start = nullptr, ev_in[4] = {nullptr, nullptr, nullptr, nullptr};
     float *d_ix = nullptr, *d_iy = nullptr;
     // calls on host arrays in netlist order: internal node -> netlist node
-    // (null: the same), and kIo arrays of n_io floats that the copies go
-    // through (made on first use)
+    // (null: the same), and kIo arrays of n_io floats that the copies go through.
+    // Made by ap_create, so that these calls need no memory of their own and find
+    // the order complete
     int *d_int2ext = nullptr;
     float *d_io = nullptr;
     size_t n_io = 0;
@@ -511,17 +512,6 @@ int build_graphs(ap_handle *h) {
 // ms, 0.30 now; reading back 32 designs' positions 2.3 ms, 1.7 now.)
 constexpr int kIo = 6;  // 0-3: netlist order, in or out; 4, 5: internal order
 
-int ensure_io(ap_handle *h) {
-    if (h->d_io) return AP_OK;
-    h->n_io = (size_t)std::max(std::max(h->n_ext, h->n_mov), 1);
-    CK(dalloc(&h->d_io, kIo * h->n_io));
-    if (!h->identity && !h->d_int2ext) {
-        CK(dalloc(&h->d_int2ext, (size_t)h->n_nodes));
-        CK(cudaMemcpy(h->d_int2ext, h->int2ext.data(), sizeof(int) * h->n_nodes, cudaMemcpyHostToDevice));
-    }
-    return AP_OK;
-}
-
 int node_blocks(int n) { return std::max(1, std::min((n + kThreads - 1) / kThreads, 4096)); }
 
 // internal nodes [0, n): positions relative to the die's corner; filler cells
@@ -547,8 +537,6 @@ __global__ void import_kernel(int n, const int *__restrict__ int2ext, const floa
 // Host positions of internal nodes [0, n) -> dx, dy; AP_ERR_NONFINITE (with
 // only dx, dy written) if one is not finite.
 int import_positions(ap_handle *h, int n, const float *x, const float *y, float *dx, float *dy) {
-    int r = ensure_io(h);
-    if (r != AP_OK) return r;
     float *ex = h->d_io, *ey = h->d_io + h->n_io;
     unsigned int *bad = h->d_counters + 4;
     CK(cudaMemcpyAsync(ex, x, sizeof(float) * h->n_ext, cudaMemcpyHostToDevice, h->stream));
@@ -558,7 +546,7 @@ int import_positions(ap_handle *h, int n, const float *x, const float *y, float 
                                                               bad);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h->h_status + 1, bad, sizeof(*bad), cudaMemcpyDeviceToHost, h->stream));
-    r = sync(h);
+    const int r = sync(h);
     return r != AP_OK ? r : h->h_status[1] ? AP_ERR_NONFINITE : AP_OK;
 }
 
@@ -1150,6 +1138,9 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     for (cudaEvent_t &e : h->ev_in) A(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     A(dalloc(&h->d_ix, std::max(1, h->n_mov)));
     A(dalloc(&h->d_iy, std::max(1, h->n_mov)));
+    h->n_io = (size_t)std::max(h->n_ext, h->n_mov);
+    A(dalloc(&h->d_io, kIo * h->n_io));
+    if (!h->identity) A(dalloc(&h->d_int2ext, N));
     if (!ok) {
         ap_destroy(h);
         return AP_ERR_CUDA;
@@ -1172,6 +1163,7 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     A(cudaGetLastError());
     A(cudaMemcpy(h->d_pins, pins.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
     A(cudaMemcpy(h->d_charge, charge.data(), sizeof(float) * N, cudaMemcpyHostToDevice));
+    if (h->d_int2ext) A(cudaMemcpy(h->d_int2ext, h->int2ext.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
     A(cudaMemset(h->d_mov_q, 0, sizeof(ull) * nb));
     if (h->d_fill_q) A(cudaMemset(h->d_fill_q, 0, sizeof(ull) * nb));
     A(cudaMemset(h->d_counters, 0, sizeof(unsigned int) * 8));
@@ -1450,8 +1442,6 @@ int ap_run(ap_handle *h, int32_t *iterations_done) {
 int ap_get_positions(ap_handle *h, float *x, float *y) {
     if (!h || !x || !y) return AP_ERR_INVALID_ARG;
     int r = read_scalars(h);
-    if (r != AP_OK) return r;
-    r = ensure_io(h);
     if (r != AP_OK) return r;
     float *ox = h->d_io, *oy = h->d_io + h->n_io;
     export_positions_kernel<<<node_blocks(h->n_nodes), kThreads, 0, h->stream>>>(

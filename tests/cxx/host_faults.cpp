@@ -1,0 +1,157 @@
+// Failure paths of the library's host code, on the stand-in runtime of
+// fake_cudart.cpp: host_faults CASE exits 0 if the case holds.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "aieplace.h"
+#include "fake_cudart.h"
+
+#define REQUIRE(cond)                                                         \
+    do {                                                                      \
+        if (!(cond)) {                                                        \
+            fprintf(stderr, "%s:%d: %s\n", __FILE__, __LINE__, #cond);        \
+            exit(1);                                                          \
+        }                                                                     \
+    } while (0)
+
+namespace {
+
+// A netlist whose internal order (movable, fixed with area, fixed without) is not
+// its own: every third node is fixed, every fourth of those without area.
+struct Netlist {
+    std::vector<int32_t> ptr{0}, pin;
+    std::vector<float> w, h, x, y;
+    std::vector<uint8_t> fixed;
+    ap_netlist nl{};
+    explicit Netlist(int n = 60, float die = 64.f) {
+        for (int i = 0; i < n; ++i) {
+            const bool f = i % 3 == 0;
+            fixed.push_back(f);
+            w.push_back(f && i % 12 == 0 ? 0.f : 1.f);
+            h.push_back(1.f);
+            x.push_back((float)(i % 8));
+            y.push_back((float)(i / 8));
+        }
+        for (int i = 0; i + 1 < n; ++i) {
+            pin.push_back(i);
+            pin.push_back(i + 1);
+            ptr.push_back((int32_t)pin.size());
+        }
+        nl.num_nodes = n;
+        nl.num_nets = n - 1;
+        nl.num_pins = (int32_t)pin.size();
+        nl.net_ptr = ptr.data();
+        nl.pin_node = pin.data();
+        nl.node_w = w.data();
+        nl.node_h = h.data();
+        nl.node_x = x.data();
+        nl.node_y = y.data();
+        nl.node_fixed = fixed.data();
+        nl.die_xh = nl.die_yh = die;
+    }
+    std::vector<int> order(int fillers) const {
+        std::vector<int> o;
+        for (int cls = 0; cls < 3; ++cls) {
+            for (int i = 0; i < nl.num_nodes; ++i)
+                if ((!fixed[i] ? 0 : w[i] * h[i] > 0.f ? 1 : 2) == cls) o.push_back(i);
+            if (cls == 0) o.insert(o.end(), (size_t)fillers, -1);
+        }
+        return o;
+    }
+};
+
+ap_params params(int bins, int solver = AP_FIELD_FP32) {
+    ap_params p;
+    ap_params_default(&p);
+    p.bins_x = p.bins_y = bins;
+    p.field_solver = solver;
+    return p;
+}
+
+ap_handle *create(const Netlist &n, const ap_params &p) {
+    ap_handle *h = nullptr;
+    REQUIRE(ap_create(&n.nl, &p, &h) == AP_OK && h);
+    return h;
+}
+
+// Calls on host arrays need no memory that ap_create did not take, and what they
+// read on the device has arrived: whichever allocation fails, every call passes, and
+// its kernels get the netlist's order.
+void host_arrays() {
+    fake::watch("import_kernel", 1);
+    fake::watch("export_positions_kernel", 1);
+    fake::watch("export_gradient_kernel", 1);
+    fake::watch("export_force_kernel", 2);
+    for (int fillers = 0; fillers < 2; ++fillers)
+        for (int fail = 0; fail <= 3; ++fail) {
+            const Netlist n;
+            ap_params p = params(32);
+            p.filler_cells = fillers;
+            ap_handle *h = create(n, p);
+            int32_t n_fill = 0;
+            REQUIRE(ap_get_fillers(h, &n_fill, nullptr, nullptr) == AP_OK && (n_fill > 0) == (fillers > 0));
+            const std::vector<int> order = n.order(n_fill);
+            std::vector<float> x(n.x), y(n.y), gx(x.size()), gy(x.size()), field(32 * 32);
+            double hp, wa;
+            fake::fail_malloc(fail);
+            fake::take_launches();
+            for (int attempt = 0; attempt < 3; ++attempt) {
+                REQUIRE(ap_init_positions(h, n.x.data(), n.y.data()) == AP_OK);
+                REQUIRE(ap_get_positions(h, x.data(), y.data()) == AP_OK);
+                REQUIRE(ap_wirelength_grad(h, n.x.data(), n.y.data(), 4.f, gx.data(), gy.data(), &hp, &wa) == AP_OK);
+                REQUIRE(ap_node_force(h, n.x.data(), n.y.data(), field.data(), field.data(), 4.f, 1.f, gx.data(),
+                                      gy.data(), nullptr, nullptr) == AP_OK);
+            }
+            int seen = 0;
+            for (const fake::Launch &l : fake::take_launches())
+                for (const void *q : l.ptr) {
+                    REQUIRE(q && fake::is_device(q));
+                    REQUIRE(!memcmp(q, order.data(), sizeof(int) * order.size()));
+                    REQUIRE(!l.early);
+                    ++seen;
+                }
+            REQUIRE(seen == 3 * 6);  // an import each but for the read-back, an export each but for the first
+            fake::fail_malloc(0);
+            REQUIRE(ap_destroy(h) == AP_OK);
+        }
+}
+
+// ap_create takes everything or nothing.
+void create_fails() {
+    const Netlist n;
+    ap_params p = params(32);
+    p.filler_cells = 1;
+    ap_destroy(create(n, p));
+    const int before = fake::mallocs();
+    ap_destroy(create(n, p));
+    const int count = fake::mallocs() - before;
+    const size_t held = fake::live_bytes();
+    for (int k = 1; k <= count; ++k) {
+        ap_handle *h = nullptr;
+        fake::fail_malloc(k);
+        REQUIRE(ap_create(&n.nl, &p, &h) == AP_ERR_CUDA && !h);
+        REQUIRE(fake::live_bytes() == held);
+        fake::fail_malloc(0);
+        ap_create(&n.nl, &p, &h);  // may report what is left of the first error
+        if (h) ap_destroy(h);
+        ap_destroy(create(n, p));
+    }
+}
+
+const std::map<std::string, std::function<void()>> kCases = {
+    {"host_arrays", host_arrays},
+    {"create_fails", create_fails},
+};
+
+}  // namespace
+
+int main(int argc, char **argv) {
+    if (argc < 2 || !kCases.count(argv[1])) return 2;
+    kCases.at(argv[1])();
+    return 0;
+}
