@@ -243,6 +243,7 @@ struct FieldSolver {
 
 int field_solver_init(FieldSolver &f, int m, float bin_ratio);
 int field_solver_matrices(FieldSolver &f);  // the tensor-core path's constants and scratch
+void field_solver_free_bf16(FieldSolver &f);  // all of the tensor-core path's
 void field_solver_free(FieldSolver &f);
 // density d (x-major) -> ex, ey; FP32 fast transforms
 // gate: the launches run only if gate is null or (1 << *gate) & gate_mask

@@ -168,9 +168,19 @@ int ensure_tensor_cores(ap_handle *h) {
     if (h->fs.tc_ready) return AP_OK;
     if (h->fs.m % 128 != 0) return AP_ERR_UNSUPPORTED;  // the tcgen05 tiles need bins a multiple of 128
     const size_t nb = (size_t)h->fs.m * h->fs.m;
-    if (!h->d_dens_hi) CK(dalloc(&h->d_dens_hi, nb));
-    if (!h->d_dens_lo) CK(dalloc(&h->d_dens_lo, nb));
-    return field_solver_bind_bf16(h->fs, h->d_dens_hi, h->d_dens_lo);
+    __nv_bfloat16 *hi = nullptr, *lo = nullptr;
+    int r = dalloc(&hi, nb) == cudaSuccess && dalloc(&lo, nb) == cudaSuccess
+                ? field_solver_bind_bf16(h->fs, hi, lo)
+                : AP_ERR_CUDA;
+    if (r != AP_OK) {  // nothing is kept
+        if (hi) cudaFree(hi);
+        if (lo) cudaFree(lo);
+        cudaGetLastError();
+        return r;
+    }
+    h->d_dens_hi = hi;
+    h->d_dens_lo = lo;
+    return AP_OK;
 }
 
 // Whether a loop trial's field is written as (ex, ey) pairs, one load a bin for

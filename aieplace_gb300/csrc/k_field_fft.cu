@@ -791,9 +791,8 @@ void launch_split_bf16(int n, const float *src, __nv_bfloat16 *hi, __nv_bfloat16
 }
 
 // The tensor-core solve's constant transform matrices as BF16 hi/lo pairs,
-// and its scratch.
+// and its scratch (field_solver_free_bf16 gives back what a failure leaves).
 int field_solver_matrices(FieldSolver &f) {
-    if (f.C_hi) return AP_OK;
     const int m = f.m;
     const size_t nn = (size_t)m * m;
     std::vector<float> C(nn), Ct(nn), St(nn);
@@ -819,6 +818,7 @@ int field_solver_matrices(FieldSolver &f) {
     for (auto &q : s) {
         if (cudaMemcpy(f.t, q.src, nn * 4, cudaMemcpyHostToDevice) != cudaSuccess) return AP_ERR_CUDA;
         launch_split_bf16((int)nn, f.t, q.hi, q.lo, 0);
+        if (cudaGetLastError() != cudaSuccess) return AP_ERR_CUDA;
     }
     return AP_OK;
 }
@@ -906,13 +906,28 @@ int field_solver_init(FieldSolver &f, int m, float bin_ratio) {
     return r;
 }
 
-void field_solver_free(FieldSolver &f) {
-    void *ptrs[] = {f.tab,     f.wx,      f.wy,      f.t,       f.u,       f.C_hi,    f.C_lo,    f.Ct_hi,
-                    f.Ct_lo,   f.St_hi,   f.St_lo,   f.b_t_hi,  f.b_t_lo,  f.b_px_hi, f.b_px_lo, f.b_py_hi,
-                    f.b_py_lo, f.b_ux_hi, f.b_ux_lo, f.b_uy_hi, f.b_uy_lo, f.tc_status, f.tc_sync, f.tc_part};
+void field_solver_free_bf16(FieldSolver &f) {
+    __nv_bfloat16 **maps[] = {&f.C_hi,   &f.C_lo,   &f.Ct_hi,   &f.Ct_lo,   &f.St_hi,   &f.St_lo,   &f.b_t_hi,  &f.b_t_lo,
+                              &f.b_px_hi, &f.b_px_lo, &f.b_py_hi, &f.b_py_lo, &f.b_ux_hi, &f.b_ux_lo, &f.b_uy_hi, &f.b_uy_lo};
+    for (__nv_bfloat16 **p : maps) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
+    }
+    void *ptrs[] = {f.tc_status, f.tc_sync, f.tc_part};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    f.tc_status = f.tc_sync = nullptr;
+    f.tc_part = nullptr;
     free(f.tc_maps);  // host-side tensor-map table
+    f.tc_maps = nullptr;
+    f.tc_ready = f.tc_pinned = 0;
+}
+
+void field_solver_free(FieldSolver &f) {
+    field_solver_free_bf16(f);
+    void *ptrs[] = {f.tab, f.wx, f.wy, f.t, f.u};
+    for (void *p : ptrs)
+        if (p) cudaFree(p);
     f = FieldSolver();
 }
 

@@ -1304,27 +1304,26 @@ void run_variant(int v, FieldSolver &f, float *ex, float *ey, cudaStream_t st, c
 // 128 x 64 with 2 so that two CTAs share an SM; 3 warm, 5 timed, CUDA
 // events) and keeps the fastest: the tile autotuner of the tensor-core path.
 // The scratch outputs are overwritten.
-int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
+static int build_solver(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
     using namespace tc;
-    if (f.m < BM || (f.m % BM) != 0) return AP_ERR_UNSUPPORTED;
     const int mr = field_solver_matrices(f);
     if (mr != AP_OK) return mr;
     TcState s{};
     if (!build_stage_maps(s.maps[0], f, d_hi, d_lo, Tile64::BN) ||
         !build_stage_maps(s.maps[1], f, d_hi, d_lo, Tile128::BN))
         return AP_ERR_UNSUPPORTED;
-    if (!f.tc_maps && !(f.tc_maps = malloc(sizeof(TcState)))) return AP_ERR_CUDA;
+    if (!(f.tc_maps = malloc(sizeof(TcState)))) return AP_ERR_CUDA;
     *reinterpret_cast<TcState *>(f.tc_maps) = s;
-    if (!f.tc_status && cudaMalloc(&f.tc_status, sizeof(unsigned int)) != cudaSuccess) return AP_ERR_CUDA;
+    if (cudaMalloc(&f.tc_status, sizeof(unsigned int)) != cudaSuccess) return AP_ERR_CUDA;
     if (cudaMemset(f.tc_status, 0, sizeof(unsigned int)) != cudaSuccess) return AP_ERR_CUDA;
     // the persistent solve's counters (queue head, CTAs finished, 4 stages x 2
     // products x row blocks, 2 stages x tiles x 4 warps of halves) and its
     // split-K partials (2 stages x 2 halves x tiles of 128 x 128 FP32)
     const size_t nm = (size_t)(f.m / BM), tiles = nm * nm;
     const size_t sync_bytes = sizeof(unsigned int) * (2 + 8 * nm + 8 * tiles);
-    if (!f.tc_sync && cudaMalloc(&f.tc_sync, sync_bytes) != cudaSuccess) return AP_ERR_CUDA;
+    if (cudaMalloc(&f.tc_sync, sync_bytes) != cudaSuccess) return AP_ERR_CUDA;
     if (cudaMemset(f.tc_sync, 0, sync_bytes) != cudaSuccess) return AP_ERR_CUDA;
-    if (!f.tc_part && cudaMalloc(&f.tc_part, sizeof(float) * 4 * tiles * BM * BM) != cudaSuccess) return AP_ERR_CUDA;
+    if (cudaMalloc(&f.tc_part, sizeof(float) * 4 * tiles * BM * BM) != cudaSuccess) return AP_ERR_CUDA;
     if (cudaFuncSetAttribute(gemm_bf16x3_kernel<Tile64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Tile64::SMEM_BYTES) != cudaSuccess ||
         cudaFuncSetAttribute(gemm_bf16x3_kernel<Tile128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1337,7 +1336,11 @@ int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv
         cudaMemset((void *)d_lo, 0, sizeof(__nv_bfloat16) * (size_t)f.m * f.m) != cudaSuccess)
         return AP_ERR_CUDA;
     cudaEvent_t e0, e1;
-    if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return AP_ERR_CUDA;
+    if (cudaEventCreate(&e0) != cudaSuccess) return AP_ERR_CUDA;
+    if (cudaEventCreate(&e1) != cudaSuccess) {
+        cudaEventDestroy(e0);
+        return AP_ERR_CUDA;
+    }
     // two passes over the candidates, each keeping its faster pass: the
     // first candidate timed on a cold GPU (clocks, caches) would otherwise
     // look slower than it is
@@ -1378,6 +1381,19 @@ int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv
     if (st) return AP_ERR_TIMEOUT;
     f.tc_ready = 1;
     return AP_OK;
+}
+
+// Whole or nothing: after a failure at any step nothing is kept, so that a later
+// call starts anew, and the runtime's last error is not left for another call.
+int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
+    if (f.m < tc::BM || (f.m % tc::BM) != 0) return AP_ERR_UNSUPPORTED;
+    field_solver_free_bf16(f);
+    const int r = build_solver(f, d_hi, d_lo);
+    if (r != AP_OK) {
+        field_solver_free_bf16(f);
+        cudaGetLastError();
+    }
+    return r;
 }
 
 int field_solve_bf16x3(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo, float *ex,

@@ -143,9 +143,55 @@ void create_fails() {
     }
 }
 
+// The tensor-core solve is made whole or not at all: whichever allocation or copy
+// fails, the call says so and keeps nothing, and the next one makes all of it.
+void tensor_cores_retry() {
+    const Netlist n;
+    fake::watch("split_kernel", 1);
+    fake::watch("split_kernel", 2);
+    fake::watch("split_kernel", 3);
+    const auto splits = [](int count) {
+        int seen = 0;
+        for (const fake::Launch &l : fake::take_launches())
+            if (!l.ptr.empty()) {
+                for (const void *q : l.ptr) REQUIRE(q && fake::is_device(q));
+                ++seen;
+            }
+        REQUIRE(seen == count);
+    };
+    int allocations = 0;
+    for (int what = 0; what < 2; ++what)
+        for (int k = 1;; ++k) {
+            ap_handle *h = create(n, params(128, AP_FIELD_BF16X3));
+            const size_t held = fake::live_bytes();
+            fake::take_launches();
+            (what ? fake::fail_upload : [](int f) { fake::fail_malloc(f); })(k);
+            const int before = fake::mallocs();
+            const int r = ap_debug_inject(h, AP_FAULT_TC_STALL, 1000000);
+            const bool failed = r != AP_OK;
+            if (failed) {
+                REQUIRE(r == AP_ERR_CUDA);
+                REQUIRE(fake::live_bytes() == held);
+                fake::take_launches();
+                REQUIRE(ap_debug_inject(h, AP_FAULT_TC_STALL, 1000000) == AP_OK);
+            } else if (what == 0) {
+                allocations = fake::mallocs() - before;
+            }
+            splits(3);  // C, C^T and S^T
+            std::vector<float> d(128 * 128, 1.f), ex(d), ey(d);
+            fake::fail_malloc(0);
+            fake::fail_upload(0);
+            REQUIRE(ap_field_solve(h, d.data(), ex.data(), ey.data(), AP_FIELD_BF16X3) == AP_OK);
+            REQUIRE(ap_destroy(h) == AP_OK);
+            if (!failed) break;
+        }
+    REQUIRE(allocations >= 21);  // two input maps, 16 maps, three of the persistent solve
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
+    {"tensor_cores_retry", tensor_cores_retry},
 };
 
 }  // namespace

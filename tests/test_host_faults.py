@@ -6,6 +6,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
   host_arrays   calls on host arrays allocate nothing after ap_create, and read no
                 array whose copy may still be on its way
   create_fails  ap_create gives back what it took, whichever allocation fails
+  tensor_cores_retry  so does the tensor-core solve made on first use, and the next call
+                makes all of it
 """
 import os
 import subprocess
@@ -37,7 +39,7 @@ def host_faults(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["host_arrays", "create_fails"])
+@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
