@@ -257,7 +257,8 @@ void field_solve_fp32(FieldSolver &f, const float *d, float *ex, float *ey, cuda
 int field_solve_maps(FieldSolver &f, const RhoArgs &rho, float2 *exy, cudaStream_t st);
 // Builds the TMA tensor maps of the tcgen05 path with (d_hi, d_lo) as the
 // density input; needs m a multiple of 128.
-int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo);
+// pin: the candidate to take ("0".."4"), or null for the fastest.
+int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo, const char *pin);
 // density as bf16 hi/lo split (the bound buffers) -> ex, ey; tcgen05 BF16x3 contraction
 int field_solve_bf16x3(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo,
                        float *ex, float *ey, cudaStream_t st, const int *gate = nullptr, int gate_mask = 0);

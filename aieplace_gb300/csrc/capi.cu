@@ -163,14 +163,15 @@ bool on_tensor_cores(const ap_handle *h, int solver) {
 
 // The tensor-core solve's matrices, buffers and candidates' times, made on
 // first use; nothing of the handle may be in flight (the tuning runs on the
-// solver's scratch).
-int ensure_tensor_cores(ap_handle *h) {
+// solver's scratch).  pin: AP_TC_VARIANT at ap_create, which alone may choose the
+// candidate and with it the solver of the handle's loop, or null.
+int ensure_tensor_cores(ap_handle *h, const char *pin = nullptr) {
     if (h->fs.tc_ready) return AP_OK;
     if (h->fs.m % 128 != 0) return AP_ERR_UNSUPPORTED;  // the tcgen05 tiles need bins a multiple of 128
     const size_t nb = (size_t)h->fs.m * h->fs.m;
     __nv_bfloat16 *hi = nullptr, *lo = nullptr;
     int r = dalloc(&hi, nb) == cudaSuccess && dalloc(&lo, nb) == cudaSuccess
-                ? field_solver_bind_bf16(h->fs, hi, lo)
+                ? field_solver_bind_bf16(h->fs, hi, lo, pin)
                 : AP_ERR_CUDA;
     if (r != AP_OK) {  // nothing is kept
         if (hi) cudaFree(hi);
@@ -1209,8 +1210,8 @@ int ap_create(const ap_netlist *nl, const ap_params *params, ap_handle **out) {
     }
     int r = ok ? field_solver_init(h->fs, p.bins_x, g.bh / g.bw) : AP_ERR_CUDA;
     if (r == AP_OK && p.bins_x % 128 == 0) {
-        if (getenv("AP_TC_VARIANT")) {
-            r = ensure_tensor_cores(h);
+        if (const char *pin = getenv("AP_TC_VARIANT")) {
+            r = ensure_tensor_cores(h, pin);
             if (r != AP_OK && p.field_solver != AP_FIELD_BF16X3) r = AP_OK;  // tensor path optional here
         }
     } else if (r == AP_OK && p.field_solver == AP_FIELD_BF16X3) {
@@ -1368,19 +1369,18 @@ int ap_set_log(ap_handle *h, const char *path, int32_t capacity) {
 
 int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *simt_tile, float *simt_ms) {
     if (!h) return AP_ERR_INVALID_ARG;
-    if (h->fs.m % 128 == 0 && !h->fs.tc_ready) {
-        CK(cudaStreamSynchronize(h->stream));
-        const int r = ensure_tensor_cores(h);
-        if (r != AP_OK) return r;
-    }
-    if (tc_variant) *tc_variant = h->fs.tc_ready ? h->fs.tc_variant : -1;
-    if (tc_ms)
-        for (int v = 0; v < kTcCandidates; ++v) tc_ms[v] = h->fs.tc_tune_ms[v];
     if (simt_tile) *simt_tile = h->fs.simt_tile;
     if (simt_ms) {
         simt_ms[0] = h->fs.simt_ms[0];
         simt_ms[1] = h->fs.simt_ms[1];
     }
+    if ((tc_variant || tc_ms) && h->fs.m % 128 == 0 && !h->fs.tc_ready) {
+        CK(cudaStreamSynchronize(h->stream));
+        (void)ensure_tensor_cores(h);  // where it cannot be made: reported as unavailable
+    }
+    if (tc_variant) *tc_variant = h->fs.tc_ready ? h->fs.tc_variant : -1;
+    if (tc_ms)
+        for (int v = 0; v < kTcCandidates; ++v) tc_ms[v] = h->fs.tc_tune_ms[v];
     return AP_OK;
 }
 

@@ -921,6 +921,7 @@ void field_solver_free_bf16(FieldSolver &f) {
     free(f.tc_maps);  // host-side tensor-map table
     f.tc_maps = nullptr;
     f.tc_ready = f.tc_pinned = 0;
+    for (float &ms : f.tc_tune_ms) ms = 0.f;
 }
 
 void field_solver_free(FieldSolver &f) {

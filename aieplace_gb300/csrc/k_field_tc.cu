@@ -1304,7 +1304,7 @@ void run_variant(int v, FieldSolver &f, float *ex, float *ey, cudaStream_t st, c
 // 128 x 64 with 2 so that two CTAs share an SM; 3 warm, 5 timed, CUDA
 // events) and keeps the fastest: the tile autotuner of the tensor-core path.
 // The scratch outputs are overwritten.
-static int build_solver(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
+static int build_solver(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo, const char *pin) {
     using namespace tc;
     const int mr = field_solver_matrices(f);
     if (mr != AP_OK) return mr;
@@ -1368,8 +1368,8 @@ static int build_solver(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bf
         if (f.tc_tune_ms[v] >= 0.f && f.tc_tune_ms[v] < f.tc_tune_ms[f.tc_variant]) f.tc_variant = v;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    // AP_TC_VARIANT=0..4 pins a candidate that ran (tests of each variant)
-    if (const char *pin = getenv("AP_TC_VARIANT")) {
+    // "0".."4" pins a candidate that ran (tests of each variant)
+    if (pin) {
         const int v = atoi(pin);
         if (v >= 0 && v < kTcVariants && f.tc_tune_ms[v] >= 0.f) {
             f.tc_variant = v;
@@ -1385,10 +1385,10 @@ static int build_solver(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bf
 
 // Whole or nothing: after a failure at any step nothing is kept, so that a later
 // call starts anew, and the runtime's last error is not left for another call.
-int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo) {
+int field_solver_bind_bf16(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfloat16 *d_lo, const char *pin) {
     if (f.m < tc::BM || (f.m % tc::BM) != 0) return AP_ERR_UNSUPPORTED;
     field_solver_free_bf16(f);
-    const int r = build_solver(f, d_hi, d_lo);
+    const int r = build_solver(f, d_hi, d_lo, pin);
     if (r != AP_OK) {
         field_solver_free_bf16(f);
         cudaGetLastError();

@@ -180,16 +180,18 @@ int ap_profile_stages(ap_handle *h, int32_t n_trials, float *stage_ms, int32_t *
 int ap_set_log(ap_handle *h, const char *path, int32_t capacity);
 
 /* Tile shapes the autotuner picked for this bin count, and the solve times it
- * measured (the tensor-core solve's on the first call that needs them): tc_variant is the tensor-core candidate (0: four
- * launches of 128 x 64 tiles, 4 pipeline stages; 1: 128 x 128, 3 stages; 2:
- * 128 x 64, 2 stages, two CTAs per SM; 3: one persistent launch over the four
- * stages' 128 x 128 tiles, K of the first two stages split in two; 4: the
- * same without the split; -1 if the
- * tensor-core path is unavailable), simt_tile the FP32 solve's block (32: up to
- * 256 threads, 64: 512 threads); tc_ms[5] the candidates' times, simt_ms[0]
- * or [1] the FP32 solve's by its block (-1: not run).  The
- * environment variable AP_TC_VARIANT=0..4, read at ap_create, pins a
- * candidate: the mixed-precision solver then runs it (for testing each one). */
+ * measured.  tc_variant is the tensor-core candidate (0: four launches of 128 x
+ * 64 tiles, 4 pipeline stages; 1: 128 x 128, 3 stages; 2: 128 x 64, 2 stages, two
+ * CTAs per SM; 3: one persistent launch over the four stages' 128 x 128 tiles, K
+ * of the first two stages split in two; 4: the same without the split; -1 if the
+ * tensor-core path is unavailable), tc_ms[5] the candidates' times (-1: not run).
+ * The first call that asks for either on a handle with bins a multiple of 128
+ * makes that solve and times it (some 60 MB at 1024 bins); where that fails the
+ * path is unavailable.  simt_tile is the FP32 solve's block (32: up to 256
+ * threads, 64: 512 threads), simt_ms[0] or [1] its time by its block (the other
+ * -1).  Any output may be NULL.  The environment variable AP_TC_VARIANT=0..4,
+ * read at ap_create only, pins a candidate: the mixed-precision solver then runs
+ * it (for testing each one). */
 int ap_solver_info(ap_handle *h, int32_t *tc_variant, float *tc_ms, int32_t *simt_tile, float *simt_ms);
 
 /* Iterates until overflow < params.target_overflow or max_iterations;

@@ -188,10 +188,50 @@ void tensor_cores_retry() {
     REQUIRE(allocations >= 21);  // two input maps, 16 maps, three of the persistent solve
 }
 
+int launches_of(const char *kernel) {
+    int seen = 0;
+    for (const fake::Launch &l : fake::take_launches()) seen += l.name.find(kernel) != std::string::npos;
+    return seen;
+}
+
+// ap_solver_info reports on an optional path: where that cannot be made it says so
+// and the handle works on, and it never changes which solver the handle runs.
+void solver_info() {
+    const Netlist n;
+    std::vector<float> d(128 * 128, 1.f), ex(d), ey(d);
+    for (int solver : {AP_FIELD_FP32, AP_FIELD_BF16X3}) {
+        ap_handle *h = create(n, params(128, solver));
+        int32_t variant = 7, tile = 0;
+        float tc_ms[5], simt_ms[2] = {0.f, 0.f};
+        fake::fail_malloc(3, true);
+        REQUIRE(ap_solver_info(h, &variant, tc_ms, &tile, simt_ms) == AP_OK);
+        REQUIRE(variant == -1 && tile == 32 && simt_ms[0] > 0.f && simt_ms[1] == -1.f);
+        fake::fail_malloc(0);
+        REQUIRE(ap_field_solve(h, d.data(), ex.data(), ey.data(), solver) == AP_OK);
+        setenv("AP_TC_VARIANT", "1", 1);  // too late for this handle
+        REQUIRE(ap_solver_info(h, &variant, tc_ms, nullptr, nullptr) == AP_OK && variant >= 0 && tc_ms[1] > 0.f);
+        unsetenv("AP_TC_VARIANT");
+        fake::take_launches();
+        REQUIRE(ap_field_solve(h, d.data(), ex.data(), ey.data(), solver) == AP_OK);
+        REQUIRE(launches_of("split_kernel") == 0);
+        REQUIRE(ap_destroy(h) == AP_OK);
+    }
+    setenv("AP_TC_VARIANT", "1", 1);
+    ap_handle *h = create(n, params(128, AP_FIELD_BF16X3));
+    unsetenv("AP_TC_VARIANT");
+    int32_t variant = 7;
+    REQUIRE(ap_solver_info(h, &variant, nullptr, nullptr, nullptr) == AP_OK && variant == 1);
+    fake::take_launches();
+    REQUIRE(ap_field_solve(h, d.data(), ex.data(), ey.data(), -1) == AP_OK);
+    REQUIRE(launches_of("split_kernel") == 1);
+    REQUIRE(ap_destroy(h) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
     {"tensor_cores_retry", tensor_cores_retry},
+    {"solver_info", solver_info},
 };
 
 }  // namespace

@@ -8,6 +8,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
   create_fails  ap_create gives back what it took, whichever allocation fails
   tensor_cores_retry  so does the tensor-core solve made on first use, and the next call
                 makes all of it
+  solver_info   ap_solver_info reports a tensor-core path that cannot be made as
+                unavailable, and does not change the handle's solver
 """
 import os
 import subprocess
@@ -39,7 +41,7 @@ def host_faults(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry"])
+@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
