@@ -24,11 +24,15 @@ namespace ap {
 // fresh array) cost the copy engine's first write to each far more than the
 // host's: they are touched here first (their contents stay).  Into fresh
 // memory, alone: 180 KB 112 -> 26 us, 1 MB 183 -> 62, 4 MB 264 -> 178, 8 MB 365 ->
-// 334; 16 MB 591 -> 647, so larger arrays are left to the copy.
+// 334; 16 MB 591 -> 647, so larger arrays are left to the copy.  Only memory that
+// the runtime knows nothing of is touched: pinned pages are there already, and a
+// device pointer is the copy's to refuse.
 cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t st) {
     constexpr size_t kTouchMost = 8u << 20;
     static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
-    if (bytes <= kTouchMost && bytes > 0) {
+    cudaPointerAttributes at;
+    if (bytes <= kTouchMost && bytes > 0 && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+        at.type == cudaMemoryTypeUnregistered) {
         char *p = static_cast<char *>(dst), *end = p + bytes;
         for (; p < end; p = reinterpret_cast<char *>(((uintptr_t)p / page + 1) * page))
             __atomic_fetch_or(p, 0, __ATOMIC_RELAXED);

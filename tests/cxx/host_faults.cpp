@@ -227,11 +227,32 @@ void solver_info() {
     REQUIRE(ap_destroy(h) == AP_OK);
 }
 
+// An output that is no host memory is the runtime's to refuse: the host does not
+// write to it.
+void device_output() {
+    const Netlist n;
+    ap_handle *h = create(n, params(64));
+    std::vector<float> d(64 * 64, 1.f), e(d);
+    void *dev = fake::device_only(64 * 64 * 8);
+    REQUIRE(ap_density_map(h, n.x.data(), n.y.data(), (int64_t *)dev) == AP_ERR_CUDA);
+    REQUIRE(ap_field_solve(h, d.data(), (float *)dev, e.data(), -1) != AP_OK);
+    ap_field_solve(h, d.data(), e.data(), e.data(), -1);  // may report what is left of the error
+    REQUIRE(ap_field_solve(h, d.data(), e.data(), e.data(), -1) == AP_OK);
+    REQUIRE(ap_destroy(h) == AP_OK);
+    ap_surrogate_config c;
+    ap_surrogate *s = nullptr;
+    REQUIRE(ap_surrogate_config_default(&c) == AP_OK && ap_surrogate_create(&c, &s) == AP_OK);
+    std::vector<float> x((c.factor * c.factor + 2) * 16 * 16);
+    REQUIRE(ap_surrogate_forward(s, x.data(), 1, 16, (float *)dev) == AP_ERR_CUDA);
+    REQUIRE(ap_surrogate_destroy(s) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
     {"tensor_cores_retry", tensor_cores_retry},
     {"solver_info", solver_info},
+    {"device_output", device_output},
 };
 
 }  // namespace

@@ -10,6 +10,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
                 makes all of it
   solver_info   ap_solver_info reports a tensor-core path that cannot be made as
                 unavailable, and does not change the handle's solver
+  device_output  a device pointer given for a host output is refused by the copy, not
+                written by the host
 """
 import os
 import subprocess
@@ -41,7 +43,7 @@ def host_faults(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info"])
+@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
