@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) persist_field_kernel(PersistQue
 
 // dynamic shared memory of a persistent launch whose largest grid has m bins
 // a side: every grid up to 2048 needs the same
-int persist_field_smem(int tile, int m) {
+constexpr int persist_field_smem(int tile, int m) {
     return std::max(fft_smem(m > 2048 ? 4096 : 512, 8 * tile), (int)sizeof(DenseSmem));
 }
 
@@ -993,7 +993,9 @@ int persist_field_smem(int tile, int m) {
 int persist_field_wave(int tile, int m) {
     const int smem = persist_field_smem(tile, m);
     const void *k = tile == 64 ? (const void *)persist_field_kernel<512> : (const void *)persist_field_kernel<256>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // what the largest grid needs, whatever this launch's: the attribute is the
+    // process's, and another thread's batch may be about to launch
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, persist_field_smem(tile, 4096));
     return wave_of(k, 8 * tile, 304, smem);
 }
 

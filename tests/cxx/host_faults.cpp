@@ -247,12 +247,27 @@ void device_output() {
     REQUIRE(ap_surrogate_destroy(s) == AP_OK);
 }
 
+// What a kernel's shared memory is allowed holds for the whole process: a batch of
+// small grids must not take back what a batch of large ones, in another thread, is
+// about to launch with.
+void shared_memory_limits() {
+    const Netlist n;
+    ap_batch *large = nullptr, *small = nullptr;
+    const ap_params pl = params(4096), ps = params(64);
+    REQUIRE(ap_create_batch(1, &n.nl, &pl, &large) == AP_OK);
+    REQUIRE(ap_create_batch(1, &n.nl, &ps, &small) == AP_OK);
+    const fake::SmemLimit s = fake::smem_limit("persist_field_kernelILi512E");
+    REQUIRE(s.most > 0 && s.last == s.most);
+    REQUIRE(ap_batch_destroy(small) == AP_OK && ap_batch_destroy(large) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
     {"tensor_cores_retry", tensor_cores_retry},
     {"solver_info", solver_info},
     {"device_output", device_output},
+    {"shared_memory_limits", shared_memory_limits},
 };
 
 }  // namespace

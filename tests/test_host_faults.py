@@ -12,6 +12,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
                 unavailable, and does not change the handle's solver
   device_output  a device pointer given for a host output is refused by the copy, not
                 written by the host
+  shared_memory_limits  a batch of small grids leaves a batch of large ones its
+                kernel's shared memory
 """
 import os
 import subprocess
@@ -43,7 +45,8 @@ def host_faults(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output"])
+@pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
+                                  "shared_memory_limits"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
