@@ -814,11 +814,12 @@ constexpr int kTrialsPerGraph = 4;
 int launch_trials(ap_handle *h, int n) {
     int i = 0;
     if (h->graph_ok && !h->surr && n >= kTrialsPerGraph) {
-        if (!h->graph_n) {
-            const int r = build_graph(h, kTrialsPerGraph, &h->graph_n);
-            if (r != AP_OK) return r;
+        if (!h->graph_n && build_graph(h, kTrialsPerGraph, &h->graph_n) != AP_OK) {
+            h->graph_n = nullptr;  // no memory for it: one trial a graph launch
+            cudaGetLastError();
         }
-        for (; n - i >= kTrialsPerGraph; i += kTrialsPerGraph) CK(cudaGraphLaunch(h->graph_n, h->stream));
+        for (; h->graph_n && n - i >= kTrialsPerGraph; i += kTrialsPerGraph)
+            CK(cudaGraphLaunch(h->graph_n, h->stream));
     }
     for (; i < n; ++i) {
         if (h->graph_ok) {

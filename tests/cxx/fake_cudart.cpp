@@ -23,7 +23,7 @@ struct State {
     std::vector<fake::Launch> launches;
     std::map<const char *, size_t> flying;  // null-stream transfers not yet waited for
     std::map<std::string, fake::SmemLimit> smem;
-    int n_malloc = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
+    int n_malloc = 0, n_graph = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
     bool malloc_after = false, inst_after = false;
     cudaError_t last = cudaSuccess;
     size_t handle = 0x1000;
@@ -114,6 +114,7 @@ namespace fake {
 void fail_malloc(int n, bool after) { S().fail_malloc = n, S().malloc_after = after; }
 void fail_upload(int n) { S().fail_upload = n; }
 void fail_instantiate(int n, bool after) { S().fail_inst = n, S().inst_after = after; }
+int graph_launches() { return S().n_graph; }
 int mallocs() { return S().n_malloc; }
 size_t live_bytes() {
     size_t t = 0;
@@ -345,6 +346,9 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long 
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
+    ++S().n_graph;
+    return e ? cudaSuccess : err(cudaErrorInvalidValue);
+}
 
 }  // extern "C"

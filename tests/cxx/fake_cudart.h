@@ -13,6 +13,7 @@ namespace fake {
 void fail_malloc(int n, bool and_after = false);
 void fail_upload(int n);
 void fail_instantiate(int n, bool and_after = false);
+int graph_launches();    // graph launches so far
 int mallocs();           // device allocations asked for so far
 size_t live_bytes();     // device memory held
 bool is_device(const void *p);

@@ -261,6 +261,28 @@ void shared_memory_limits() {
     REQUIRE(ap_batch_destroy(small) == AP_OK && ap_batch_destroy(large) == AP_OK);
 }
 
+// The graph of four trials is made by the first call that can use it: where that
+// fails the loop runs on the graph of one, which the initial placement made.
+void trial_graphs() {
+    const Netlist n;
+    ap_handle *h = create(n, params(32));
+    REQUIRE(ap_init_positions(h, n.x.data(), n.y.data()) == AP_OK);
+    const auto launches = [&](int trials) {
+        const int before = fake::graph_launches();
+        REQUIRE(ap_step_async(h, trials) == AP_OK);
+        return fake::graph_launches() - before;
+    };
+    fake::fail_instantiate(1, true);
+    REQUIRE(launches(10) == 10);
+    REQUIRE(launches(3) == 3);
+    fake::fail_instantiate(0);
+    REQUIRE(launches(10) == 2 + 2);
+    REQUIRE(launches(3) == 3);
+    REQUIRE(ap_init_positions(h, n.x.data(), n.y.data()) == AP_OK);
+    REQUIRE(launches(8) == 2);
+    REQUIRE(ap_destroy(h) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -268,6 +290,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"solver_info", solver_info},
     {"device_output", device_output},
     {"shared_memory_limits", shared_memory_limits},
+    {"trial_graphs", trial_graphs},
 };
 
 }  // namespace

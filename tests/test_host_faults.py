@@ -14,6 +14,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
                 written by the host
   shared_memory_limits  a batch of small grids leaves a batch of large ones its
                 kernel's shared memory
+  trial_graphs  the loop runs on one trial a graph launch where the graph of four
+                cannot be made
 """
 import os
 import subprocess
@@ -46,7 +48,7 @@ def host_faults(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
-                                  "shared_memory_limits"])
+                                  "shared_memory_limits", "trial_graphs"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
