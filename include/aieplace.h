@@ -162,8 +162,10 @@ int ap_step_async(ap_handle *h, int32_t n_trials);
 
 /* Runs n_trials trial steps with one CUDA event between stages and returns
  * the mean milliseconds per stage: [0] density scatter + position update,
- * [1] density -> solver input + overflow, [2] wirelength gradient,
- * [3] field solve, [4] field gather + step control.  *n_stages = 5. */
+ * [1] density -> solver input + overflow (0 where the field solve's first pass
+ * does it: without a surrogate or a pinned tensor-core solve), [2] wirelength
+ * gradient, [3] field solve, [4] field gather + step control.  The kernels are
+ * those of the loop's trials.  *n_stages = 5. */
 int ap_profile_stages(ap_handle *h, int32_t n_trials, float *stage_ms, int32_t *n_stages);
 
 /* Per-trial trajectory log, one JSON object a line: eval, iteration,

@@ -5,6 +5,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -283,6 +284,34 @@ void trial_graphs() {
     REQUIRE(ap_destroy(h) == AP_OK);
 }
 
+// ap_profile_stages times the loop's own kernels.
+void profile_launches() {
+    const Netlist n;
+    const auto names = [] {
+        std::multiset<std::string> s;
+        for (const fake::Launch &l : fake::take_launches()) s.insert(l.name);
+        return s;
+    };
+    for (int c = 0; c < 5; ++c) {
+        ap_params p = params(c == 0 ? 32 : c < 3 ? 64 : 128, c < 3 ? AP_FIELD_FP32 : AP_FIELD_BF16X3);
+        p.filler_cells = c == 2;
+        p.use_graph = 0;
+        if (c == 4) setenv("AP_TC_VARIANT", "1", 1);
+        ap_handle *h = create(n, p);
+        unsetenv("AP_TC_VARIANT");
+        REQUIRE(ap_init_positions(h, n.x.data(), n.y.data()) == AP_OK);
+        names();
+        REQUIRE(ap_step_async(h, 1) == AP_OK);
+        const auto loop = names();
+        float ms[8];
+        int32_t stages = 0;
+        REQUIRE(ap_profile_stages(h, 1, ms, &stages) == AP_OK && stages == 5);
+        REQUIRE(!loop.empty() && names() == loop);
+        REQUIRE((ms[1] > 0.f) == (c == 4) && ms[0] > 0.f && ms[2] > 0.f && ms[3] > 0.f && ms[4] > 0.f);
+        REQUIRE(ap_destroy(h) == AP_OK);
+    }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -291,6 +320,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"device_output", device_output},
     {"shared_memory_limits", shared_memory_limits},
     {"trial_graphs", trial_graphs},
+    {"profile_launches", profile_launches},
 };
 
 }  // namespace

@@ -16,6 +16,7 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
                 kernel's shared memory
   trial_graphs  the loop runs on one trial a graph launch where the graph of four
                 cannot be made
+  profile_launches  ap_profile_stages launches the kernels that a trial does
 """
 import os
 import subprocess
@@ -48,7 +49,7 @@ def host_faults(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
-                                  "shared_memory_limits", "trial_graphs"])
+                                  "shared_memory_limits", "trial_graphs", "profile_launches"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
