@@ -35,14 +35,17 @@ import subprocess
 import sys
 import time
 
+import numpy as np
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
 sys.path.insert(0, os.path.join(HERE, "oracle"))
 
 METRIC = "Nesterov iters/s & time-to-10% overflow, 2M cells: mixed+surrogate vs plain"
 UNIT = "iters/s"
-# per trial: update, scatter, rho, 4x WA (degree buckets), the field solve, gather
-KERNELS_BESIDE_FIELD = 8
+# resident blocks of one launch over all nets (k_wirelength.cu): up to so many, the
+# wirelength gradient is one launch, beyond four
+WA_ONE_LAUNCH_BLOCKS = 456
 
 
 def tensor_cores(solver: str) -> bool:
@@ -51,13 +54,27 @@ def tensor_cores(solver: str) -> bool:
     return solver == "bf16x3" and bool(os.environ.get("AP_TC_VARIANT"))
 
 
-def field_launches(info: dict, solver: str) -> int:
-    """Launches of one field solve: three FP32 passes; of a tensor-core solve
-    that AP_TC_VARIANT pins four stage launches, or one for its persistent
-    candidates (3, 4)."""
-    if not tensor_cores(solver):
-        return 3
-    return 1 if info.get("tc_variant", -1) in (3, 4) else 4
+def wa_launches(nl) -> int:
+    d = np.diff(nl["net_ptr"])
+    d = d[d >= 2]
+    blocks = 0
+    for lo, hi, lanes, most in ((2, 2, 1, 2432), (3, 4, 1, 2432), (5, 8, 1, 2432), (9, 16, 8, 608), (17, 32, 16, 608),
+                                (33, 64, 16, 608), (65, 1 << 30, 32, 608)):
+        items = int(((d >= lo) & (d <= hi)).sum()) * lanes
+        blocks += min(max(1, (items + 255) // 256), most)
+    return 1 if blocks <= WA_ONE_LAUNCH_BLOCKS else 4
+
+
+def trial_launches(nl, info: dict, solver: str) -> int:
+    """Kernels of one loop trial: position update, bin adds, wirelength gradient,
+    field solve, gather.  The solve is three FP32 passes, the first with the density
+    (32 bins: one launch); where AP_TC_VARIANT pins a tensor-core candidate it is
+    the density and four stage launches, or one of the persistent candidates (3, 4)."""
+    if tensor_cores(solver):
+        field = 1 + (1 if info.get("tc_variant", -1) in (3, 4) else 4)
+    else:
+        field = 1 if int(nl["bins"]) == 32 else 3
+    return 1 + 1 + wa_launches(nl) + field + 1
 
 
 STAGES = ["scatter+update", "density+overflow", "wirelength", "field", "gather+control"]
@@ -80,14 +97,14 @@ def workload_desc(nl, preset):
 
 
 def stage_model(nl, solver):
-    """Algorithmic bytes (HBM) or FLOPs per launch of each stage."""
+    """Algorithmic bytes (HBM) or FLOPs per launch of each stage that the loop has."""
     n_nodes = len(nl["node_w"])
     n_mov = int((nl["node_fixed"] == 0).sum())
     e = len(nl["net_ptr"]) - 1
     p = len(nl["pin_node"])
     m2 = int(nl["bins"]) ** 2
     m3 = int(nl["bins"]) ** 3
-    return {
+    model = {
         # update: read v, g, u, w, h, write u', v' and the 20-byte bin record;
         # bin adds: read the record; int64 map written once
         "scatter+update": ("hbm", 88 * n_mov + 8 * m2),
@@ -95,12 +112,15 @@ def stage_model(nl, solver):
         "density+overflow": ("hbm", 36 * m2),
         # net_ptr, pin_node, node positions, int64 gradient per movable node
         "wirelength": ("hbm", 4 * (e + 1) + 4 * p + 8 * n_nodes + 16 * n_mov),
-        # density in, both fields out; pinned to the tensor cores: 6 dense
-        # m x m x m contractions (useful FLOPs)
-        "field": ("tensor", 12 * m3) if tensor_cores(solver) else ("hbm", 12 * m2),
+        # mov, fixed, fixed-scaled maps in, mov cleared, both fields out; pinned to the
+        # tensor cores: 6 dense m x m x m contractions (useful FLOPs)
+        "field": ("tensor", 12 * m3) if tensor_cores(solver) else ("hbm", 40 * m2),
         # bin record, int64 WA gradient read+clear, pins, charge, g_prev, g out; field maps
         "gather+control": ("hbm", 60 * n_mov + 8 * m2),
     }
+    if not tensor_cores(solver):  # the density is part of the field solve's first pass
+        del model["density+overflow"]
+    return model
 
 
 class ClockSampler:
@@ -278,8 +298,8 @@ def batch_mode(args):
     stepped together.  Reports instance-iterations per second over K graph
     launches for the persistent form (six persistent launches per trial step
     over all instances, FP32 field, the default), for the graph of
-    per-instance branches with the FP32 field and with the BF16x3 tensor-core
-    field, the wall time until every instance is below 10% overflow, and the
+    per-instance branches with the FP32 field and, where AP_TC_VARIANT pins a
+    candidate, with the BF16x3 tensor-core field, the wall time until every instance is below 10% overflow, and the
     instances stepped one after another on their own graphs."""
     import torch
 
@@ -291,7 +311,7 @@ def batch_mode(args):
     nls = [ap.synth.generate(s, seed=100 + i) for i, s in enumerate(specs)]
     cells = sum(int((nl["node_fixed"] == 0).sum()) for nl in nls)
     forms = {}
-    for form in ("persistent", "graph", "graph_bf16x3"):
+    for form in ("persistent", "graph") + (("graph_bf16x3",) if tensor_cores("bf16x3") else ()):
         solver = "bf16x3" if form == "graph_bf16x3" else "fp32"
         with ap.BatchPlacer(nls, field_solver=solver, max_iterations=4000, check_interval=32) as bp:
             bp.set_form("graph" if form == "graph_bf16x3" else form)
@@ -600,7 +620,7 @@ def main():
     se1 = pl.stats()
     e2e_iters = se1["iteration"] - se0["iteration"]
     n_mov = int((nl["node_fixed"] == 0).sum())
-    launches_per_trial = KERNELS_BESIDE_FIELD + field_launches(pl.solver_info(), solver)
+    launches_per_trial = trial_launches(nl, pl.solver_info() if tensor_cores(solver) else {}, solver)
     pl.close()
 
     t_max = ms / 1000.0
@@ -634,6 +654,8 @@ def main():
         # every stage against its own roof (HBM copy or dense BF16 burst)
         per_stage = []
         for i, name in enumerate(STAGES):
+            if name not in model:
+                continue
             b_i, amt_i = model[name]
             sec = stage_ms[i] / 1000.0
             if b_i == "hbm":
