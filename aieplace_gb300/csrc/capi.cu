@@ -1856,6 +1856,7 @@ int ap_restore(ap_handle *h, const void *buf, size_t bytes) {
     CK(cudaMemset(h->d_mov_q, 0, sizeof(ull) * (size_t)h->p.bins_x * h->p.bins_y));
     if (h->d_fill_q) CK(cudaMemset(h->d_fill_q, 0, sizeof(ull) * (size_t)h->p.bins_x * h->p.bins_y));
     CK(cudaMemset(h->d_counters, 0, sizeof(unsigned int) * 8));
+    CK(cudaStreamSynchronize(0));  // the handle's streams do not wait for the null stream
     h->initialized = true;
     if (h->p.use_graph && !h->graph_ok) return build_graphs(h);
     return AP_OK;
@@ -2182,6 +2183,7 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
     CK(cudaMemcpy(pp.d_dep, dep.data(), sizeof(int) * dep.size(), cudaMemcpyHostToDevice));
     CK(dalloc(&pp.d_cnt, kFieldDone + dep.size()));
     CK(cudaMemset(pp.d_cnt, 0, sizeof(unsigned int) * (kFieldDone + dep.size())));
+    CK(cudaStreamSynchronize(0));  // the batch's streams do not wait for the null stream
     return AP_OK;
 }
 
@@ -2385,7 +2387,8 @@ int ap_create_batch(int32_t n, const ap_netlist *netlists, const ap_params *para
                        cudaEventCreateWithFlags(&b->wa_fork, cudaEventDisableTiming) != cudaSuccess ||
                        cudaEventCreateWithFlags(&b->wa_join, cudaEventDisableTiming) != cudaSuccess ||
                        dalloc(&b->d_status, 1) != cudaSuccess ||
-                       cudaMemset(b->d_status, 0, sizeof(unsigned int)) != cudaSuccess))
+                       cudaMemset(b->d_status, 0, sizeof(unsigned int)) != cudaSuccess ||
+                       cudaStreamSynchronize(0) != cudaSuccess))
         r = AP_ERR_CUDA;
     for (int i = 0; i < n && r == AP_OK; ++i) {
         cudaEvent_t ev;
@@ -2481,7 +2484,10 @@ int ap_batch_debug_inject(ap_batch *b, int32_t kind, int64_t wait_ns) {
     CK(cudaStreamSynchronize(b->main));
     b->never_arrive = kind == AP_FAULT_NEVER_ARRIVE;
     b->wait_ns = kind == AP_FAULT_NEVER_ARRIVE ? (unsigned long long)wait_ns : 1000000000ull;
-    if (kind == AP_FAULT_NONE) CK(cudaMemset(b->d_status, 0, sizeof(unsigned int)));
+    if (kind == AP_FAULT_NONE) {
+        CK(cudaMemset(b->d_status, 0, sizeof(unsigned int)));
+        CK(cudaStreamSynchronize(0));
+    }
     return b->graph ? batch_build_graph(b) : AP_OK;
 }
 
@@ -2492,8 +2498,8 @@ int ap_batch_init_seeded(ap_batch *b, uint64_t seed, float sigma) {
         int r = ap_init_seeded(b->inst[i], seed + i, sigma);
         if (r != AP_OK) return r;
     }
-    CK(cudaDeviceSynchronize());  // the instances' streams before the batch stream's first launch
     CK(cudaMemset(b->d_status, 0, sizeof(unsigned int)));
+    CK(cudaDeviceSynchronize());  // the instances' streams before the batch stream's first launch
     b->active.assign(b->inst.size(), 1);
     return batch_build_graph(b);
 }

@@ -1407,7 +1407,10 @@ int field_solve_bf16x3(FieldSolver &f, const __nv_bfloat16 *d_hi, const __nv_bfl
 
 int field_solver_clear_status(FieldSolver &f) {
     if (!f.tc_status) return AP_OK;
-    return cudaMemset(f.tc_status, 0, sizeof(unsigned int)) == cudaSuccess ? AP_OK : AP_ERR_CUDA;
+    // (the solve's streams do not wait for the null stream)
+    return cudaMemset(f.tc_status, 0, sizeof(unsigned int)) == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess
+               ? AP_OK
+               : AP_ERR_CUDA;
 }
 
 }  // namespace ap

@@ -1272,7 +1272,7 @@ int ap_surrogate_create(const ap_surrogate_config *cfg, ap_surrogate **out) {
               ap::dmalloc(&n.d_v, off);
     ok = ok && cudaMemcpy(n.d_params, p.data(), sizeof(float) * off, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemset(n.d_m, 0, sizeof(float) * off) == cudaSuccess &&
-         cudaMemset(n.d_v, 0, sizeof(float) * off) == cudaSuccess;
+         cudaMemset(n.d_v, 0, sizeof(float) * off) == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     if (!ok) {
         ap_surrogate_destroy(s);
         return AP_ERR_CUDA;
@@ -1309,6 +1309,7 @@ int ap_surrogate_set_params(ap_surrogate *s, const float *params, int32_t n) {
     CKS(cudaMemcpy(s->net.d_params, params, sizeof(float) * n, cudaMemcpyHostToDevice));
     CKS(cudaMemset(s->net.d_m, 0, sizeof(float) * n));
     CKS(cudaMemset(s->net.d_v, 0, sizeof(float) * n));
+    CKS(cudaStreamSynchronize(0));  // a loop's streams do not wait for the null stream
     s->net.adam_t = 0;
     return AP_OK;
 }

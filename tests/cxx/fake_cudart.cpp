@@ -23,7 +23,7 @@ struct State {
     std::vector<fake::Launch> launches;
     std::map<const char *, size_t> flying;  // null-stream transfers not yet waited for
     std::map<std::string, fake::SmemLimit> smem;
-    int n_malloc = 0, n_graph = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
+    int n_malloc = 0, n_graph = 0, n_early = 0, capturing = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
     bool malloc_after = false, inst_after = false;
     cudaError_t last = cudaSuccess;
     size_t handle = 0x1000;
@@ -90,6 +90,7 @@ void record(const void *fn, void **args, cudaStream_t st) {
             l.ptr.push_back(*(const void **)args[w.second]);
             l.early = l.early || (st && find(S().flying, l.ptr.back()));
         }
+    if (st && !S().capturing && !S().flying.empty()) ++S().n_early;
     S().launches.push_back(l);
 }
 struct Config {
@@ -115,6 +116,7 @@ void fail_malloc(int n, bool after) { S().fail_malloc = n, S().malloc_after = af
 void fail_upload(int n) { S().fail_upload = n; }
 void fail_instantiate(int n, bool after) { S().fail_inst = n, S().inst_after = after; }
 int graph_launches() { return S().n_graph; }
+int early_launches() { return S().n_early; }
 int mallocs() { return S().n_malloc; }
 size_t live_bytes() {
     size_t t = 0;
@@ -313,12 +315,19 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
     *ms = 1.f;
     return cudaSuccess;
 }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
-cudaError_t cudaStreamBeginCaptureToGraph(cudaStream_t, cudaGraph_t, const cudaGraphNode_t *, const cudaGraphEdgeData *,
-                                          size_t, cudaStreamCaptureMode) {
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    ++S().capturing;
     return cudaSuccess;
 }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return make(g); }
+cudaError_t cudaStreamBeginCaptureToGraph(cudaStream_t, cudaGraph_t, const cudaGraphNode_t *, const cudaGraphEdgeData *,
+                                          size_t, cudaStreamCaptureMode) {
+    ++S().capturing;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) {
+    --S().capturing;
+    return make(g);
+}
 cudaError_t cudaStreamGetCaptureInfo(cudaStream_t, cudaStreamCaptureStatus *s, unsigned long long *, cudaGraph_t *g,
                                      const cudaGraphNode_t **d, const cudaGraphEdgeData **e, size_t *n) {
     *s = cudaStreamCaptureStatusActive;
@@ -333,7 +342,9 @@ cudaError_t cudaStreamUpdateCaptureDependencies(cudaStream_t, cudaGraphNode_t *,
     return cudaSuccess;
 }
 cudaError_t cudaGraphAddNode(cudaGraphNode_t *n, cudaGraph_t, const cudaGraphNode_t *, const cudaGraphEdgeData *, size_t,
-                             cudaGraphNodeParams *) {
+                             cudaGraphNodeParams *p) {
+    static cudaGraph_t bodies[8];
+    if (p->type == cudaGraphNodeTypeConditional) p->conditional.phGraph_out = bodies;
     return make(n);
 }
 cudaError_t cudaGraphConditionalHandleCreate(cudaGraphConditionalHandle *h, cudaGraph_t, unsigned, unsigned) {
@@ -346,8 +357,9 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long 
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t st) {
     ++S().n_graph;
+    if (st && !S().flying.empty()) ++S().n_early;
     return e ? cudaSuccess : err(cudaErrorInvalidValue);
 }
 

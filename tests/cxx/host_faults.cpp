@@ -312,6 +312,62 @@ void profile_launches() {
     }
 }
 
+// What a call puts on the null stream has arrived before anything of the library's
+// non-blocking streams is launched.
+void null_stream_waits() {
+    const Netlist n;
+    const auto waited = [](const char *what) {
+        if (fake::early_launches()) {
+            fprintf(stderr, "%s: %d launches too early\n", what, fake::early_launches());
+            exit(1);
+        }
+    };
+    std::vector<float> d(128 * 128, 1.f), ex(d), ey(d);
+    for (int pinned = 0; pinned < 2; ++pinned) {
+        if (pinned) setenv("AP_TC_VARIANT", "1", 1);
+        ap_handle *h = create(n, params(128, AP_FIELD_BF16X3));
+        unsetenv("AP_TC_VARIANT");
+        REQUIRE(ap_init_positions(h, n.x.data(), n.y.data()) == AP_OK && ap_step_async(h, 5) == AP_OK);
+        waited("ap_create, ap_init_positions");
+        size_t bytes = 0;
+        REQUIRE(ap_snapshot_size(h, &bytes) == AP_OK);
+        std::vector<char> blob(bytes);
+        REQUIRE(ap_snapshot(h, blob.data(), bytes) == AP_OK && ap_restore(h, blob.data(), bytes) == AP_OK);
+        REQUIRE(ap_step_async(h, 1) == AP_OK);
+        waited("ap_restore");
+        REQUIRE(ap_debug_inject(h, AP_FAULT_TC_STALL, 1000000) == AP_OK && ap_debug_inject(h, AP_FAULT_NONE, 0) == AP_OK);
+        REQUIRE(ap_field_solve(h, d.data(), ex.data(), ey.data(), -1) == AP_OK);
+        waited("ap_debug_inject");
+        ap_surrogate_config c;
+        ap_surrogate *s = nullptr;
+        REQUIRE(ap_surrogate_config_default(&c) == AP_OK && ap_surrogate_create(&c, &s) == AP_OK);
+        REQUIRE(ap_attach_surrogate(h, s, nullptr) == AP_OK && ap_step_async(h, 1) == AP_OK);
+        waited("ap_surrogate_create, ap_attach_surrogate");
+        int32_t np = 0;
+        REQUIRE(ap_surrogate_num_params(s, &np) == AP_OK);
+        std::vector<float> w((size_t)np);
+        REQUIRE(ap_surrogate_set_params(s, w.data(), np) == AP_OK && ap_step_async(h, 1) == AP_OK);
+        waited("ap_surrogate_set_params");
+        REQUIRE(ap_destroy(h) == AP_OK && ap_surrogate_destroy(s) == AP_OK);
+    }
+    for (int solver : {AP_FIELD_FP32, AP_FIELD_BF16X3}) {
+        const ap_params p[2] = {params(128, solver), params(128, solver)};
+        const ap_netlist nl[2] = {n.nl, n.nl};
+        ap_batch *b = nullptr;
+        REQUIRE(ap_create_batch(2, nl, p, &b) == AP_OK);
+        waited("ap_create_batch");
+        REQUIRE(ap_batch_init_seeded(b, 1, 1.f) == AP_OK && ap_batch_step(b, 2) == AP_OK);
+        waited("ap_batch_init_seeded");
+        if (solver == AP_FIELD_FP32) {
+            REQUIRE(ap_batch_set_item_blocks(b, 1) == AP_OK && ap_batch_step(b, 1) == AP_OK);
+            waited("ap_batch_set_item_blocks");
+            REQUIRE(ap_batch_debug_inject(b, AP_FAULT_NONE, 0) == AP_OK && ap_batch_step(b, 1) == AP_OK);
+            waited("ap_batch_debug_inject");
+        }
+        REQUIRE(ap_batch_destroy(b) == AP_OK);
+    }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -321,6 +377,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"shared_memory_limits", shared_memory_limits},
     {"trial_graphs", trial_graphs},
     {"profile_launches", profile_launches},
+    {"null_stream_waits", null_stream_waits},
 };
 
 }  // namespace

@@ -17,6 +17,8 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
   trial_graphs  the loop runs on one trial a graph launch where the graph of four
                 cannot be made
   profile_launches  ap_profile_stages launches the kernels that a trial does
+  null_stream_waits  what a call copies or clears on the null stream has arrived before
+                a launch on a stream of the library's own
 """
 import os
 import subprocess
@@ -49,7 +51,7 @@ def host_faults(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
-                                  "shared_memory_limits", "trial_graphs", "profile_launches"])
+                                  "shared_memory_limits", "trial_graphs", "profile_launches", "null_stream_waits"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
