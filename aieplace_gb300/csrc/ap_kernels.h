@@ -307,13 +307,18 @@ struct FieldRec {
 bool field_records(const FieldSolver &f, const float *d, float2 *exy, int tile, FieldRec rec[4]);
 int field_rec_blocks(const FieldRec &r, int tile);
 
-// one persistent launch of a stage over the records `recs` (device memory)
-// with the grid persist_*_wave() (one wave of resident blocks)
+// one persistent launch of a stage over the records `recs` (device memory) of
+// `items` work items, with one wave of resident blocks (persist_*_wave(): the most
+// that a stage's launch takes)
+// Blocks of a persistent launch: no more than it has items.  (The blocks of an SM come
+// for their first items together: 128 items on a full wave of three an SM ran on a
+// third of the SMs, the bin adds of 128 designs of 1000 cells in 50 us, 27 as here.)
+inline int persist_blocks(int wave, int items) { return items < 1 ? 1 : items < wave ? items : wave; }
 int persist_density_wave(int stage);
 int persist_wa_wave();
 int persist_field_wave(int tile, int m);  // m: the largest grid of the launch
-void launch_persist_density(int stage, const PersistQueue &q, const void *recs, cudaStream_t st);
-void launch_persist_wa(const PersistQueue &q, const WaArgs *recs, cudaStream_t st);
-void launch_persist_field(const PersistQueue &q, const FieldRec *recs, int tile, int m, cudaStream_t st);
+void launch_persist_density(int stage, const PersistQueue &q, int items, const void *recs, cudaStream_t st);
+void launch_persist_wa(const PersistQueue &q, int items, const WaArgs *recs, cudaStream_t st);
+void launch_persist_field(const PersistQueue &q, int items, const FieldRec *recs, int tile, int m, cudaStream_t st);
 
 }  // namespace ap

@@ -2228,17 +2228,19 @@ int gather_reset_n(const PersistPlan &pp) { return kFieldDone - 4 + pp.n_rec[PS_
 // density/overflow -> field; the gather with each instance's accept / retry.
 int enqueue_persist(ap_batch *b, cudaStream_t st) {
     const PersistPlan &pp = b->plan;
-    launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.d_recs[PS_UPDATE], st);
+    launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.items[PS_UPDATE], pp.d_recs[PS_UPDATE], st);
     CK(cudaEventRecord(b->wa_fork, st));
     CK(cudaStreamWaitEvent(b->wa_stream, b->wa_fork, 0));
-    launch_persist_wa(plan_queue(b, PS_WA, 0, 0), static_cast<const WaArgs *>(pp.d_recs[PS_WA]), b->wa_stream);
+    launch_persist_wa(plan_queue(b, PS_WA, 0, 0), pp.items[PS_WA], static_cast<const WaArgs *>(pp.d_recs[PS_WA]),
+                      b->wa_stream);
     CK(cudaEventRecord(b->wa_join, b->wa_stream));
-    launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.d_recs[PS_SCATTER], st);
-    launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.d_recs[PS_RHO], st);
-    launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]),
-                         pp.field_tile, pp.field_m, st);
+    launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.items[PS_SCATTER], pp.d_recs[PS_SCATTER], st);
+    launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.items[PS_RHO], pp.d_recs[PS_RHO], st);
+    launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), pp.items[PS_FIELD],
+                         static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]), pp.field_tile, pp.field_m, st);
     CK(cudaStreamWaitEvent(st, b->wa_join, 0));
-    launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.d_recs[PS_GATHER], st);
+    launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.items[PS_GATHER],
+                           pp.d_recs[PS_GATHER], st);
     return cudaGetLastError() == cudaSuccess ? AP_OK : AP_ERR_CUDA;
 }
 
@@ -2255,19 +2257,19 @@ int persist_profile(ap_batch *b, int n_trials, float *ms) {
     cudaStream_t st = b->main;
     for (int t = 0; t < n_trials && r == AP_OK; ++t) {
         CK(cudaEventRecord(ev[0], st));
-        launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.d_recs[PS_UPDATE], st);
+        launch_persist_density(PS_UPDATE, plan_queue(b, PS_UPDATE, 0, 1), pp.items[PS_UPDATE], pp.d_recs[PS_UPDATE], st);
         CK(cudaEventRecord(ev[1], st));
-        launch_persist_wa(plan_queue(b, PS_WA, 0, 0), static_cast<const WaArgs *>(pp.d_recs[PS_WA]), st);
+        launch_persist_wa(plan_queue(b, PS_WA, 0, 0), pp.items[PS_WA], static_cast<const WaArgs *>(pp.d_recs[PS_WA]), st);
         CK(cudaEventRecord(ev[2], st));
-        launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.d_recs[PS_SCATTER], st);
+        launch_persist_density(PS_SCATTER, plan_queue(b, PS_SCATTER, 1, 1), pp.items[PS_SCATTER], pp.d_recs[PS_SCATTER], st);
         CK(cudaEventRecord(ev[3], st));
-        launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.d_recs[PS_RHO], st);
+        launch_persist_density(PS_RHO, plan_queue(b, PS_RHO, 2, 1), pp.items[PS_RHO], pp.d_recs[PS_RHO], st);
         CK(cudaEventRecord(ev[4], st));
-        launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]),
-                         pp.field_tile, pp.field_m, st);
+        launch_persist_field(plan_queue(b, PS_FIELD, 3, 1), pp.items[PS_FIELD],
+                             static_cast<const FieldRec *>(pp.d_recs[PS_FIELD]), pp.field_tile, pp.field_m, st);
         CK(cudaEventRecord(ev[5], st));
-        launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.d_recs[PS_GATHER],
-                               st);
+        launch_persist_density(PS_GATHER, plan_queue(b, PS_GATHER, 4, gather_reset_n(pp)), pp.items[PS_GATHER],
+                               pp.d_recs[PS_GATHER], st);
         CK(cudaEventRecord(ev[6], st));
         r = batch_sync(b);
         // the events around each stage, in the order update, scatter, rho, WA, field, gather
@@ -2346,7 +2348,7 @@ int batch_tune_field(ap_batch *b) {
             if (cudaMemsetAsync(b->plan.d_cnt + kFieldDone - 1, 0, sizeof(unsigned int) * (1 + nf), b->main) !=
                 cudaSuccess)
                 r = AP_ERR_CUDA;
-            launch_persist_field(plan_queue(b, PS_FIELD, 3, 0),
+            launch_persist_field(plan_queue(b, PS_FIELD, 3, 0), b->plan.items[PS_FIELD],
                                  static_cast<const FieldRec *>(b->plan.d_recs[PS_FIELD]),
                                  b->plan.field_tile, b->plan.field_m, b->main);
         }

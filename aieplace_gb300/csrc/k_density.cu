@@ -1304,7 +1304,15 @@ __global__ void numerics_selftest_kernel(long long n, ull seed, int *mism) {
 // sums depend on it the grid that the launchers above give it (plan_build); an
 // instance's sums fold in its last block, as in its own launch.
 
-__global__ void __launch_bounds__(kThreads, 5) persist_update_kernel(PersistQueue q, const ScatterArgs *recs) {
+// The position update and the gather come with fewer and with more blocks an SM, the
+// more at the cost of spilled registers: more only where that saves a round of
+// resident blocks (persist_pick).  A step with five an SM always / with this rule and
+// no idle blocks (persist_blocks), at overflow 0.05: 128 designs of 2000 cells on 32 bins
+// (128 items) 132 / 103 us, 128 of 1000 on 64 bins 183 / 161, 8 of 200k 415 / 395, 2 of 1M
+// 473 / 442; where five save a round, 128 of 10k (640 items; 456, 608 and 760 blocks are
+// resident) 350 / 349 and 32 of 5k-150k 281 / 280, with four always 367 and 293.
+template <int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) persist_update_kernel(PersistQueue q, const ScatterArgs *recs) {
     persist_loop(q, recs, [](const ScatterArgs &a, VBlock vb, int) {
         update_body<false>(a, vb);
         if (arrive_last(a.counter, vb.n)) update_fold(a, vb.n);
@@ -1322,53 +1330,80 @@ __global__ void __launch_bounds__(kThreads) persist_rho_kernel(PersistQueue q, c
     });
 }
 
-__global__ void __launch_bounds__(kThreads, 5) persist_gather_kernel(PersistQueue q, const GatherArgs *recs) {
+template <int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) persist_gather_kernel(PersistQueue q, const GatherArgs *recs) {
     persist_loop(q, recs, [](const GatherArgs &a, VBlock vb, int) {
         gather_body<GATHER_STEP, true>(a, vb);
         if (arrive_last(a.counter, vb.n)) gather_fold(a, vb.n);
     });
 }
 
+// A kernel and the most blocks of it that are resident at once.
+template <class Args>
+struct Resident {
+    void (*kernel)(PersistQueue, const Args *);
+    int wave;
+};
+
+// The candidate (fewest blocks an SM first) that runs `items` items in the fewest
+// rounds.
+template <class Args, int N>
+static const Resident<Args> &persist_pick(const Resident<Args> (&c)[N], int items) {
+    int best = 0;
+    for (int k = 1; k < N; ++k)
+        if ((items + c[k].wave - 1) / c[k].wave < (items + c[best].wave - 1) / c[best].wave) best = k;
+    return c[best];
+}
+
+template <class Args>
+static Resident<Args> resident(void (*kernel)(PersistQueue, const Args *), int threads, int fallback, int smem = 0) {
+    if (smem) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return {kernel, wave_of((const void *)kernel, threads, fallback, smem)};
+}
+
+static const Resident<ScatterArgs> (&update_forms())[3] {
+    static const Resident<ScatterArgs> r[3] = {resident(persist_update_kernel<3>, kThreads, 456),
+                                               resident(persist_update_kernel<4>, kThreads, 608),
+                                               resident(persist_update_kernel<5>, kThreads, 760)};
+    return r;
+}
+static const Resident<GatherArgs> (&gather_forms())[2] {
+    static const Resident<GatherArgs> r[2] = {resident(persist_gather_kernel<4>, kThreads, 608),
+                                              resident(persist_gather_kernel<5>, kThreads, 760)};
+    return r;
+}
+static const Resident<ScatterArgs> &scatter_form() {
+    static const Resident<ScatterArgs> r = resident(persist_scatter_kernel, kScatterThreads, 304, kScatterSmem);
+    return r;
+}
+static const Resident<RhoArgs> &rho_form() {
+    static const Resident<RhoArgs> r = resident(persist_rho_kernel, kThreads, 1216);
+    return r;
+}
+
 int persist_density_wave(int stage) {
-    static int waves[4] = {0, 0, 0, 0};
     switch (stage) {
-    case PS_UPDATE:
-        if (!waves[0]) waves[0] = wave_of((const void *)persist_update_kernel, kThreads, 1216);
-        return waves[0];
-    case PS_SCATTER:
-        if (!waves[1]) {
-            cudaFuncSetAttribute(persist_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScatterSmem);
-            waves[1] = wave_of((const void *)persist_scatter_kernel, kScatterThreads, 304, kScatterSmem);
-        }
-        return waves[1];
-    case PS_RHO:
-        if (!waves[2]) waves[2] = wave_of((const void *)persist_rho_kernel, kThreads, 1216);
-        return waves[2];
-    case PS_GATHER:
-        if (!waves[3]) waves[3] = wave_of((const void *)persist_gather_kernel, kThreads, 608);
-        return waves[3];
-    default:
-        return 0;
+    case PS_UPDATE: return update_forms()[2].wave;
+    case PS_SCATTER: return scatter_form().wave;
+    case PS_RHO: return rho_form().wave;
+    case PS_GATHER: return gather_forms()[1].wave;
+    default: return 0;
     }
 }
 
-void launch_persist_density(int stage, const PersistQueue &q, const void *recs, cudaStream_t st) {
-    const int w = persist_density_wave(stage);
+template <class Args>
+static void launch_resident(const Resident<Args> &r, const PersistQueue &q, int items, int threads, int smem,
+                            const void *recs, cudaStream_t st) {
+    r.kernel<<<persist_blocks(r.wave, items), threads, smem, st>>>(q, static_cast<const Args *>(recs));
+}
+
+void launch_persist_density(int stage, const PersistQueue &q, int items, const void *recs, cudaStream_t st) {
     switch (stage) {
-    case PS_UPDATE:
-        persist_update_kernel<<<w, kThreads, 0, st>>>(q, static_cast<const ScatterArgs *>(recs));
-        break;
-    case PS_SCATTER:
-        persist_scatter_kernel<<<w, kScatterThreads, kScatterSmem, st>>>(q, static_cast<const ScatterArgs *>(recs));
-        break;
-    case PS_RHO:
-        persist_rho_kernel<<<w, kThreads, 0, st>>>(q, static_cast<const RhoArgs *>(recs));
-        break;
-    case PS_GATHER:
-        persist_gather_kernel<<<w, kThreads, 0, st>>>(q, static_cast<const GatherArgs *>(recs));
-        break;
-    default:
-        break;
+    case PS_UPDATE: launch_resident(persist_pick(update_forms(), items), q, items, kThreads, 0, recs, st); break;
+    case PS_SCATTER: launch_resident(scatter_form(), q, items, kScatterThreads, kScatterSmem, recs, st); break;
+    case PS_RHO: launch_resident(rho_form(), q, items, kThreads, 0, recs, st); break;
+    case PS_GATHER: launch_resident(persist_pick(gather_forms(), items), q, items, kThreads, 0, recs, st); break;
+    default: break;
     }
 }
 

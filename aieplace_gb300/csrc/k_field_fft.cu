@@ -999,8 +999,8 @@ int persist_field_wave(int tile, int m) {
     return wave_of(k, 8 * tile, 304, smem);
 }
 
-void launch_persist_field(const PersistQueue &q, const FieldRec *recs, int tile, int m, cudaStream_t st) {
-    const int w = persist_field_wave(tile, m), smem = persist_field_smem(tile, m);
+void launch_persist_field(const PersistQueue &q, int items, const FieldRec *recs, int tile, int m, cudaStream_t st) {
+    const int w = persist_blocks(persist_field_wave(tile, m), items), smem = persist_field_smem(tile, m);
     if (tile == 64)
         persist_field_kernel<512><<<w, 512, smem, st>>>(q, recs);
     else

@@ -563,8 +563,8 @@ int persist_wa_wave() {
     return wave;
 }
 
-void launch_persist_wa(const PersistQueue &q, const WaArgs *recs, cudaStream_t st) {
-    persist_wa_kernel<<<persist_wa_wave(), kThreads, 0, st>>>(q, recs);
+void launch_persist_wa(const PersistQueue &q, int items, const WaArgs *recs, cudaStream_t st) {
+    persist_wa_kernel<<<persist_blocks(persist_wa_wave(), items), kThreads, 0, st>>>(q, recs);
 }
 
 }  // namespace ap

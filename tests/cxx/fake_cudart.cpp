@@ -83,8 +83,8 @@ cudaError_t make(T *out) {
     *out = (T)(S().handle += 0x10);
     return cudaSuccess;
 }
-void record(const void *fn, void **args, cudaStream_t st) {
-    fake::Launch l{S().kernels.count(fn) ? S().kernels[fn] : "?", st, {}, false};
+void record(const void *fn, dim3 grid, void **args, cudaStream_t st) {
+    fake::Launch l{S().kernels.count(fn) ? S().kernels[fn] : "?", st, grid.x * grid.y * grid.z, {}, false};
     for (auto &w : S().watched)
         if (l.name.find(w.first) != std::string::npos) {
             l.ptr.push_back(*(const void **)args[w.second]);
@@ -174,12 +174,12 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fn) {
     *k = (cudaKernel_t)fn;
     return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **args, size_t, cudaStream_t st) {
-    record((const void *)k, args, st);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3, void **args, size_t, cudaStream_t st) {
+    record((const void *)k, grid, args, st);
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fn, void **args) {
-    record(fn, args, c->stream);
+    record(fn, c->gridDim, args, c->stream);
     return cudaSuccess;
 }
 cudaError_t cudaGetSymbolAddress(void **p, const void *sym) {

@@ -25,6 +25,7 @@ void *device_only(size_t bytes);  // a device pointer that the host cannot touch
 struct Launch {
     std::string name;
     const void *stream;
+    unsigned blocks;
     std::vector<const void *> ptr;  // the arguments named by watch(), as pointers
     bool early;                     // one of them was still in flight on
                                     // the null stream: a copy from pageable memory

@@ -368,6 +368,32 @@ void null_stream_waits() {
     }
 }
 
+// A batch of few work items launches no more blocks than it has items, and of the
+// kernels that come in several occupancies the one without spilled registers.
+void batch_blocks() {
+    const Netlist n;
+    const ap_params p[3] = {params(32), params(64), params(32)};
+    const ap_netlist nl[3] = {n.nl, n.nl, n.nl};
+    ap_batch *b = nullptr;
+    REQUIRE(ap_create_batch(3, nl, p, &b) == AP_OK && ap_batch_init_seeded(b, 1, 1.f) == AP_OK);
+    ap_batch_info info;
+    float ms[6];
+    REQUIRE(ap_batch_get_info(b, &info) == AP_OK && info.form == AP_BATCH_PERSISTENT);
+    fake::take_launches();
+    REQUIRE(ap_batch_profile(b, 1, ms) == AP_OK);
+    const char *stage[6] = {"persist_update_kernelILi3E", "persist_scatter_kernel", "persist_rho_kernel", "persist_wa_kernel",
+                            "persist_field_kernel", "persist_gather_kernelILi4E"};
+    int seen = 0;
+    for (const fake::Launch &l : fake::take_launches())
+        for (int k = 0; k < 6; ++k)
+            if (l.name.find(stage[k]) != std::string::npos) {
+                REQUIRE(l.blocks >= 1 && (int)l.blocks <= info.items[k]);
+                ++seen;
+            }
+    REQUIRE(seen == 6);
+    REQUIRE(ap_batch_destroy(b) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -378,6 +404,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"trial_graphs", trial_graphs},
     {"profile_launches", profile_launches},
     {"null_stream_waits", null_stream_waits},
+    {"batch_blocks", batch_blocks},
 };
 
 }  // namespace

@@ -19,6 +19,7 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
   profile_launches  ap_profile_stages launches the kernels that a trial does
   null_stream_waits  what a call copies or clears on the null stream has arrived before
                 a launch on a stream of the library's own
+  batch_blocks  a batch of few work items launches no more blocks than items
 """
 import os
 import subprocess
@@ -51,7 +52,8 @@ def host_faults(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
-                                  "shared_memory_limits", "trial_graphs", "profile_launches", "null_stream_waits"])
+                                  "shared_memory_limits", "trial_graphs", "profile_launches", "null_stream_waits",
+                                  "batch_blocks"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
