@@ -202,6 +202,7 @@ void launch_perturb(int n_mov, const float *vx, const float *vy, const float *gx
 
 // ---- host arrays --------------------------------------------------------------
 // device array -> the caller's memory, whose untouched pages it touches first
+void touch_out(void *dst, size_t bytes);  // without the copy
 cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t st);
 
 // ---- field solve ------------------------------------------------------------

@@ -1322,8 +1322,9 @@ int ap_surrogate_forward(ap_surrogate *s, const float *x, int32_t batch, int32_t
     CKS(cudaMemcpy(s->d_a[0], x, sizeof(float) * batch * s->net.cin0 * RR, cudaMemcpyHostToDevice));
     ap::net_infer(s->net, batch, res, s->d_a[0], s->d_a, s->d_a[kSurrLayers], 0);
     CKS(cudaGetLastError());
-    CKS(ap::copy_out(y, s->d_a[kSurrLayers], sizeof(float) * batch * s->net.cout * RR, 0));
-    CKS(cudaStreamSynchronize(0));
+    const size_t bytes = sizeof(float) * batch * s->net.cout * RR;
+    ap::touch_out(y, bytes);
+    CKS(cudaMemcpy(y, s->d_a[kSurrLayers], bytes, cudaMemcpyDeviceToHost));
     return AP_OK;
 }
 

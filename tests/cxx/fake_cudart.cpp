@@ -23,7 +23,7 @@ struct State {
     std::vector<fake::Launch> launches;
     std::map<const char *, size_t> flying;  // null-stream transfers not yet waited for
     std::map<std::string, fake::SmemLimit> smem;
-    int n_malloc = 0, n_graph = 0, n_early = 0, capturing = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
+    int n_malloc = 0, n_graph = 0, n_early = 0, n_wait = 0, capturing = 0, fail_malloc = 0, fail_upload = 0, fail_inst = 0;
     bool malloc_after = false, inst_after = false;
     cudaError_t last = cudaSuccess;
     size_t handle = 0x1000;
@@ -115,6 +115,7 @@ namespace fake {
 void fail_malloc(int n, bool after) { S().fail_malloc = n, S().malloc_after = after; }
 void fail_upload(int n) { S().fail_upload = n; }
 void fail_instantiate(int n, bool after) { S().fail_inst = n, S().inst_after = after; }
+int stream_waits() { return S().n_wait; }
 int graph_launches() { return S().n_graph; }
 int early_launches() { return S().n_early; }
 int mallocs() { return S().n_malloc; }
@@ -299,6 +300,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return make(s
 cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int) { return make(s); }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
+    ++S().n_wait;
     if (!st) S().flying.clear();
     return cudaSuccess;
 }

@@ -16,6 +16,7 @@ void fail_instantiate(int n, bool and_after = false);
 // launches on non-blocking streams, eager or of graphs, while a copy from pageable
 // memory or a memset on the null stream may not have arrived (no stream waits for it)
 int early_launches();
+int stream_waits();      // cudaStreamSynchronize calls so far
 int graph_launches();    // graph launches so far
 int mallocs();           // device allocations asked for so far
 size_t live_bytes();     // device memory held

@@ -394,6 +394,38 @@ void batch_blocks() {
     REQUIRE(ap_batch_destroy(b) == AP_OK);
 }
 
+// Small designs: a call on host arrays waits for the device once, a network's
+// inference not beyond its read-back.
+void small_calls() {
+    const Netlist n;
+    ap_handle *h = create(n, params(32));
+    std::vector<float> x(n.x), y(n.y), gx(x), gy(x), field(32 * 32);
+    std::vector<int64_t> rho(32 * 32);
+    double hp, wa;
+    REQUIRE(ap_init_positions(h, x.data(), y.data()) == AP_OK);
+    const auto waits = [](const std::function<int()> &call) {
+        const int before = fake::stream_waits();
+        REQUIRE(call() == AP_OK);
+        return fake::stream_waits() - before;
+    };
+    REQUIRE(waits([&] { return ap_get_positions(h, x.data(), y.data()); }) == 1);
+    REQUIRE(waits([&] { return ap_density_map(h, x.data(), y.data(), rho.data()); }) == 1);
+    REQUIRE(waits([&] {
+                return ap_wirelength_grad(h, x.data(), y.data(), 4.f, gx.data(), gy.data(), &wa, &hp);
+            }) == 1);
+    REQUIRE(waits([&] {
+                return ap_node_force(h, x.data(), y.data(), field.data(), field.data(), 4.f, 1.f, gx.data(), gy.data(),
+                                     nullptr, nullptr);
+            }) == 1);
+    REQUIRE(ap_destroy(h) == AP_OK);
+    ap_surrogate_config c;
+    ap_surrogate *s = nullptr;
+    REQUIRE(ap_surrogate_config_default(&c) == AP_OK && ap_surrogate_create(&c, &s) == AP_OK);
+    std::vector<float> in((c.factor * c.factor + 2) * 16 * 16), out(2 * c.factor * c.factor * 16 * 16);
+    REQUIRE(waits([&] { return ap_surrogate_forward(s, in.data(), 1, 16, out.data()); }) == 0);
+    REQUIRE(ap_surrogate_destroy(s) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -405,6 +437,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"profile_launches", profile_launches},
     {"null_stream_waits", null_stream_waits},
     {"batch_blocks", batch_blocks},
+    {"small_calls", small_calls},
 };
 
 }  // namespace

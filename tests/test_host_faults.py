@@ -20,6 +20,7 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
   null_stream_waits  what a call copies or clears on the null stream has arrived before
                 a launch on a stream of the library's own
   batch_blocks  a batch of few work items launches no more blocks than items
+  small_calls   calls on host arrays of a small design wait for the device once
 """
 import os
 import subprocess
@@ -53,7 +54,7 @@ def host_faults(tmp_path_factory):
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
                                   "shared_memory_limits", "trial_graphs", "profile_launches", "null_stream_waits",
-                                  "batch_blocks"])
+                                  "batch_blocks", "small_calls"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
