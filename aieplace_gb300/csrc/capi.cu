@@ -22,13 +22,15 @@ namespace ap {
 
 // Device array -> the caller's.  Pages that the caller has not touched yet (a
 // fresh array) cost the copy engine's first write to each far more than the
-// host's: they are touched here first (their contents stay).  Into fresh
-// memory, alone: 180 KB 112 -> 26 us, 1 MB 183 -> 62, 4 MB 264 -> 178, 8 MB 365 ->
-// 334; 16 MB 591 -> 647, so larger arrays are left to the copy.  Only memory that
+// host's: they are touched here first (their contents stay).  An inference whose
+// result of 0.5 MB goes to fresh memory, untouched / touched: 210 / 90 us; 4 MB 386 /
+// 272, 8 MB 592 / 473, 16 MB 987 / 895, 32 MB 1792 / 1727, 48 MB 2572 / 2536; 64 MB
+// 3352 / 3368, 96 MB 4907 / 5002, so beyond 48 MB it is left to the copy.  (Into
+// memory in use it costs nothing that shows, 144 / 143 us at 4 MB.)  Only memory that
 // the runtime knows nothing of is touched: pinned pages are there already, and a
 // device pointer is the copy's to refuse.
 void touch_out(void *dst, size_t bytes) {
-    constexpr size_t kTouchMost = 8u << 20;
+    constexpr size_t kTouchMost = 48u << 20;
     static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
     cudaPointerAttributes at;
     if (bytes <= kTouchMost && bytes > 0 && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&

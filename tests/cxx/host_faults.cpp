@@ -1,5 +1,8 @@
 // Failure paths of the library's host code, on the stand-in runtime of
 // fake_cudart.cpp: host_faults CASE exits 0 if the case holds.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -426,6 +429,41 @@ void small_calls() {
     REQUIRE(ap_surrogate_destroy(s) == AP_OK);
 }
 
+// Results end where the caller's memory does: between pages that fault, at every
+// offset of the end, and past the size from which pages are no longer touched first.
+void outputs_in_bounds() {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const Netlist n;
+    for (int bins : {32, 64}) {
+        ap_handle *h = create(n, params(bins));
+        const size_t bytes = sizeof(int64_t) * bins * bins, span = (bytes + page - 1) / page * page;
+        char *m = (char *)mmap(nullptr, span + 2 * page, PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        REQUIRE(m != MAP_FAILED && mprotect(m + page, span, PROT_READ | PROT_WRITE) == 0);
+        memset(m + page, 7, span);
+        REQUIRE(ap_density_map(h, n.x.data(), n.y.data(), (int64_t *)(m + page + span - bytes)) == AP_OK);
+        for (size_t i = 0; i < span - bytes; ++i) REQUIRE(m[page + i] == 7);
+        REQUIRE(ap_density_map(h, n.x.data(), n.y.data(), (int64_t *)(m + page)) == AP_OK);
+        munmap(m, span + 2 * page);
+        REQUIRE(ap_destroy(h) == AP_OK);
+    }
+    ap_surrogate_config c;
+    ap_surrogate *s = nullptr;
+    REQUIRE(ap_surrogate_config_default(&c) == AP_OK);
+    c.factor = 1;
+    REQUIRE(ap_surrogate_create(&c, &s) == AP_OK);
+    for (int res : {16, 48, 512}) {
+        for (int batch : {1, 3, 24, 25}) {  // 24 and 25 maps of 512: 48 MB and beyond
+            const size_t px = (size_t)batch * res * res, bytes = sizeof(float) * 2 * px, span = (bytes + page - 1) / page * page;
+            std::vector<float> in(3 * px);
+            char *m = (char *)mmap(nullptr, span + 2 * page, PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+            REQUIRE(m != MAP_FAILED && mprotect(m + page, span, PROT_READ | PROT_WRITE) == 0);
+            REQUIRE(ap_surrogate_forward(s, in.data(), batch, res, (float *)(m + page + span - bytes)) == AP_OK);
+            munmap(m, span + 2 * page);
+        }
+    }
+    REQUIRE(ap_surrogate_destroy(s) == AP_OK);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"host_arrays", host_arrays},
     {"create_fails", create_fails},
@@ -438,6 +476,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"null_stream_waits", null_stream_waits},
     {"batch_blocks", batch_blocks},
     {"small_calls", small_calls},
+    {"outputs_in_bounds", outputs_in_bounds},
 };
 
 }  // namespace

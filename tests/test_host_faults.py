@@ -21,6 +21,7 @@ fail.  Each case of tests/cxx/host_faults.cpp runs as a process of its own.
                 a launch on a stream of the library's own
   batch_blocks  a batch of few work items launches no more blocks than items
   small_calls   calls on host arrays of a small design wait for the device once
+  outputs_in_bounds  the host touches no page outside a result's array
 """
 import os
 import subprocess
@@ -54,7 +55,7 @@ def host_faults(tmp_path_factory):
 
 @pytest.mark.parametrize("case", ["host_arrays", "create_fails", "tensor_cores_retry", "solver_info", "device_output",
                                   "shared_memory_limits", "trial_graphs", "profile_launches", "null_stream_waits",
-                                  "batch_blocks", "small_calls"])
+                                  "batch_blocks", "small_calls", "outputs_in_bounds"])
 def test_host_faults(host_faults, case):
     r = subprocess.run([host_faults, case], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, f"exit {r.returncode}\n{r.stderr}"
