@@ -5,16 +5,16 @@
 // as ONE launch over all instances.  The launch executes the blocks of many
 // ordinary launches -- "records", one per instance and stage, record r of
 // nblk[r] blocks -- as work items of `chunk` consecutive blocks each (record
-// r holds items [start[r], start[r + 1])), and its resident blocks pull
-// items off a device queue (an atomic head) until the space is exhausted,
+// r holds items [start[r], start[r + 1])), and its resident blocks, no more than
+// there are items, pull items off a device queue (an atomic head) until the space is exhausted,
 // so instances of uneven size share the GPU without per-instance grids, and
 // the graph of a trial step holds six kernel nodes instead of a dozen per
 // instance.  A record's blocks run the same body the
 // instance's own launch runs (VBlock{id, n} for blockIdx.x / gridDim.x), so
 // each instance's results are the same bit for bit as its own launches'.
 //
-// Records may depend on one another within a launch (the field solve's four
-// contractions of one instance): an item of record r first waits until
+// Records may depend on one another within a launch (the field solve's passes of
+// one instance, the last in two halves): an item of record r first waits until
 // every item of dep[r] has finished.  Items are pulled in order and every
 // dependency points at a record earlier in the item space, so an awaited
 // item was always taken earlier by a running block and the launch cannot

@@ -529,8 +529,8 @@ int build_graphs(ap_handle *h) {
 // The caller's arrays are copied as they are; the order, the die's offset,
 // the check for finite values and the fixed point's conversion are kernels.
 // (As loops over vectors on the host they were most of these calls: the four
-// stage calls on 200k cells 3.9 ms, 1.0 now; a field solve of 1024^2 bins 1.31
-// ms, 0.30 now; reading back 32 designs' positions 2.3 ms, 1.7 now.)
+// stage calls on 200k cells 4.0 ms, 1.0 now; a field solve of 1024^2 bins 1.36
+// ms, 0.30 now.)
 constexpr int kIo = 6;  // 0-3: netlist order, in or out; 4, 5: internal order
 
 int node_blocks(int n) { return std::max(1, std::min((n + kThreads - 1) / kThreads, 4096)); }
@@ -2061,8 +2061,9 @@ void plan_free(PersistPlan &pp) {
     pp.item_blocks = ib;
 }
 
-// Whether the persistent form serves every instance: the FP32 field solve,
-// no surrogate.
+// Whether the persistent form serves every instance: the FP32 field solve, no
+// surrogate.  (The mixed solver's instances, which may be pinned to the tensor cores,
+// stay with the graph form.)
 bool persist_supported(const ap_batch *b) {
     for (const ap_handle *h : b->inst)
         if (h->p.field_solver == AP_FIELD_BF16X3 || h->surr) return false;
@@ -2071,16 +2072,8 @@ bool persist_supported(const ap_batch *b) {
 
 constexpr int kFieldDone = 6;  // first field done counter in PersistPlan::d_cnt
 
-int stage_wave(int k) {
-    switch (k) {
-    case PS_WA:
-        return persist_wa_wave();
-    case PS_FIELD:
-        return persist_field_wave(32, 512);  // not asked for: a field item is one block
-    default:
-        return persist_density_wave(k);
-    }
-}
+// resident blocks of a stage's launch (not of the field's, whose items are blocks)
+int stage_wave(int k) { return k == PS_WA ? persist_wa_wave() : persist_density_wave(k); }
 
 // Blocks per work item of a stage: every stage but the field (whose items
 // are transform passes waited on one by one) takes about kItemsPerBlock
@@ -2125,8 +2118,9 @@ int plan_build(ap_batch *b, PersistPlan &pp) {
     // resident blocks twice over and let the WA launch's blocks in between
     // (a step of 32 instances of 5k-150k cells at overflow 0.97 / 0.05, items of
     // 512, 1024, 2048 nodes, one round of equal items: 271 / 312, 264 / 316, 276 /
-    // 334, 271 / 380 us); the density sums one round of resident blocks (26 ->
-    // 22 us a stage).
+    // 334, 271 / 380 us; of larger designs 1024 and 2048 within 5% of each other: 8 of
+    // 200k 356 / 402 and 355 / 391, 2 of 1M 388 / 443 and 405 / 446); the density sums one
+    // round of resident blocks (26 -> 22 us a stage).
     long long rb = 0;
     for (size_t i = 0; i < b->inst.size(); ++i)
         if (b->active[i]) rb += rho_grid(b->inst[i]->p.bins_x * b->inst[i]->p.bins_y);

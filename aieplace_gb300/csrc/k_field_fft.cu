@@ -27,11 +27,10 @@
 // T[x/4][v][x%4] and U[x/2][v][x%2] (ux, uy), so that the passes along y
 // read and write whole rows of tiles and the pass along x whole 32-byte
 // sectors; within 64 registers a thread, so that every block of a pass is
-// resident at once (72: 15.1 us for P2, a second wave).  Measured (m = 1024,
-// launches alone under ncu): 6.3 + 13.7 + 9.0 us, shared memory 61-77% busy;
-// a 2M-cell loop's iteration 727 us with the matrices' 460 us solve, 234 with
-// this one; 200k cells, m = 512: 208 and 79 us; 32 instances of 128 and 256
-// bins in the persistent launch: 8.57 and 6.92 ms for ten steps and the positions' read-back.
+// resident at once (72: 15.1 us for P2, a second wave).  Measured (m = 1024, launches
+// alone under ncu): 7.4 + 14.4 + 9.4 us, the first 15.0 with the density in it; shared
+// memory 44-64% busy.  The solve alone in a loop of launches, against the dense
+// contractions on the FP32 pipes: 18 and 460 us; at 512 11 and 125.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -877,7 +876,7 @@ int field_solver_init(FieldSolver &f, int m, float bin_ratio) {
         return AP_ERR_CUDA;
     fill_tables(f, 0);
     // the solve's time for ap_solver_info (2 warm, 4 timed; the values do not
-    // matter), on its own scratch: the map read is the first pass's output
+    // matter), on maps of its own
     cudaEvent_t e0, e1;
     if (cudaEventCreate(&e0) != cudaSuccess) return AP_ERR_CUDA;
     if (cudaEventCreate(&e1) != cudaSuccess) {

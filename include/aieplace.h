@@ -314,11 +314,11 @@ int ap_restore(ap_handle *h, const void *buf, size_t bytes);
  *                        over all instances: its resident blocks pull
  *                        (instance, block)
  *                        work items off a device queue, so instances of uneven
- *                        size share the GPU; the field solve's four
+ *                        size share the GPU; the field solve's three
  *                        passes of an instance wait on one another
  *                        inside the launch (bounded waits, below), with the
- *                        tile chosen by the batch's autotuner.  Needs the FP32
- *                        field solve and no surrogate; the default where it
+ *                        block chosen by the batch's autotuner.  Needs
+ *                        AP_FIELD_FP32 and no surrogate; the default where it
  *                        serves every instance.
  *   AP_BATCH_GRAPH       every instance's own launches as parallel branches.
  * Instances keep their own parameters (bin counts may differ) and produce,
@@ -328,8 +328,8 @@ enum { AP_BATCH_GRAPH = 0, AP_BATCH_PERSISTENT = 1 };
 typedef struct {
     int32_t form;                /* AP_BATCH_* */
     int32_t instances, active;
-    int32_t field_tile;          /* persistent form: field tile of the autotuner (32 or 64; 0 = not tuned) */
-    float field_tune_ms[2];      /* its measured field launch with 32 and with 64 tiles */
+    int32_t field_tile;          /* persistent form: field block of the autotuner (8 x 32 or 8 x 64 threads; 0 = not tuned) */
+    float field_tune_ms[2];      /* its measured field launch with either (-1: not run) */
     int32_t records[6];          /* work records per persistent launch: update, scatter, rho, WA, field, gather */
     int32_t item_blocks[6];      /* blocks of a record's own launch per work item */
     int32_t items[6];            /* work items per persistent launch */
